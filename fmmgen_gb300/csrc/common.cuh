@@ -50,7 +50,12 @@ __host__ __device__ __forceinline__ MI fmm_decode(int i) {
 template <typename T>
 __host__ __device__ __forceinline__ void quadrupole_p2p(T x, T y, T z, const T *s, T &phi, T &ex, T &ey, T &ez) {
   const T r2 = x * x + y * y + z * z;
-  const T rinv = T(1) / sqrt(r2), ri2 = rinv * rinv;
+#ifdef __CUDA_ARCH__
+  const T rinv = sizeof(T) == 8 ? T(rsqrt((double)r2)) : T(1) / sqrt(r2);  // FP64: without the division
+#else
+  const T rinv = T(1) / sqrt(r2);
+#endif
+  const T ri2 = rinv * rinv;
   const T r5 = ri2 * ri2 * rinv, r7 = r5 * ri2;
   const T h = T(0.5);
   const T ax = s[0] * x + h * (s[1] * y + s[2] * z);

@@ -1274,69 +1274,3 @@ void fmm_eval_times(DevTree *t) {
     t->kernel_ms[k] = ms;
   }
 }
-
-// ---------------------------------------------------------------------------
-// direct O(N^2) sum in FP64 (example/calculate.cpp:252-264)
-// ---------------------------------------------------------------------------
-#define DIR_BS 128
-__global__ void __launch_bounds__(DIR_BS) k_direct(const double *pos, const double *S, long N, const long *targets,
-                                                   long nt, int so, int potential, int field, double *F) {
-  __shared__ double sx[DIR_BS], sy[DIR_BS], sz[DIR_BS], sq[DIR_BS][6];
-  long t = blockIdx.x * (long)DIR_BS + threadIdx.x;
-  long i = t < nt ? (targets ? targets[t] : t) : -1;
-  double xi = 0, yi = 0, zi = 0;
-  if (i >= 0) { xi = pos[3 * i]; yi = pos[3 * i + 1]; zi = pos[3 * i + 2]; }
-  double phi = 0, ex = 0, ey = 0, ez = 0;
-  for (long b = 0; b < N; b += DIR_BS) {
-    __syncthreads();
-    long j = b + threadIdx.x;
-    if (j < N) {
-      sx[threadIdx.x] = pos[3 * j]; sy[threadIdx.x] = pos[3 * j + 1]; sz[threadIdx.x] = pos[3 * j + 2];
-      if (so == 0) sq[threadIdx.x][0] = S[j];
-      else if (so == 1) { sq[threadIdx.x][0] = S[3 * j]; sq[threadIdx.x][1] = S[3 * j + 1]; sq[threadIdx.x][2] = S[3 * j + 2]; }
-      else for (int k = 0; k < 6; k++) sq[threadIdx.x][k] = S[6 * j + k];
-    }
-    __syncthreads();
-    int cnt = (int)min((long)DIR_BS, N - b);
-    if (i < 0) continue;
-    for (int jj = 0; jj < cnt; jj++) {
-      if (b + jj == i) continue;
-      double dx = xi - sx[jj], dy = yi - sy[jj], dz = zi - sz[jj];
-      if (so == 2) {
-        quadrupole_p2p<double>(dx, dy, dz, sq[jj], phi, ex, ey, ez);
-        continue;
-      }
-      double R = sqrt(dx * dx + dy * dy + dz * dz);
-      double rinv = 1.0 / R;
-      double r3 = rinv * rinv * rinv;
-      if (so == 0) {
-        double q = sq[jj][0];
-        phi += q * rinv;
-        ex += q * dx * r3; ey += q * dy * r3; ez += q * dz * r3;
-      } else {
-        double a = sq[jj][0], bb = sq[jj][1], c = sq[jj][2];
-        double sr = a * dx + bb * dy + c * dz;
-        double r5 = r3 * rinv * rinv;
-        phi -= sr * r3;
-        ex += a * r3 - 3.0 * sr * dx * r5; ey += bb * r3 - 3.0 * sr * dy * r5; ez += c * r3 - 3.0 * sr * dz * r5;
-      }
-    }
-  }
-  if (i >= 0) {
-    int outsize = (potential ? 1 : 0) + (field ? 3 : 0);
-    size_t o = (size_t)t * outsize;
-    int k = 0;
-    if (potential) F[o + k++] = phi;
-    if (field) { F[o + k] = ex; F[o + k + 1] = ey; F[o + k + 2] = ez; }
-  }
-}
-
-int fmm_direct(const double *pos, const double *S, long N, const long *targets, long ntargets, int so,
-               int potential, int field, double *F, cudaStream_t st) {
-  if (!pos || !S || !F || N < 1 || (!potential && !field) || so < 0 || so > 2) return FMM_ERR_ARG;
-  long nt = targets ? ntargets : N;
-  if (nt < 1) return FMM_OK;
-  fmm_note_launch(), k_direct<<<fmm_blocks(nt, DIR_BS), DIR_BS, 0, st>>>(pos, S, N, targets, nt, so, potential, field, F);
-  FMM_CUDA_TRY(cudaGetLastError());
-  return FMM_OK;
-}

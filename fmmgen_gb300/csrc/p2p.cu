@@ -1,76 +1,184 @@
 // p2p.cu -- near-field particle-particle interactions (P2P) over the P2P list
 // (P2P_Cells / evaluate_P2P_lazy, example/calculate.cpp:24-40, 208-216), in FP64
 // and in the mixed-precision form, plus the per-evaluate FP32 staging.
+#include <algorithm>
+#include <cooperative_groups.h>
 #include "internal.h"
 
 // ---------------------------------------------------------------------------
-// P2P in FP64, one warp per target leaf (example/calculate.cpp:24-40, 208-216)
+// P2P in FP64 (example/calculate.cpp:24-40, 208-216)
 // ---------------------------------------------------------------------------
+// Bound by the FP64 pipe: 1.60 operations per clock and SM measured on this
+// part (FP32: 120), so a warp's FP64 instruction takes 20 clocks of its SM and
+// everything else -- shared-memory reads, index arithmetic, shuffles, staging
+// the sources again -- hides behind it.  What counts is that no lane idles.
+// A leaf's targets are therefore cut into groups that fill the warp: chunks of
+// 32, then 16 and 8 targets with 2 and 4 lanes each, then the last m <= 7 with
+// floor(32 / m) lanes each; the f lanes of a target take every f-th source of
+// the stream and their sums are added at the end.  One warp per (leaf, group):
+// the groups of a leaf are independent warps, so leaves of several chunks do
+// not make a tail of long warps.  With one lane per target and chunks of 32 a
+// leaf of 14 left 56 % of the lanes idle and one of 40 took two full passes.
+// The sources of the leaf's list are one stream (the leaves' particle ranges
+// one after the other), staged 64 at a time.
+// Measured (one GB300): 10^6 uniform charges, 30 per leaf, 4.79e9 interactions:
+// 229 -> 158 ms; 100,003 clustered charges, 14 per leaf: the whole step 28.0 -> 17.1 ms; 86,400 dipoles, 11 per
+// leaf: 25.8 -> 10.2 ms.
 #define P2P_WARPS 4
-__global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int *leaf_cells, int nleaves, const int *pstart,
-                                                          const int *pcount, const int *off_, const int *src,
-                                                          const double *px, const double *py, const double *pz,
-                                                          const uint32_t *perm, const double *S, int so,
+#define P64_CHUNK 64
+// components staged per source
+__host__ __device__ constexpr int p64_nq(int so) { return so == 0 ? 1 : so == 1 ? 3 : 6; }
+
+// One source on one target.  SELF: the chunk may hold the target itself.
+template <int SO, bool SELF, bool POT>
+__device__ __forceinline__ void p64_one(double dx, double dy, double dz, const double (*q)[P64_CHUNK], int jj,
+                                        bool self, double &phi, double &ex, double &ey, double &ez) {
+  if (SO == 2) {
+    if (SELF && self) return;
+    const double s[6] = {q[0][jj], q[1][jj], q[2][jj], q[3][jj], q[4][jj], q[5][jj]};
+    quadrupole_p2p<double>(dx, dy, dz, s, phi, ex, ey, ez);
+    return;
+  }
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  double rinv = rsqrt(r2);
+  if (SELF) rinv = self ? 0.0 : rinv;  // l2 != l1
+  const double rr = rinv * rinv;
+  if (SO == 0) {
+    const double qr = q[0][jj] * rinv;
+    if (POT) phi += qr;
+    const double qr3 = qr * rr;
+    ex += qr3 * dx;
+    ey += qr3 * dy;
+    ez += qr3 * dz;
+  } else {
+    const double sx = q[0][jj], sy = q[1][jj], sz = q[2][jj];
+    const double r3 = rr * rinv;
+    const double u = (sx * dx + sy * dy + sz * dz) * r3;
+    if (POT) phi -= u;
+    const double r5 = (3.0 * rr) * u;
+    ex += sx * r3 - r5 * dx;
+    ey += sy * r3 - r5 * dy;
+    ez += sz * r3 - r5 * dz;
+  }
+}
+
+template <int SO, bool POT>
+__global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int *leaf_cells, int nleaves, int nlb, int nchunk,
+                                                          const int *pstart, const int *pcount, const int *off_,
+                                                          const int *src, const double *px, const double *py,
+                                                          const double *pz, const uint32_t *perm, const double *S,
                                                           double *Fnear) {
-  __shared__ double sx[P2P_WARPS][32], sy[P2P_WARPS][32], sz[P2P_WARPS][32], sq[P2P_WARPS][32][6];
+  constexpr int NQ = p64_nq(SO);
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ double sp[P2P_WARPS][3][P64_CHUNK], sq[P2P_WARPS][NQ][P64_CHUNK];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int leaf = blockIdx.x * P2P_WARPS + w;
+  const int y = blockIdx.x / nlb;  // blocks by group: every leaf's first chunk, then the second ones, ...
+  const int leaf = (blockIdx.x - y * nlb) * P2P_WARPS + w;
   if (leaf >= nleaves) return;
   const int A = leaf_cells[leaf];
   const int a0 = pstart[A], na = pcount[A];
+  // this warp's group of targets: [tb, tb + m)
+  const int full = na & ~31, rest = na & 31;
+  int tb, m;
+  if (y < nchunk) {  // a chunk of 32
+    tb = 32 * y;
+    m = tb < full ? 32 : 0;
+  } else if (y == nchunk) {
+    tb = full;
+    m = rest & 16;
+  } else if (y == nchunk + 1) {
+    tb = full + (rest & 16);
+    m = rest & 8;
+  } else {
+    tb = full + (rest & 24);
+    m = rest & 7;
+  }
+  if (m == 0) return;
+  const int f = 32 / m;  // lanes per target
+  const int tl = lane / f, slice = lane - tl * f;
+  const bool ok = tl < m;
+  const int i = a0 + tb + (ok ? tl : 0);
+  const double xi = px[i], yi = py[i], zi = pz[i];
+  double phi = 0, ex = 0, ey = 0, ez = 0;
   const int k0 = off_[A], k1 = off_[A + 1];
-  for (int tb = 0; tb < na; tb += 32) {
-    const int i = a0 + tb + lane;
-    const bool ok = tb + lane < na;
-    double xi = 0, yi = 0, zi = 0;
-    if (ok) { xi = px[i]; yi = py[i]; zi = pz[i]; }
-    double phi = 0, ex = 0, ey = 0, ez = 0;
-    for (int k = k0; k < k1; k++) {
-      const int B = src[k];
-      const int b0 = pstart[B], nb = pcount[B];
-      for (int sb = 0; sb < nb; sb += 32) {
-        __syncwarp();
-        int j = b0 + sb + lane;
-        if (sb + lane < nb) {
-          sx[w][lane] = px[j]; sy[w][lane] = py[j]; sz[w][lane] = pz[j];
-          uint32_t o = perm[j];
-          if (so == 0) sq[w][lane][0] = S[o];
-          else if (so == 1) { sq[w][lane][0] = S[3 * (size_t)o]; sq[w][lane][1] = S[3 * (size_t)o + 1]; sq[w][lane][2] = S[3 * (size_t)o + 2]; }
-          else for (int k = 0; k < 6; k++) sq[w][lane][k] = S[6 * (size_t)o + k];
+  for (int kb = k0; kb < k1; kb += 32) {
+    // up to 32 source leaves: lane q holds leaf kb + q's particle range and the
+    // exclusive prefix of the counts (its offset in the stream)
+    const int nbat = min(32, k1 - kb);
+    int B = -1, start = 0, cnt = 0;
+    if (lane < nbat) {
+      B = src[kb + lane];
+      start = pstart[B];
+      cnt = pcount[B];
+    }
+    int incl = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(FULL, incl, d);
+      if (lane >= d) incl += v;
+    }
+    const int excl = incl - cnt;
+    const int total = __shfl_sync(FULL, incl, 31);
+    const unsigned selfq = __ballot_sync(FULL, B == A);
+    const int self_lo = selfq ? __shfl_sync(FULL, excl, __ffs(selfq) - 1) : -1;
+    for (int cb = 0; cb < total; cb += P64_CHUNK) {
+      const int n = min(P64_CHUNK, total - cb);
+      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < P64_CHUNK / 32; u++) {
+        // the lane's source: the last leaf q whose stream offset is <= s
+        const int s = cb + 32 * u + lane;
+        int q = 0;
+#pragma unroll
+        for (int stp = 16; stp; stp >>= 1) {
+          const int cand = q + stp;
+          const int v = __shfl_sync(FULL, excl, cand & 31);
+          if (cand < nbat && v <= s) q = cand;
         }
-        __syncwarp();
-        const int cnt = min(32, nb - sb);
-        if (ok) {
-          for (int jj = 0; jj < cnt; jj++) {
-            if (b0 + sb + jj == i) continue;  // l2 != l1
-            double dx = xi - sx[w][jj], dy = yi - sy[w][jj], dz = zi - sz[w][jj];
-            if (so == 2) {  // quadrupole sources
-              quadrupole_p2p<double>(dx, dy, dz, sq[w][jj], phi, ex, ey, ez);
-              continue;
-            }
-            double r2 = dx * dx + dy * dy + dz * dz;
-            double rinv = rsqrt(r2);
-            double r3 = rinv * rinv * rinv;
-            if (so == 0) {
-              double q = sq[w][jj][0];
-              phi += q * rinv;
-              double qr3 = q * r3;
-              ex += qr3 * dx; ey += qr3 * dy; ez += qr3 * dz;
-            } else {
-              double sxj = sq[w][jj][0], syj = sq[w][jj][1], szj = sq[w][jj][2];
-              double sr = sxj * dx + syj * dy + szj * dz;
-              double r5 = 3.0 * sr * r3 * rinv * rinv;
-              phi -= sr * r3;
-              ex += sxj * r3 - r5 * dx; ey += syj * r3 - r5 * dy; ez += szj * r3 - r5 * dz;
-            }
-          }
+        const int jb = __shfl_sync(FULL, start, q), je = __shfl_sync(FULL, excl, q);
+        if (s < total) {
+          const int j = jb + (s - je);
+          const size_t o = perm[j];
+          sp[w][0][32 * u + lane] = px[j];
+          sp[w][1][32 * u + lane] = py[j];
+          sp[w][2][32 * u + lane] = pz[j];
+#pragma unroll
+          for (int k = 0; k < NQ; k++) sq[w][k][32 * u + lane] = S[NQ * o + k];
         }
       }
+      __syncwarp();
+      if (!ok) continue;  // the spare lanes of a group of 3, 5, 6 or 7
+      const int me = self_lo + tb + tl - cb;  // the target's own place in the chunk
+      if (self_lo >= 0 && self_lo < cb + n && self_lo + na > cb) {
+        for (int jj = slice; jj < n; jj += f)
+          p64_one<SO, true, POT>(xi - sp[w][0][jj], yi - sp[w][1][jj], zi - sp[w][2][jj], sq[w], jj, jj == me, phi, ex,
+                                 ey, ez);
+      } else {
+#pragma unroll 2
+        for (int jj = slice; jj < n; jj += f)
+          p64_one<SO, false, POT>(xi - sp[w][0][jj], yi - sp[w][1][jj], zi - sp[w][2][jj], sq[w], jj, false, phi, ex,
+                                  ey, ez);
+      }
     }
-    if (ok) {
-      Fnear[4 * (size_t)i] = phi; Fnear[4 * (size_t)i + 1] = ex;
-      Fnear[4 * (size_t)i + 2] = ey; Fnear[4 * (size_t)i + 3] = ez;
+  }
+  // the f partial sums of each target
+  __syncwarp();
+  for (int o = 16; o; o >>= 1) {
+    if (o >= f) continue;
+    const double v0 = __shfl_down_sync(FULL, phi, o), v1 = __shfl_down_sync(FULL, ex, o);
+    const double v2 = __shfl_down_sync(FULL, ey, o), v3 = __shfl_down_sync(FULL, ez, o);
+    if (slice < o && slice + o < f) {
+      phi += v0;
+      ex += v1;
+      ey += v2;
+      ez += v3;
     }
+  }
+  if (ok && slice == 0) {
+    Fnear[4 * (size_t)i] = phi;
+    Fnear[4 * (size_t)i + 1] = ex;
+    Fnear[4 * (size_t)i + 2] = ey;
+    Fnear[4 * (size_t)i + 3] = ez;
   }
 }
 
@@ -449,10 +557,17 @@ int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st, boo
     fmm_note_launch(), k<<<grid, 32 * wp, 0, st>>>(t->leaf_cells.p, nl, t->pstart.p, t->pcount.p, t->p2p_off.p,
                                                    t->p2p_src.p, t->phi4.p, t->plo4.p, t->sdip.p, t->Fnear.p);
   } else {
+    // a leaf holds fewer than ncrit particles (a root leaf fewer than N): its full chunks of 32, then three groups
+    const bool pot = t->pass_potential;
+    const int nchunk = (int)(std::min(t->ncrit - 1, t->N) / 32);
+    const int nlb = (int)fmm_blocks(nl, P2P_WARPS);
+    decltype(&k_p2p64<0, true>) k = so == 0   ? (pot ? k_p2p64<0, true> : k_p2p64<0, false>)
+                                    : so == 1 ? (pot ? k_p2p64<1, true> : k_p2p64<1, false>)
+                                              : k_p2p64<2, true>;
     if (int rc = fmm_mark_kernel(t, 2, st)) return rc;
-    fmm_note_launch(), k_p2p64<<<fmm_blocks(nl, P2P_WARPS), 32 * P2P_WARPS, 0, st>>>(
-        t->leaf_cells.p, nl, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p, t->py.p, t->pz.p,
-        t->perm.p, S, so, t->Fnear.p);
+    fmm_note_launch(), k<<<(unsigned)nlb * (nchunk + 3), 32 * P2P_WARPS, 0, st>>>(
+        t->leaf_cells.p, nl, nlb, nchunk, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p, t->py.p, t->pz.p,
+        t->perm.p, S, t->Fnear.p);
   }
   FMM_CUDA_TRY(cudaGetLastError());
   return fmm_mark_kernel(t, 3, st);
@@ -464,5 +579,126 @@ int fmm_stage_particles(DevTree *t, const double *S, cudaStream_t st) {
       t->leaf_cells.p, t->nleaves, t->pstart.p, t->pcount.p, t->csys.p, t->roots.p, t->px.p, t->py.p, t->pz.p,
       t->perm.p, S, t->so, t->phi4.p, t->plo4.p, t->sdip.p);
   FMM_CUDA_TRY(cudaGetLastError());
+  return FMM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// direct O(N^2) sum in FP64 (example/calculate.cpp:252-264)
+// ---------------------------------------------------------------------------
+// FP64-bound like k_p2p64.  A group of 32 targets (one per lane; fewer than 32
+// targets in all share the lanes) is one cluster of blocks: its 8 warps per block
+// take the source chunks in turn, and the partial sums are added in a fixed
+// order through (distributed) shared memory.  The cluster is as large as it
+// takes to give every SM its share of warps: one thread per target over all
+// sources was 235 blocks of 128 threads at 30,011 targets, two waves of which
+// the second was half empty.  30,011 x 30,011 charges: 57.8 -> 32.9 ms (the square
+// root and division of every pair became one reciprocal square root).
+#define DIR_WARPS 8
+template <int SO>
+__global__ void __launch_bounds__(32 * DIR_WARPS) k_direct(const double *pos, const double *S, long N,
+                                                           const long *targets, long nt, int m, int potential,
+                                                           int field, double *F) {
+  constexpr int NQ = p64_nq(SO);
+  constexpr unsigned FULL = 0xffffffffu;
+  // one warp's staged sources, later its 32 lanes' sums
+  constexpr int AREA = (3 + NQ) * P64_CHUNK;
+  static_assert(AREA >= 4 * 32, "the sums reuse the staging area");
+  __shared__ double sm[DIR_WARPS][AREA];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned nrank = cluster.num_blocks(), rank = cluster.block_rank();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double(*sp)[P64_CHUNK] = (double(*)[P64_CHUNK])sm[w];
+  double(*sq)[P64_CHUNK] = sp + 3;
+  // m targets per group, f = 32 / m lanes per target
+  const int f = 32 / m, tl = lane / f, slice = lane - tl * f;
+  const long t = (long)(blockIdx.x / nrank) * m + tl;
+  const bool ok = tl < m && t < nt;
+  const long i = ok ? (targets ? targets[t] : t) : -1;
+  double xi = 0, yi = 0, zi = 0;
+  if (ok) {
+    xi = pos[3 * i];
+    yi = pos[3 * i + 1];
+    zi = pos[3 * i + 2];
+  }
+  double phi = 0, ex = 0, ey = 0, ez = 0;
+  for (long b = (long)(rank * DIR_WARPS + w) * P64_CHUNK; b < N; b += (long)nrank * DIR_WARPS * P64_CHUNK) {
+    const int n = (int)min((long)P64_CHUNK, N - b);
+    __syncwarp();
+    for (int j = lane; j < n; j += 32) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) sp[k][j] = pos[3 * (b + j) + k];
+#pragma unroll
+      for (int k = 0; k < NQ; k++) sq[k][j] = S[NQ * (b + j) + k];
+    }
+    __syncwarp();
+    if (!ok) continue;
+    const int me = i >= b && i < b + n ? (int)(i - b) : -1;
+#pragma unroll 2
+    for (int jj = slice; jj < n; jj += f)
+      p64_one<SO, true, true>(xi - sp[0][jj], yi - sp[1][jj], zi - sp[2][jj], sq, jj, jj == me, phi, ex, ey, ez);
+  }
+  __syncwarp();
+  double v[4] = {phi, ex, ey, ez};
+  for (int o = 16; o; o >>= 1) {
+    if (o >= f) continue;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const double u = __shfl_down_sync(FULL, v[k], o);
+      if (slice < o && slice + o < f) v[k] += u;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) sm[w][32 * k + lane] = v[k];
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      v[k] = sm[0][32 * k + lane];
+      for (int u = 1; u < DIR_WARPS; u++) v[k] += sm[u][32 * k + lane];
+      sm[0][32 * k + lane] = v[k];
+    }
+  }
+  cluster.sync();
+  if (rank == 0 && w == 0) {
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      for (unsigned r = 1; r < nrank; r++) v[k] += cluster.map_shared_rank(&sm[0][0], r)[32 * k + lane];
+    if (ok && slice == 0) {
+      double *o = F + (size_t)t * ((potential ? 1 : 0) + (field ? 3 : 0));
+      if (potential) *o++ = v[0];
+      if (field) {
+        o[0] = v[1];
+        o[1] = v[2];
+        o[2] = v[3];
+      }
+    }
+  }
+  cluster.sync();  // the sums stay readable until rank 0 has added them
+}
+
+int fmm_direct(const double *pos, const double *S, long N, const long *targets, long ntargets, int so,
+               int potential, int field, double *F, cudaStream_t st) {
+  if (!pos || !S || !F || N < 1 || (!potential && !field) || so < 0 || so > 2) return FMM_ERR_ARG;
+  const long nt = targets ? ntargets : N;
+  if (nt < 1) return FMM_OK;
+  const int m = (int)std::min(nt, 32L);
+  const long groups = (nt + m - 1) / m;
+  // at least four blocks of warps per SM, as long as every warp has sources to take
+  int c = 1;
+  while (c < 8 && groups * c < 4 * 152 && (long)c * DIR_WARPS * P64_CHUNK < N) c *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(groups * c));
+  cfg.blockDim = dim3(32 * DIR_WARPS);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)c;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  fmm_note_launch();
+  FMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, so == 0 ? k_direct<0> : so == 1 ? k_direct<1> : k_direct<2>, pos, S, N,
+                                  targets, nt, m, potential, field, F));
   return FMM_OK;
 }
