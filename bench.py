@@ -368,11 +368,10 @@ def main():
         r = tree.autotune(precision="mixed", reps=3)
         autotune = {"chosen": r["best"], "candidates_ms": [
             [c["impl"], c["nslots"], c["grouping"], c["overlap"], round(c["ms"], 3)] for c in r["table"]],
-            "legend": "impl 0 tensor cores (row gather) / 1 generated CUDA-core / 2 contraction engine / 3 tensor cores "
-                      "(level-grid boxes) / 4 generated class-major / 5 generated target-major; nslots = tensor-core "
+            "legend": "impl 0 the default (as 5) / 1 generated CUDA-core / 2 contraction engine / 3 tensor cores "
+                      "(level-grid boxes) / 4 generated class-major / 5 harmonic coefficients; nslots = tensor-core "
                       "pipeline depth; grouping 0 by octant / 1 Morton; overlap 1 / 2 = M2L and P2P side by side "
-                      "(P2P blocks of 4 / 2 warps); "
-                      "M2L + P2P median ms"}
+                      "(P2P blocks of 4 / 2 warps); M2L + P2P median ms"}
     model = None
     if a.dist == "mixture":  # learned per-pair M2L orders: every pass predicts them from its multipoles
         from fmmgen_gb300 import learned
@@ -568,25 +567,24 @@ def main():
     alg_tf = m2l_flops / (m2l_ms / 1e3) / 1e12 if m2l_ms > 0 else 0.0
     tuned = tree.get_tune()["impl"]
     if m2l_steps:
-        m2l_kernel = ("M2L (k_m2l_tcg, tcgen05 kind::f16, source rows boxed from level grids)" if m2l_boxes
-                      else "M2L (k_m2l_tc, tcgen05 kind::f16)")
+        m2l_kernel = "M2L (k_m2l_tcg, tcgen05 kind::f16, source rows boxed from level grids)"
     elif learned_info:
-        m2l_kernel = ("M2L (k_m2l_tp_*, generated FP32, a thread per target, each pair at its own order; the phase "
-                      "includes the pairs' features and the order model's inference)")
+        m2l_kernel = ("M2L (k_m2lh_*, generated FP32 over harmonic coefficients, a thread per target, each pair at its "
+                      "own order; the phase includes the pairs' features and the order model's inference)")
     else:
         m2l_kernel = {1: "M2L (k_m2l_reg_*, generated FP32, a thread per target)",
                       4: "M2L (k_m2l_cm_*, generated FP32, class-major)",
-                      5: "M2L (k_m2l_tp_*, generated FP32, a thread per target)",
-                      2: "M2L (k_m2l_pk, FP32 contraction engine)"}.get(tuned, "M2L (CUDA cores)")
+                      2: "M2L (k_m2l_pk, FP32 contraction engine)"}.get(
+                          tuned, "M2L (k_m2lh_*, generated FP32 over harmonic coefficients, a thread per target)")
     roofline_m2l = {"kernel": m2l_kernel,
                     "bound": "tensor", "achieved": exec_tf, "algorithmic_tflops": alg_tf, "peak": tpeak,
                     "unit": "TFLOP/s", "frac": exec_tf / tpeak if tpeak else None,
                     "algorithmic_frac": alg_tf / tpeak if tpeak else None,
                     "class_steps": m2l_steps, "mma_instructions": m2l_mmas,
                     "executed_flops_per_launch": m2l_exec_flops, "algorithmic_flops_per_launch": m2l_flops,
-                    "source_rows": "boxed from level grids (tensor-map copies)" if m2l_boxes else "gathered row by row",
+                    "source_rows": "boxed from level grids (tensor-map copies)" if m2l_boxes else None,
                     "note": "executed = MMA flops issued (3 FP16 products per 16-term chunk, 1 for the chunks of "
-                            "degree >= 6 in the level-grid kernel; 128-row tiles over the union of the tile's classes, "
+                            "degree >= 6; 128-row tiles over the union of the tile's classes, "
                             "triangular N per chunk); algorithmic = 2*C(p+6,6) per pair; "
                             "peak = measured bf16 dense (MEASURED_PEAKS.json)"}
 

@@ -31,7 +31,7 @@ def _headers():
 def _generate():
     """(Re)write the generated kernels (csrc/m2l_gen.cuh, csrc/m2l_cm*) when
     their generator is newer."""
-    from . import gen_m2l, gen_m2l_cm
+    from . import gen_m2l, gen_m2l_cm, gen_m2l_h
 
     out, src = gen_m2l.OUT, os.path.abspath(gen_m2l.__file__)
     if not os.path.exists(out) or os.path.getmtime(out) < os.path.getmtime(src):
@@ -41,6 +41,9 @@ def _generate():
                                                   for so, pm in gen_m2l_cm.FAMILIES]
     if any(not os.path.exists(o) or os.path.getmtime(o) < os.path.getmtime(src) for o in outs):
         gen_m2l_cm.generate()
+    src = os.path.abspath(gen_m2l_h.__file__)
+    if any(not os.path.exists(o) or os.path.getmtime(o) < os.path.getmtime(src) for o in gen_m2l_h.outputs()):
+        gen_m2l_h.generate()
 
 
 def build(verbose=False, ptxas_verbose=False):

@@ -680,29 +680,31 @@ static int run_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L, 
   return FMM_OK;
 }
 
-// M2L implementation of a pass: per-pair orders when set; else (mixed pass)
-// the tuned choice or, by default, tensor cores where the order allows
-// (p <= 9, precision "mixed": with source rows boxed from level grids when
-// every level is complete, else gathered row by row), else the generated
-// CUDA-core kernels where this order has them (register-resident, p <= 8;
-// then the target-major kernels of every order up to 12), else the warp
-// contraction engine; FP64: the engine.
-enum { M2L_TC = 0, M2L_GEN = 1, M2L_ENGINE = 2, M2L_TCG = 3, M2L_CM = 4, M2L_TP = 5 };
-static inline bool is_tc(int impl) { return impl == M2L_TC || impl == M2L_TCG; }
+// M2L implementation of a pass: the tuned choice, else the harmonic kernels
+// (m2l_h.cu), in every precision and for per-pair orders.  Against the other
+// mixed kernels they measured (M2L alone, one GB300): 10^6 uniform charges,
+// p = 8: 1.63 ms (tensor cores 2.58, class-major 5.3); p = 6: 0.86 (1.74, 1.87);
+// p = 4: 0.50 (0.95, 1.06); 10^4 charges, p = 4: 25 us (466); 2x10^6 Plummer
+// dipoles, p = 6: 2.8 ms (24.6); 3x10^5 charges, p = 12: 1.03 ms (the 18,564-term
+// kernels 24); FP64, 10^6 charges, p = 8: 48.9 ms (engine 184).
+// Choice 0, once tensor cores with source rows gathered one by one, is the
+// harmonic kernels: its best, 4.04 ms at 10^6 charges and p = 8, was never the
+// faster one.
+enum { M2L_GATHER = 0, M2L_GEN = 1, M2L_ENGINE = 2, M2L_TCG = 3, M2L_CM = 4, M2L_H = 5 };
+static inline bool is_tc(int impl) { return impl == M2L_TCG; }
 bool fmm_m2l_gen_supported(int p, int so) {
   m2l_reg_kernel kg[4];
   int kt[4];
   return m2l_reg_kernels(p, so, kg, kt) > 0;
 }
 static int m2l_impl(const DevTree *t, int precision) {
-  if (precision == 0) return M2L_ENGINE;
+  if (precision == 0) return t->tune.impl == M2L_ENGINE ? M2L_ENGINE : M2L_H;
   const bool tc_ok = fmm_m2l_tc_supported(t->order, t->so), gen_ok = fmm_m2l_gen_supported(t->order, t->so);
   int impl = t->tune.impl;
-  if (impl < 0) impl = precision == 1 ? M2L_TCG : M2L_GEN;
-  if (is_tc(impl) && (!tc_ok || t->nclasses > 262144)) impl = M2L_GEN;  // class bitmap of the tile schedule
-  if (impl == M2L_CM && (!fmm_m2l_cm_supported(t->order, t->so) || t->nclasses > 262144)) impl = M2L_GEN;
-  if (impl == M2L_TP && !fmm_m2l_cm_supported(t->order, t->so)) impl = M2L_GEN;
-  if (impl == M2L_GEN && !gen_ok) impl = fmm_m2l_cm_supported(t->order, t->so) ? M2L_TP : M2L_ENGINE;
+  if (impl < 0 || impl == M2L_GATHER) impl = M2L_H;
+  if (is_tc(impl) && (!tc_ok || t->nclasses > 262144)) impl = M2L_H;  // class bitmap of the tile schedule
+  if (impl == M2L_CM && (!fmm_m2l_cm_supported(t->order, t->so) || t->nclasses > 262144)) impl = M2L_H;
+  if (impl == M2L_GEN && !gen_ok) impl = M2L_H;
   return impl;
 }
 
@@ -747,6 +749,8 @@ static int m2l_phase(DevTree *t, const PlanSet *ps, const T *M, T *L, bool mixed
                      int dstr, cudaStream_t st) {
   const int p = t->order, so = t->so, nc = t->ncells;
   t->tc_ran = 0;
+  // level grids need every level to be complete
+  if (is_tc(impl) && t->ord_mode == 0 && t->nm2l > 0 && !fmm_m2l_tc_boxes_ok(t, st)) impl = M2L_H;
   // every M2L but the tensor cores' reads the target lists
   if (t->ord_mode != 0 || !(mixed && (is_tc(impl) || impl == M2L_CM))) TRY(fmm_m2l_csr(t, st));
   // a tuned choice pins the per-pair-order kernels: 2 the engine, 4 class-major, else target-major
@@ -758,12 +762,13 @@ static int m2l_phase(DevTree *t, const PlanSet *ps, const T *M, T *L, bool mixed
       fmm_set_error_text("per-pair M2L orders were set for an earlier build");
       return FMM_ERR_STATE;
     }
-    if constexpr (std::is_same<T, float>::value) {
-      // mixed: the generated kernels, each lane truncating at its pair's order
-      const int rc = timpl == M2L_ENGINE ? FMM_ERR_STATE
-                     : timpl == M2L_CM   ? fmm_m2l_cm(t, M, mstr, L, lstr, t->m2l_ord.p, st)
-                                         : fmm_m2l_tp(t, M, mstr, L, lstr, t->m2l_ord.p, st);
-      if (rc != FMM_ERR_STATE) return rc;
+    if (timpl != M2L_ENGINE) {  // the generated kernels, each lane truncating at its pair's order
+      if constexpr (std::is_same<T, float>::value)
+        if (timpl == M2L_CM) {
+          const int rc = fmm_m2l_cm(t, M, mstr, L, lstr, t->m2l_ord.p, st);
+          if (rc != FMM_ERR_STATE) return rc;
+        }
+      return fmm_m2l_h(t, M, mstr, L, lstr, t->m2l_ord.p, st);
     }
     FMM_CUDA_TRY(cudaMemsetAsync(L, 0, sizeof(T) * (size_t)nc * lstr, st));
     TRY(fmm_mark_kernel(t, 0, st));
@@ -782,11 +787,11 @@ static int m2l_phase(DevTree *t, const PlanSet *ps, const T *M, T *L, bool mixed
     }
     TRY(fmm_mark_kernel(t, 1, st));
   } else if (mixed && is_tc(impl)) {
-    TRY(fmm_m2l_tc(t, (const float *)(const void *)M, mstr, (float *)(void *)L, lstr, st, impl == M2L_TCG));
+    TRY(fmm_m2l_tc(t, (const float *)(const void *)M, mstr, (float *)(void *)L, lstr, st));
   } else if (mixed && impl == M2L_CM) {
     TRY(fmm_m2l_cm(t, (const float *)(const void *)M, mstr, (float *)(void *)L, lstr, nullptr, st));
-  } else if (mixed && impl == M2L_TP) {
-    TRY(fmm_m2l_tp(t, (const float *)(const void *)M, mstr, (float *)(void *)L, lstr, nullptr, st));
+  } else if (impl == M2L_H) {
+    TRY(fmm_m2l_h(t, M, mstr, L, lstr, nullptr, st));
   } else if (mixed && impl == M2L_GEN) {
     m2l_reg_kernel kg[4];
     int kthreads[4];

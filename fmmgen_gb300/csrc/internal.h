@@ -73,8 +73,9 @@ struct DevTree {
   DevBuf<int> m2l_order;                  // cells in M2L processing order (level, then the grouping below)
   // M2L choices (set by fmmgen_tree_set_tune / the autotuner; -1 / 0: the default rules)
   struct M2LTune {
-    int impl = -1;      // mixed pass: 0 tensor cores, 1 generated CUDA-core kernels, 2 contraction engine
-    int nslots = 0;     // tensor-core pipeline depth (row-gather slots), 0: as many as fit
+    int impl = -1;      // -1, 0, 5 harmonic kernels, 1 generated CUDA-core, 2 contraction engine, 3 tensor cores
+                        // (level grids), 4 class-major
+    int nslots = 0;     // tensor-core pipeline depth (operand slots), 0: as many as fit
     int grouping = 0;   // cell order within a level: 0 by octant within the parent, 1 Morton
     int overlap = 0;    // tensor-core M2L on a high-priority side stream, P2P beside it on the SMs' spare
                         // room in blocks of 4 (1) or 2 (2) warps
@@ -107,8 +108,6 @@ struct DevTree {
 #define FMM_PINNED_TCERR 12               // h_pinned words 12..15: last tensor-core M2L error flags, class steps
   // tensor-core M2L operands (m2l_tc.cu)
   DevBuf<unsigned char> tc_T;             // split, swizzled operator records per class
-  DevBuf<uint16_t> tc_Mh, tc_Ml;          // scaled, split source multipoles (FP16 bits)
-  DevBuf<int> tc_mexp;                    // per cell: scale exponent of its multipole row
   DevBuf<uint32_t> d_tcerr;               // kernel timeout flags
   uint64_t build_serial = 0, tc_serial = ~0ull;  // tc_T belongs to the build with this serial
   DevBuf<int> tc_sched_off;               // class-step schedule of the tensor-core M2L tiles
@@ -118,8 +117,11 @@ struct DevTree {
   DevBuf<unsigned char> cm_otab;          // per class step: each tile row's per-pair M2L order
   DevBuf<int> cm_woff, cm_wstep;          // per (tile, warp of 32 rows): its steps with a pair
   uint64_t cm_wserial = ~0ull, cm_wversion = ~0ull;  // ... of this schedule (build, cell order)
+  DevBuf<char> hM, hL, hD;                // harmonic M2L: folded multipoles, outputs, operators (m2l_h.cu)
   DevBuf<int> tp_perm;                    // per target list: pair indices by descending per-pair order
-  DevBuf<int> tp_tgt;                     // targets by level, then by their count of high-order pairs
+  DevBuf<int> tp_tgt;                     // targets by list length (of this build and cell order); with per-pair
+                                          // orders by level, then by their count of high-order pairs
+  uint64_t tgt_serial = ~0ull, tgt_version = ~0ull;
   void *tcg = nullptr;                    // level-grid tensor-core M2L state (m2l_tc.cu, fmm_tcg_release)
   int tc_boxes_last = 0;                  // the last tensor-core M2L boxed its source rows from level grids
   int tc_ran = 0;                         // the last pass's M2L ran on the tensor cores
@@ -205,9 +207,9 @@ int fmm_mlp_train_step(const float *params, const float *X, const unsigned char 
                        float *work, cudaStream_t st);
 int fmm_mlp_adam(float *params, const float *grad, float *m, float *v, int step, float lr, cudaStream_t st);
 int fmm_learned_orders(DevTree *t, cudaStream_t st);
-bool fmm_m2l_tc_step_work(int p, int so, bool boxes, long long *mmas, double *flops);
-// boxes: source rows by tensor-map box loads from level grids where every level is complete
-int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStream_t st, bool boxes);
+bool fmm_m2l_tc_step_work(int p, int so, long long *mmas, double *flops);
+// tensor-core M2L with source rows boxed from level grids (FMM_ERR_STATE where a level is not complete)
+int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStream_t st);
 void fmm_tcg_release(DevTree *t);
 // marks the start (which 0) / end (1) of the pass's M2L kernels, the start (2) / end (3) of its
 // P2P kernel, on their streams
@@ -217,9 +219,14 @@ int fmm_tc_schedule(DevTree *t, cudaStream_t st);
 // class-major generated CUDA-core M2L over that schedule (m2l_cm_s*.cu); ord: per-pair orders in target-list
 // order or null; FMM_ERR_STATE when no family covers (order, source order) or the schedule cannot be built
 int fmm_m2l_cm(DevTree *t, const float *M, int mstr, float *L, int lstr, const unsigned char *ord, cudaStream_t st);
-// the same kernel bodies, one thread per target cell over its target list (m2l_cm_s*.cu)
-int fmm_m2l_tp(DevTree *t, const float *M, int mstr, float *L, int lstr, const unsigned char *ord, cudaStream_t st);
 bool fmm_m2l_cm_supported(int p, int so);
+// M2L over harmonic coefficients, a thread per target cell over its list (m2l_h.cu); every order and source order
+int fmm_m2l_h(DevTree *t, const float *M, int mstr, float *L, int lstr, const unsigned char *ord, cudaStream_t st);
+int fmm_m2l_h(DevTree *t, const double *M, int mstr, double *L, int lstr, const unsigned char *ord, cudaStream_t st);
+bool fmm_m2l_h_supported(int p, int so);
+// targets of the harmonic M2L (tp_tgt): by list length, longest first; with per-pair orders by their high-order pairs,
+// and each list by descending order (tp_perm)
+int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st);
 bool fmm_m2l_tc_boxes_ok(DevTree *t, cudaStream_t st);  // the level-grid path can run on this build
 // M2M of the parents / L2L into the children of cells [lo, hi), FP32 scaled expansions (shift.cu)
 int fmm_m2m_tab(DevTree *t, int lo, int hi, float *M, int mstr, cudaStream_t st);

@@ -23,30 +23,16 @@
 // FP32 registers with round-to-nearest -- the per-pair partial sums of the
 // CUDA-core kernels.
 //
-// Tiles take 128 cells of one level and one octant-within-parent, parents in
-// Morton order: those cells have near-identical interaction lists, so a tile
-// visits ~1.4x the classes of one list.  The class steps of every tile (the
-// sorted union of its rows' classes) and each step's source per row (-1 for a
-// row without a source in the class) are scattered once per build straight
-// from the walk-order pairs, with no sort (k_tc_bitmap .. k_tc_scatter): the
-// kernel's warps then follow that schedule independently, coupled only
-// through mbarriers.
-//
-// Per CTA (one per SM, persistent), 17 warps:
-//  * warps 0-7 gather the source rows of each (class, 64-term K-block) step
-//    (warps w and w+4: rows 32 (w % 4) .. + 31, one half of the chunks each)
-//    into a stage slot with cp.async, in the 128-byte swizzled K-major layout,
-//    and arrive on the slot's mbarrier when their copies land
-//    (cp.async.mbarrier.arrive); thread 0 also fetches the class's pre-split
-//    operator chunks (32-byte swizzled) and column scales with bulk copies.  A
-//    row without a source in the class is not copied: its accumulator row
-//    holds garbage that the fold leaves out;
-//  * warps 8-15 fold each finished class step out of tensor memory (warps w
-//    and w+4 take the two column halves of lane quarter w % 4) and store the
-//    tile's rows;
-//  * warp 16 allocates 512 tensor-memory columns (two accumulators) and one of
-//    its lanes issues the MMAs.
-// Stage slots and accumulators circulate through mbarriers; every wait is
+// The sources of a tile's rows in one class are boxed from dense level grids by
+// tensor-map copies (k_m2l_tcg below), which needs every level to be complete;
+// other trees run the harmonic kernels (m2l_h.cu), which measure faster on
+// these too (10^6 charges, p = 8: 1.63 against 2.58 ms) and are the default: this
+// kernel runs where it is chosen.
+// The class-step schedule of tiles of 128 cells in M2L processing order (the
+// sorted union of its rows' classes, each step's source per row) is scattered
+// once per build straight from the walk-order pairs, with no sort
+// (k_tc_bitmap .. k_tc_scatter), for the class-major kernels (m2l_cm_s*.cu).
+// Operand slots and accumulators circulate through mbarriers; every wait is
 // bounded and reports a timeout through an error flag instead of hanging.
 #include <algorithm>
 #include <cstddef>
@@ -60,39 +46,15 @@ namespace {
 
 constexpr int TC_ROWS = 128;      // target cells per tile (MMA M)
 constexpr int TC_CH = 16;         // multipole terms per K chunk (one kind::f16 MMA)
-constexpr int TC_KB = 64;         // terms per K-block: one 128-byte swizzle row of FP16
 constexpr int TC_A_BYTES = TC_ROWS * 128;  // one operand half (hi or lo) of a K-block
 constexpr int TC_MAXCH = 16;      // K chunks (p <= 9: at most 14)
 constexpr int TC_MAXKB = 4;
-constexpr int TC_GWARPS = 8;      // gather warps 0-7
-constexpr int TC_FWARPS = 8;      // fold warps 8-15
-constexpr int TC_MWARP = TC_GWARPS + TC_FWARPS;  // warp 16: tensor memory + MMA issue
-constexpr int TC_GATHER = 32 * TC_GWARPS;
+constexpr int TC_FWARPS = 8;      // fold warps
 constexpr int TC_FOLD = 32 * TC_FWARPS;
-constexpr int TC_THREADS = 32 * (TC_MWARP + 1);
 constexpr int TC_MAXSLOTS = 4;
 constexpr int TC_ACC_COLS = 256;  // tensor-memory columns per accumulator
 constexpr int TC_EBIAS = 14;      // operands are scaled to [2^14, 2^15) in magnitude
-constexpr unsigned TC_NONE = 0xffffffffu;
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 24;
-
-struct TcParams {
-  const int *order;               // cells in M2L processing order
-  int ncells, ntiles;
-  const int *sched_off;           // [ntiles + 1] class steps of each tile
-  const unsigned *sched_cls;      // [steps] class of the step
-  const int *stab;                // [steps][128] source cell of each tile row in the step, -1: none
-  const __half *Mh, *Ml;          // scaled, split source multipoles, row stride kpad
-  const int *mexp;                // per cell: row scale exponent (M~ = 2^mexp (Mh + Ml))
-  const unsigned char *T;         // per class: split, swizzled operator chunks, then column scales
-  float *L;                       // scaled local expansions (FP32), row stride lstride
-  int lstride, lsize, kpad, kch, nkb, nslots;
-  int cls_bytes, cls_scale, slot_bytes, nout;
-  int nch[TC_MAXCH];              // MMA N of each K chunk
-  int choff[TC_MAXCH + 1];        // byte offset of each chunk's (hi, lo) block in a class record
-  uint32_t *err;                  // [0] bit 0: a gather-side wait timed out, bit 1: an MMA-side wait;
-                                  // [2..3] class steps issued (u64, for the executed-work count)
-};
 
 __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -123,14 +85,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   return false;
 }
 
-__device__ __forceinline__ void cp16(uint32_t dst, const void *src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-// arrive on the mbarrier when all cp.async copies this thread issued so far have landed
-__device__ __forceinline__ void cp_arrive(uint32_t bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // make this thread's generic-proxy shared-memory writes visible to the async proxy (tensor cores)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -236,13 +190,12 @@ namespace {
 struct TcShared {
   alignas(16) float colf[2][TC_ACC_COLS];  // column scales 2^g of the class in each accumulator (bulk-copy
                                            // destination: 16-byte aligned)
-  uint64_t full[TC_MAXSLOTS];   // slot filled: 256 cp.async arrivals + thread 0's expect_tx arrival
+  uint64_t full[TC_MAXSLOTS];   // slot filled: its producer's expect_tx arrival and the copies' bytes
   uint64_t empty[TC_MAXSLOTS];  // slot consumed: MMA commit
   uint64_t accfull[2];          // class step accumulated: MMA commit
   uint64_t accempty[2];         // accumulator folded out: 256 fold arrivals
   uint64_t colfull[2];          // column scales of the class in each accumulator landed (bulk copy)
   uint64_t drain;               // every MMA complete (before tensor memory is released)
-  int hdr[TC_MAXSLOTS];         // K-block of the slot's step; -1: end of work
   uint32_t ch_idesc[TC_MAXCH];  // per K chunk: instruction descriptor (N of the chunk)
   uint32_t ch_boff[TC_MAXCH];   // per K chunk: offset of its hi block in the slot's operator area, >> 4
   uint32_t ch_nlo[TC_MAXCH];    // per K chunk: offset of its lo block from its hi block, >> 4
@@ -261,267 +214,6 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok = 0;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity) ? 1u : 0u;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-
-// Add class step v's accumulator (this thread's lane, HALF columns from col0),
-// times its row scale 2^e and the class's column scales, into the FP32 running
-// sums -- rows with a source in the step only -- and hand the accumulator back
-// to the MMA issuer.
-template <int HALF>
-__device__ __forceinline__ bool fold(float *acc, uint32_t tlane, int col0, uint32_t v, int e, bool mine,
-                                     uint32_t accfull0, uint32_t accempty0, uint32_t colfull0, TcShared *cs) {
-  const uint32_t b = v & 1;
-  if (!warp_wait(colfull0 + 8 * b, (v >> 1) & 1) || !warp_wait(accfull0 + 8 * b, (v >> 1) & 1)) return false;
-  tc_fence_after();
-  __syncwarp();  // tcgen05.ld is warp-collective
-  const float rowf = ldexpf(1.f, e);
-  const float *cf = cs->colf[b] + col0;
-  // columns in loads of 16, then 8 (one wait each)
-  constexpr int N16 = HALF / 16, N8 = (HALF % 16) / 8;
-#pragma unroll
-  for (int j = 0; j < N16; j++) {
-    float t[16];
-    tmem_ld16(tlane + b * TC_ACC_COLS + 16 * j, t);  // warp-collective: every lane loads
-    if (mine)  // a row without a source in the step holds garbage: left out
-#pragma unroll
-      for (int i = 0; i < 16; i++) acc[16 * j + i] = fmaf(t[i], rowf * cf[16 * j + i], acc[16 * j + i]);
-  }
-  if (N8) {
-    constexpr int c0 = 16 * N16;
-    float t[8];
-    tmem_ld8(tlane + b * TC_ACC_COLS + c0, t);
-    if (mine)
-#pragma unroll
-      for (int i = 0; i < 8; i++) acc[c0 + i] = fmaf(t[i], rowf * cf[c0 + i], acc[c0 + i]);
-  }
-  tc_fence_before();
-  mbar_arrive(accempty0 + 8 * b);
-  return true;
-}
-
-template <int NOUT>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_m2l_tc(const TcParams P) {
-  constexpr int HALF = NOUT / 2;  // accumulator columns folded by each epilogue thread
-  extern __shared__ __align__(1024) unsigned char tc_smem[];
-  const uint32_t raw = su32(tc_smem);
-  const uint32_t base = (raw + 1023u) & ~1023u;  // the 128-byte swizzle pattern repeats every 1024 bytes
-  TcShared *cs = (TcShared *)(tc_smem + (base - raw) + P.nslots * P.slot_bytes);
-  const uint32_t full0 = su32(&cs->full[0]), empty0 = su32(&cs->empty[0]);
-  const uint32_t accfull0 = su32(&cs->accfull[0]), accempty0 = su32(&cs->accempty[0]);
-  const uint32_t colfull0 = su32(&cs->colfull[0]), drain = su32(&cs->drain);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-  if (tid < TC_MAXCH) {
-    const int ch = tid;
-    cs->ch_idesc[ch] = ch < P.kch ? idesc_f16(P.nch[ch]) : 0u;
-    cs->ch_boff[ch] = ch < P.kch ? (uint32_t)(P.choff[ch] - P.choff[ch & ~3]) >> 4 : 0u;
-    cs->ch_nlo[ch] = ch < P.kch ? (uint32_t)P.nch[ch] * 2u : 0u;  // nch rows x 32 bytes, >> 4
-  }
-  if (tid == 0) {
-    for (int i = 0; i < P.nslots; i++) {
-      mbar_init(full0 + 8 * i, TC_GATHER + 1);  // every gather thread + thread 0's expect_tx
-      mbar_init(empty0 + 8 * i, 1);
-    }
-    for (int i = 0; i < 2; i++) {
-      mbar_init(accfull0 + 8 * i, 1);
-      mbar_init(accempty0 + 8 * i, TC_FOLD);
-      mbar_init(colfull0 + 8 * i, 1);
-    }
-    mbar_init(drain, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == TC_MWARP) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&cs->tmem)),
-                 "r"(2 * TC_ACC_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = cs->tmem;
-
-  if (warp < TC_GWARPS) {
-    // ---------------- gather ----------------
-    const int quarter = warp & 3, chalf = warp >> 2;  // rows 32 quarter .. + 31, chunks 4 chalf .. + 3
-    const int row = 32 * quarter + lane;  // tile row whose list this thread walks
-    uint32_t g = 0, u = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < P.ntiles && ok; tile += gridDim.x) {
-      const int s0 = P.sched_off[tile], s1 = P.sched_off[tile + 1];
-      // the row's source in the next step, loaded a step before it is needed
-      int hsrc = s0 < s1 ? P.stab[(size_t)s0 * TC_ROWS + row] : -1;
-      for (int st = s0; st < s1; st++, u++) {
-        const unsigned c = P.sched_cls[st];
-        const int mysrc = hsrc;
-        if (st + 1 < s1) hsrc = P.stab[(size_t)(st + 1) * TC_ROWS + row];
-        for (int kb = 0; kb < P.nkb; kb++) {
-          const int slot = (int)(g % (uint32_t)P.nslots);
-          const uint32_t use = g / (uint32_t)P.nslots;
-          if (!warp_wait(empty0 + 8 * slot, (use & 1) ^ 1)) { ok = false; break; }
-          const uint32_t sa = base + (uint32_t)slot * P.slot_bytes;
-          const int qn = min(8, (P.kpad - TC_KB * kb) >> 3);  // valid 16-byte chunks of the K-block
-#pragma unroll
-          for (int jj = 0; jj < 4; jj++) {
-            const int rl = 8 * jj + (lane >> 2), q = 4 * chalf + (lane & 3);  // 8 rows x 4 chunks per instruction
-            const int r = 32 * quarter + rl;
-            const int sr = __shfl_sync(0xffffffffu, mysrc, rl);
-            if (sr >= 0 && q < qn) {
-              const size_t e = (size_t)sr * P.kpad + TC_KB * kb + 8 * q;
-              const uint32_t o = (uint32_t)r * 128u + ((uint32_t)(q ^ (r & 7)) << 4);
-              cp16(sa + o, P.Mh + e, 16u);
-              cp16(sa + TC_A_BYTES + o, P.Ml + e, 16u);
-            }
-          }
-          if (tid == 0) {
-            cs->hdr[slot] = kb;
-            const unsigned char *rec = P.T + (size_t)c * P.cls_bytes;
-            const uint32_t b0 = P.choff[4 * kb], b1 = P.choff[min(4 * kb + 4, P.kch)];
-            mbar_arrive_tx(full0 + 8 * slot, b1 - b0);
-            bulk_g2s(sa + 2 * TC_A_BYTES, rec + b0, b1 - b0, full0 + 8 * slot);
-            if (kb == 0) {
-              // the class's column scales, for the fold of this step, into
-              // buffer u & 1 once the fold of step u - 2 has read it
-              const uint32_t cb = colfull0 + 8 * (u & 1), sc = 4u * (uint32_t)P.nout;
-              if (!mbar_wait(accempty0 + 8 * (u & 1), ((u >> 1) & 1) ^ 1)) ok = false;
-              fence_async_smem();
-              mbar_arrive_tx(cb, sc);
-              bulk_g2s(su32(cs->colf[u & 1]), rec + P.cls_scale, sc, cb);
-            }
-          }
-          cp_arrive(full0 + 8 * slot);
-          g++;
-        }
-        if (!__all_sync(0xffffffffu, ok)) ok = false;
-        if (!ok) break;
-      }
-    }
-    // end of work: one more slot carrying only the end mark
-    if (ok) {
-      const int slot = (int)(g % (uint32_t)P.nslots);
-      const uint32_t use = g / (uint32_t)P.nslots;
-      if (warp_wait(empty0 + 8 * slot, (use & 1) ^ 1)) {
-        if (tid == 0) {
-          cs->hdr[slot] = -1;
-          mbar_arrive(full0 + 8 * slot);
-        }
-        mbar_arrive(full0 + 8 * slot);
-      } else {
-        ok = false;
-      }
-    }
-    cp_wait_all();
-    if (!ok && lane == 0) atomicOr(P.err, 1u);
-    if (tid == 0) atomicAdd((unsigned long long *)(P.err + 2), (unsigned long long)u);
-  } else if (warp < TC_MWARP) {
-    // ---------------- fold + store ----------------
-    const int fw = warp - TC_GWARPS;
-    const int quarter = warp & 3, half = fw >> 2;  // tensor-memory lanes 32 (warp % 4) .. + 31
-    const int row = 32 * quarter + lane;
-    const uint32_t tlane = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(half * HALF);
-    uint32_t u = 0;
-    bool ok = true;
-    float acc[HALF];
-    for (int tile = blockIdx.x; tile < P.ntiles && ok; tile += gridDim.x) {
-      const int rr = tile * TC_ROWS + row;
-      const int A = rr < P.ncells ? P.order[rr] : -1;
-      float *Lrow = A >= 0 ? P.L + (size_t)A * P.lstride + half * HALF : nullptr;
-      const int ncol = min(HALF, P.lsize - half * HALF);  // stored columns of this half
-#pragma unroll
-      for (int i = 0; i < HALF; i++) acc[i] = 0.f;
-      const int s0 = P.sched_off[tile], s1 = P.sched_off[tile + 1];
-      int hsrc = s0 < s1 ? P.stab[(size_t)s0 * TC_ROWS + row] : -1;
-      for (int st = s0; st < s1; st++, u++) {
-        const bool mine = hsrc >= 0;
-        const int e = mine ? P.mexp[hsrc] : 0;
-        if (st + 1 < s1) hsrc = P.stab[(size_t)(st + 1) * TC_ROWS + row];
-        if (!fold<HALF>(acc, tlane, half * HALF, u, e, mine, accfull0, accempty0, colfull0, cs)) {
-          ok = false;
-          break;
-        }
-      }
-      if (!ok) break;
-      if (Lrow)
-#pragma unroll
-        for (int i = 0; i < HALF; i++)
-          if (i < ncol) Lrow[i] = acc[i];
-    }
-    if (!ok && lane == 0) atomicOr(P.err, 1u);
-  } else if (lane == 0) {
-    // ---------------- MMA issue (one thread of warp 16) ----------------
-    // Per-chunk instruction descriptors and operator offsets live in
-    // registers (compile-time indices below), so nothing but descriptor
-    // arithmetic sits between consecutive MMAs.
-    uint32_t idr[TC_MAXCH], bor[TC_MAXCH], nlr[TC_MAXCH];
-#pragma unroll
-    for (int ch = 0; ch < TC_MAXCH; ch++) {
-      idr[ch] = cs->ch_idesc[ch];
-      bor[ch] = cs->ch_boff[ch];
-      nlr[ch] = cs->ch_nlo[ch];
-    }
-    const int kch = P.kch;
-    uint32_t g = 0, u = 0;
-    bool ok = true;
-    while (true) {
-      const int slot = (int)(g % (uint32_t)P.nslots);
-      if (!mbar_wait(full0 + 8 * slot, (g / (uint32_t)P.nslots) & 1)) { ok = false; break; }
-      fence_async_smem();  // the gathered rows were written by cp.async (generic proxy)
-      tc_fence_after();
-      const int kb = cs->hdr[slot];
-      if (kb < 0) break;
-      const uint32_t b = u & 1;
-      if (kb == 0) {  // a class step starts: its accumulator must have been folded out
-        if (!mbar_wait(accempty0 + 8 * b, ((u >> 1) & 1) ^ 1)) { ok = false; break; }
-        tc_fence_after();
-      }
-      // descriptors: the slot's base descriptors plus per-chunk offsets in
-      // 16-byte units (all shared addresses stay below 256 KB, so the 14-bit
-      // start-address field never carries)
-      const uint32_t sa = base + (uint32_t)slot * P.slot_bytes;
-      const uint64_t ah0 = sw128_desc(sa), al0 = sw128_desc(sa + TC_A_BYTES);
-      const uint64_t b0 = sw32_desc(sa + 2 * TC_A_BYTES);
-      const uint32_t d = tmem + b * TC_ACC_COLS;
-#define TC_CHUNK(KB, J)                                                                 \
-  if (4 * (KB) + (J) < kch) {                                                           \
-    const uint64_t bh = b0 + bor[4 * (KB) + (J)], bl = bh + nlr[4 * (KB) + (J)];        \
-    const uint64_t ah = ah0 + 2 * (J), al = al0 + 2 * (J); /* 32 bytes along the row */ \
-    mma_f16(d, ah, bh, idr[4 * (KB) + (J)], ((KB) == 0 && (J) == 0) ? 0u : 1u);         \
-    mma_f16(d, ah, bl, idr[4 * (KB) + (J)], 1u);                                        \
-    mma_f16(d, al, bh, idr[4 * (KB) + (J)], 1u);                                        \
-  }
-#define TC_KBLOCK(KB) \
-  TC_CHUNK(KB, 0)     \
-  TC_CHUNK(KB, 1)     \
-  TC_CHUNK(KB, 2)     \
-  TC_CHUNK(KB, 3)
-      switch (kb) {
-        case 0: { TC_KBLOCK(0) } break;
-        case 1: { TC_KBLOCK(1) } break;
-        case 2: { TC_KBLOCK(2) } break;
-        default: { TC_KBLOCK(3) } break;
-      }
-#undef TC_KBLOCK
-#undef TC_CHUNK
-      mma_commit(empty0 + 8 * slot);
-      if (kb == P.nkb - 1) {
-        mma_commit(accfull0 + 8 * b);
-        u++;
-      }
-      g++;
-    }
-    // every MMA issued has completed before tensor memory is released
-    mma_commit(drain);
-    if (!mbar_wait(drain, 0)) ok = false;
-    if (!ok) atomicOr(P.err, 2u);
-  }
-  __syncwarp();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == TC_MWARP) {
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TC_ACC_COLS)
-                 : "memory");
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -582,7 +274,8 @@ struct TcgParams {
   int nfull;                  // leading K chunks with all three products (the rest: hi x hi only)
   int nch[TC_MAXCH];
   int choff[TC_MAXCH + 1];
-  uint32_t *err;              // as TcParams::err
+  uint32_t *err;              // [0] bit 0: a producer's wait timed out, bit 1: an MMA-side wait;
+                              // [2..3] class steps issued (u64, for the executed-work count)
 };
 
 __device__ __forceinline__ void tma_box5(uint32_t dst, const CUtensorMap *map, int c1, int c2, int c3, int c4,
@@ -594,9 +287,11 @@ __device__ __forceinline__ void tma_box5(uint32_t dst, const CUtensorMap *map, i
       : "memory");
 }
 
-// Fold of the level-grid kernel: as fold(), with the step's row factor 2^e
-// (one per source level, from shared memory) and the accumulator read 32
-// columns per wait.
+// Adds a class step's accumulator (this thread's lane, HALF columns from col0),
+// times the step's row factor 2^e (one per source level, from shared memory) and
+// the class's column scales, into the FP32 running sums -- rows with a source in
+// the step only -- and hands the accumulator back to the MMA issuer; the
+// accumulator is read 32 columns per wait.
 template <int HALF>
 __device__ __forceinline__ bool fold_g(float *acc, uint32_t tlane, int col0, uint32_t v, bool mine,
                                        uint32_t accfull0, uint32_t accempty0, uint32_t colfull0, int lev,
@@ -1046,26 +741,6 @@ __global__ void k_tc_scatter(const int *tgt, const int *src, const int *cls, lon
   stab[(size_t)st * TC_ROWS + (row % TC_ROWS)] = src[k];
 }
 
-// Source multipoles as 2^e (hi + lo), hi and lo FP16 rows of kpad terms, e per
-// cell from the row's largest magnitude (one warp per cell).
-__global__ void k_tc_split(const float *M, int ncells, int mstr, int msize, int kpad, __half *Mh, __half *Ml,
-                           int *mexp) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= ncells) return;
-  const float *row = M + (size_t)w * mstr;
-  float mx = 0.f;
-  for (int i = lane; i < msize; i += 32) mx = fmaxf(mx, fabsf(row[i]));
-  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const int e = scale_exp(mx);
-  if (lane == 0) mexp[w] = e;
-  for (int i = lane; i < kpad; i += 32) {
-    __half hi, lo;
-    split_f16(i < msize ? row[i] : 0.f, e, hi, lo);
-    Mh[(size_t)w * kpad + i] = hi;
-    Ml[(size_t)w * kpad + i] = lo;
-  }
-}
-
 
 // ---- level-grid operands and schedule ----
 // raster index of every cell within its (complete) level
@@ -1201,13 +876,6 @@ int tc_sm_count() {
   return n;
 }
 
-template <int NOUT> int tc_launch(const TcParams &P, int smem, int grid, cudaStream_t st) {
-  FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tc<NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  fmm_note_launch(), k_m2l_tc<NOUT><<<grid, TC_THREADS, smem, st>>>(P);
-  FMM_CUDA_TRY(cudaGetLastError());
-  return FMM_OK;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -1266,7 +934,7 @@ TcgState *tcg_state(DevTree *t) {
 }
 
 // Schedule, grids and tensor maps of a build whose levels are all complete;
-// eligible = 0 when the tree does not qualify (the row-gather kernel runs).
+// eligible = 0 when the tree does not qualify (the harmonic kernels run).
 int tcg_prepare(DevTree *t, const TcPlan &pl, cudaStream_t st) {
   TcgState *s = tcg_state(t);
   s->serial = t->build_serial;
@@ -1495,13 +1163,12 @@ int fmm_m2l_tc_max_slots(int p, int so) {
 }
 
 // Executed tensor work of one class step of a 128-row tile: MMA instructions
-// and flops (each 2 x 128 x 16 x N): 3 products per K chunk in the row-gather
-// kernel; in the level-grid kernel (boxes) 3 for the leading chunks, 1 for
+// and flops (each 2 x 128 x 16 x N): 3 products for the leading K chunks, 1 for
 // the chunks of degree TCG_SPLIT_DEG and up.
-bool fmm_m2l_tc_step_work(int p, int so, bool boxes, long long *mmas, double *flops) {
+bool fmm_m2l_tc_step_work(int p, int so, long long *mmas, double *flops) {
   TcPlan pl;
   if (!tc_plan(p, so, pl)) return false;
-  const int nfull = boxes ? tcg_full_chunks(pl) : pl.kch;
+  const int nfull = tcg_full_chunks(pl);
   long long m = 0;
   double n = 0;
   for (int k = 0; k < pl.kch; k++) {
@@ -1570,7 +1237,7 @@ int fmm_tc_schedule(DevTree *t, cudaStream_t st) {
   return FMM_OK;
 }
 
-int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStream_t st, bool boxes) {
+int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStream_t st) {
   TcPlan pl;
   if (!tc_plan(t->order, t->so, pl)) return FMM_ERR_ARG;
   const int nc = t->ncells;
@@ -1592,74 +1259,10 @@ int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStr
     t->tc_order = t->order;
     t->tc_so = t->so;
   }
-  // complete levels: source rows by tensor-map box loads from level grids
-  t->tc_boxes_last = 0;
-  if (boxes) {
-    const int rc = tcg_run(t, pl, M, mstr, L, lstr, st);
-    if (rc != FMM_ERR_STATE) {
-      t->tc_boxes_last = rc == FMM_OK;
-      return rc;
-    }
-  }
-  // class-step schedule of the tiles: once per build and cell order
-  const int ntiles = (nc + TC_ROWS - 1) / TC_ROWS;
-  if (int rc = fmm_tc_schedule(t, st)) return rc;
-  const size_t nm = (size_t)nc * pl.kpad;
-  if (fmm_reserve(t->tc_Mh, nm) || fmm_reserve(t->tc_Ml, nm) || fmm_reserve(t->tc_mexp, nc) ||
-      fmm_reserve(t->d_tcerr, 4))
-    return FMM_ERR_CUDA;
-  fmm_note_launch(), k_tc_split<<<fmm_blocks((size_t)nc * 32, 256), 256, 0, st>>>(
-      M, nc, mstr, pl.msize, pl.kpad, (__half *)t->tc_Mh.p, (__half *)t->tc_Ml.p, t->tc_mexp.p);
-  FMM_CUDA_TRY(cudaGetLastError());
-  FMM_CUDA_TRY(cudaMemsetAsync(t->d_tcerr.p, 0, 4 * sizeof(uint32_t), st));
-
-  TcParams P;
-  P.order = t->m2l_order.p;
-  P.ncells = nc;
-  P.ntiles = ntiles;
-  P.sched_off = t->tc_sched_off.p;
-  P.sched_cls = t->tc_sched_cls.p;
-  P.stab = t->tc_stab.p;
-  P.Mh = (const __half *)t->tc_Mh.p;
-  P.Ml = (const __half *)t->tc_Ml.p;
-  P.mexp = t->tc_mexp.p;
-  P.T = t->tc_T.p;
-  P.L = L;
-  P.lstride = lstr;
-  P.lsize = pl.lsize;
-  P.kpad = pl.kpad;
-  P.kch = pl.kch;
-  P.nkb = pl.nkb;
-  // pipeline depth: as many row-gather slots as fit, or fewer when tuned so
-  P.nslots = t->tune.nslots >= 2 ? std::min(pl.nslots, t->tune.nslots) : pl.nslots;
-  const int smem = 1024 + P.nslots * pl.slot_bytes + (int)sizeof(TcShared);
-  P.cls_bytes = pl.cls_bytes;
-  P.cls_scale = pl.cls_scale;
-  P.slot_bytes = pl.slot_bytes;
-  P.nout = pl.nout;
-  for (int k = 0; k < TC_MAXCH; k++) P.nch[k] = k < pl.kch ? pl.nch[k] : 0;
-  for (int k = 0; k <= TC_MAXCH; k++) P.choff[k] = k <= pl.kch ? pl.choff[k] : pl.cls_scale;
-  P.err = t->d_tcerr.p;
-  const int grid = std::min(P.ntiles, tc_sm_count());
-  int rc;
-  if ((rc = fmm_mark_kernel(t, 0, st))) return rc;
-  switch (pl.nout) {
-    case 16: rc = tc_launch<16>(P, smem, grid, st); break;
-    case 32: rc = tc_launch<32>(P, smem, grid, st); break;
-    case 48: rc = tc_launch<48>(P, smem, grid, st); break;
-    case 64: rc = tc_launch<64>(P, smem, grid, st); break;
-    case 96: rc = tc_launch<96>(P, smem, grid, st); break;
-    case 128: rc = tc_launch<128>(P, smem, grid, st); break;
-    case 176: rc = tc_launch<176>(P, smem, grid, st); break;
-    case 224: rc = tc_launch<224>(P, smem, grid, st); break;
-    default: return FMM_ERR_ARG;
-  }
-  if (rc || (rc = fmm_mark_kernel(t, 1, st))) return rc;
-  t->tc_ran = 1;
-  // timeout flags reach the host with the stream (read by fmmgen_tree_times)
-  FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned + FMM_PINNED_TCERR, t->d_tcerr.p, 4 * sizeof(uint32_t),
-                               cudaMemcpyDeviceToHost, st));
-  return FMM_OK;
+  // source rows by tensor-map box loads from level grids
+  const int rc = tcg_run(t, pl, M, mstr, L, lstr, st);
+  t->tc_boxes_last = rc == FMM_OK;
+  return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -1813,49 +1416,37 @@ int fmm_m2l_cm(DevTree *t, const float *M, int mstr, float *L, int lstr, const u
   return rc ? rc : fmm_mark_kernel(t, 1, st);
 }
 
-int fmm_m2l_tp(DevTree *t, const float *M, int mstr, float *L, int lstr, const unsigned char *ord, cudaStream_t st) {
+// key per target in processing order: its list length, longest first
+__global__ void k_h_lengths(const int *off, const int *order, int nc, unsigned *key, unsigned *val) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc) return;
+  const int A = order[i];
+  key[i] = 65535u - (unsigned)min(off[A + 1] - off[A], 65535);
+  val[i] = (unsigned)A;
+}
+
+int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st) {
   const int p = t->order, so = t->so, nc = t->ncells;
-  if (!fmm_m2l_cm_supported(p, so) || (mstr & 3) || p - so > 32) return FMM_ERR_STATE;
-  const int lsize = fmm_nterms(p - so);
-  if (t->nm2l == 0) {
-    FMM_CUDA_TRY(cudaMemset2DAsync(L, sizeof(float) * lstr, 0, sizeof(float) * lsize, nc, st));
-    return FMM_OK;
-  }
-  if (int rc = fmm_m2l_csr(t, st)) return rc;
-  if (ord) {
-    const size_t nbh = fmm_rs_nblocks(nc), hist_n = 256 * nbh;
-    if (fmm_reserve(t->tp_perm, (size_t)t->nm2l) || fmm_reserve(t->tp_tgt, nc) ||
-        fmm_reserve(t->tmp, (size_t)nc * 12 + hist_n * 4 + fmm_scan_tmp_elems<uint32_t>(hist_n) * 4 + 256))
-      return FMM_ERR_CUDA;
-    char *q = t->tmp.p;
-    unsigned *k1 = (unsigned *)q; q += (size_t)nc * 4;
-    unsigned *k2 = (unsigned *)q; q += (size_t)nc * 4;
-    uint32_t *v2 = (uint32_t *)q; q += (size_t)nc * 4;
-    uint32_t *hist = (uint32_t *)q; q += hist_n * 4;
-    uint32_t *stmp = (uint32_t *)q;
+  if (p - so > 32) return FMM_ERR_STATE;
+  if (!ord && t->tgt_serial == t->build_serial && t->tgt_version == t->order_version) return FMM_OK;
+  const size_t nbh = fmm_rs_nblocks(nc), hist_n = 256 * nbh;
+  if (fmm_reserve(t->tp_tgt, nc) || (ord && fmm_reserve(t->tp_perm, (size_t)t->nm2l)) ||
+      fmm_reserve(t->tmp, (size_t)nc * 12 + hist_n * 4 + fmm_scan_tmp_elems<uint32_t>(hist_n) * 4 + 256))
+    return FMM_ERR_CUDA;
+  char *q = t->tmp.p;
+  unsigned *k1 = (unsigned *)q; q += (size_t)nc * 4;
+  unsigned *k2 = (unsigned *)q; q += (size_t)nc * 4;
+  uint32_t *v2 = (uint32_t *)q; q += (size_t)nc * 4;
+  uint32_t *hist = (uint32_t *)q; q += hist_n * 4;
+  uint32_t *stmp = (uint32_t *)q;
+  if (ord)
     fmm_note_launch(), k_tp_perm<<<fmm_blocks((size_t)nc * 32, 256), 256, 0, st>>>(
         t->m2l_off.p, ord, t->m2l_order.p, t->clevel.p, nc, so + 1, p, t->tp_perm.p, k1, (unsigned *)t->tp_tgt.p);
-    FMM_CUDA_TRY(cudaGetLastError());
-    if (int rc = fmm_radix_sort<unsigned>(k1, (uint32_t *)t->tp_tgt.p, k2, v2, nc, 0, 32, hist, stmp, st)) return rc;
-  }
-  TpParams P;
-  P.tgt = ord ? t->tp_tgt.p : t->m2l_order.p;
-  P.ntgt = nc;
-  P.off = t->m2l_off.p;
-  P.src = t->m2l_src.p;
-  P.cls = t->m2l_cls.p;
-  P.perm = ord ? t->tp_perm.p : nullptr;
-  P.ord = ord;
-  P.p = p;
-  P.D = (const float *)t->cls_Df.p;
-  P.dstr = fmm_stride4(fmm_nterms(p));
-  P.clevel = t->clevel.p;
-  P.M = M;
-  P.mstr = mstr;
-  P.L = L;
-  P.lstr = lstr;
-  P.lsize = lsize;
-  int rc = fmm_mark_kernel(t, 0, st);
-  if (!rc) rc = fmm_m2l_tp_launch(so, P, st);
-  return rc ? rc : fmm_mark_kernel(t, 1, st);
+  else
+    fmm_note_launch(), k_h_lengths<<<fmm_blocks(nc, 256), 256, 0, st>>>(t->m2l_off.p, t->m2l_order.p, nc, k1,
+                                                                        (unsigned *)t->tp_tgt.p);
+  FMM_CUDA_TRY(cudaGetLastError());
+  t->tgt_serial = ord ? ~0ull : t->build_serial;
+  t->tgt_version = t->order_version;
+  return fmm_radix_sort<unsigned>(k1, (uint32_t *)t->tp_tgt.p, k2, v2, nc, 0, ord ? 32 : 16, hist, stmp, st);
 }

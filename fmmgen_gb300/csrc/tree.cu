@@ -1148,6 +1148,7 @@ void fmm_tree_destroy(DevTree *t) {
   fmm_release(t->child_mask); fmm_release(t->clevel); fmm_release(t->leaf_cells); fmm_release(t->cell_leaf);
   fmm_release(t->m2l_off); fmm_release(t->m2l_src); fmm_release(t->m2l_cls); fmm_release(t->m2l_order);
   fmm_release(t->m2l_cls_raw);
+  fmm_release(t->hM); fmm_release(t->hL); fmm_release(t->hD);
   t->csr_serial = ~0ull;
   fmm_release(t->p2p_off); fmm_release(t->p2p_src);
   fmm_release(t->cls_key4); fmm_release(t->cls_D); fmm_release(t->cls_Df); fmm_release(t->cls_table);
@@ -1158,7 +1159,7 @@ void fmm_tree_destroy(DevTree *t) {
   fmm_release(t->fa); fmm_release(t->fb); fmm_release(t->fa2); fmm_release(t->fb2);
   fmm_release(t->m2l_tgt_raw); fmm_release(t->m2l_src_raw);
   fmm_release(t->p2p_tgt_raw); fmm_release(t->p2p_src_raw);
-  fmm_release(t->tc_T); fmm_release(t->tc_Mh); fmm_release(t->tc_Ml); fmm_release(t->tc_mexp);
+  fmm_release(t->tc_T);
   fmm_release(t->d_tcerr);
   fmm_release(t->tc_sched_off); fmm_release(t->tc_sched_cls); fmm_release(t->tc_bitmap); fmm_release(t->tc_rank);
   fmm_release(t->tc_stab); fmm_release(t->tc_pos); fmm_release(t->cm_otab);

@@ -2,12 +2,11 @@
 // M2L is one OpenMP loop, example/calculate.cpp:190-206).
 //
 // Candidates, for the tree's order and source order:
-//   implementation: tensor cores (p <= 9) with source rows gathered row by row
-//                   or (trees whose levels are all complete) boxed from level
-//                   grids, generated CUDA-core kernels (orders that have them),
-//                   class-major and target-major generated CUDA-core kernels
-//                   (every order up to 12), warp contraction engine;
-//   tensor-core pipeline depth: 2 .. the row-gather slots that fit in shared memory;
+//   implementation: the harmonic kernels; in mixed passes the generated
+//                   CUDA-core kernels (orders that have them), the class-major
+//                   ones, and on trees whose levels are all complete the tensor
+//                   cores (p <= 9); the warp contraction engine;
+//   tensor-core pipeline depth: 2 .. the operand slots that fit in shared memory;
 //   tensor cores alone, or overlapped with the P2P (in 4- or 2-warp blocks);
 //   grouping of the cells into tiles / warps: by octant within the parent, or Morton.
 // One evaluation pass computes the multipoles and stages the particles; then
@@ -32,20 +31,17 @@ int fmm_autotune(DevTree *t, const double *S, int precision, int reps, int max_c
   const int maxs = fmm_m2l_tc_max_slots(t->order, t->so);
   const bool gen = fmm_m2l_gen_supported(t->order, t->so);
   const bool cm = fmm_m2l_cm_supported(t->order, t->so) && t->nclasses <= 262144;
-  const bool tp = fmm_m2l_cm_supported(t->order, t->so);
   const bool boxes = precision != 0 && maxs > 0 && fmm_m2l_tc_boxes_ok(t, st);
   for (int g = 0; g < 2; g++) {
     if (precision != 0) {
-      for (int ov = 0; ov < 3; ov++)
-        for (int s = 2; s <= maxs; s++) {
-          cands.push_back({0, s, g, ov});
-          // level-grid boxes (their tiles do not depend on the grouping)
-          if (g == 0 && boxes) cands.push_back({3, s, g, ov});
-        }
+      if (g == 0 && boxes)  // (their tiles do not depend on the grouping)
+        for (int ov = 0; ov < 3; ov++)
+          for (int s = 2; s <= maxs; s++) cands.push_back({3, s, g, ov});
       if (gen) cands.push_back({1, 0, g, 0});
       if (cm) cands.push_back({4, 0, g, 0});
-      if (tp) cands.push_back({5, 0, g, 0});
     }
+    // the harmonic kernels, by a number that set_tune takes for this order and source order
+    cands.push_back({maxs > 0 ? 0 : cm ? 5 : -1, 0, g, 0});
     cands.push_back({2, 0, g, 0});
   }
   // one pass for the multipoles (the field into a scratch output)

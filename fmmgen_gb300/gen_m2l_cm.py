@@ -25,18 +25,11 @@ unrolled body outgrows the SM's instruction cache stalls on instruction fetch
 instructions).  An output group's chunks are split over several kernels; the
 first stores the group's outputs, the others add to them.
 
-Two schedules of the pairs:
-  class-major (k_m2l_cm_*): the tiles of the tensor-core path's class-step
-      schedule (128 target cells in M2L processing order; a step gives every
-      row its source of one class, or none), one warp per 32 rows walking the
-      steps that have a pair in its rows.  The class's derivative vector is
-      the same for the whole warp: it is staged once in shared memory and read
-      as broadcasts.
-  target-major (k_m2l_tp_*): one thread per target cell walking its own pair
-      list (by descending order when orders are per pair, so a warp's lanes
-      reach pairs of similar order together); the lanes read their own
-      classes' derivative vectors through the L1 cache.  No lane idles on a
-      class its target does not have -- the better schedule on adaptive trees.
+The pairs go class by class (k_m2l_cm_*): the tiles of the tensor-core path's
+class-step schedule (128 target cells in M2L processing order; a step gives every
+row its source of one class, or none), one warp per 32 rows walking the steps
+that have a pair in its rows.  The class's derivative vector is the same for the
+whole warp: it is staged once in shared memory and read as broadcasts.
 
 Run:  python -m fmmgen_gb300.gen_m2l_cm   (build.py runs it when this file changes)
 """
@@ -60,7 +53,6 @@ RMAX = 208              # register estimate per thread an output group may reach
 OVERHEAD = 32           # registers besides accumulators, temporaries and the chunk
 PARTIAL_MIN_TERMS = 21  # outputs with at least this many terms per pair (in a kernel) sum per pair first
 ROWS = 128              # threads of a block (class-major: rows of a schedule tile)
-TP_PREFETCH_QUADS = 2   # target-major: operator quads of the next degree block loaded a block ahead
 MIN_BLOCKS = 2          # resident blocks per SM the register allocation must allow
 
 
@@ -152,12 +144,9 @@ def plan(so, pmax):
 COMP = "xyzw"
 
 
-def chunk_body(so, pmax, c, kern, srcexpr, dload, ind, prefetch_quads=0):
+def chunk_body(so, pmax, c, kern, srcexpr, dload, ind):
     """Multiply one staged chunk: its multipole terms from shared memory
-    (scaled by the level difference), the terms nested by degree; with
-    prefetch_quads, each degree block first loads that many of the next
-    block's operator quads (global loads, whose latency the block's own
-    multiply-adds then cover)."""
+    (scaled by the level difference), the terms nested by degree."""
     mono = monomials(pmax)
     moff = nterms(so - 1)
     i0 = kern["outs"][0]
@@ -184,37 +173,12 @@ def chunk_body(so, pmax, c, kern, srcexpr, dload, ind, prefetch_quads=0):
     for t in c["terms"]:
         by_d.setdefault(t[0], []).append(t)
     dlo, dhi = min(by_d), max(by_d)
-    # the quads each degree block loads first, in order of use
-    first = {}
-    seen = set()
-    for d in range(dlo, dhi + 1):
-        first[d] = []
-        for (_, k, i, jj) in by_d.get(d, []):
-            if k // 4 not in seen:
-                seen.add(k // 4)
-                first[d].append(k // 4)
     depth = 0
     loaded = set()
-
-    def prefetch(d, ii, guard):
-        # the first quads of block d, loaded a block ahead (warp-uniform: d <= qmax <= the pass's order,
-        # so every load stays inside the class's row)
-        for kq in first.get(d, [])[:prefetch_quads]:
-            if guard:
-                L.append(ii + f"float4 dq{kq} = make_float4(0.f, 0.f, 0.f, 0.f);")
-                L.append(ii + f"if (qmax >= {d}) dq{kq} = {dload(kq)};")
-            else:
-                L.append(ii + f"const float4 dq{kq} = {dload(kq)};")
-            loaded.add(kq)
-
-    if prefetch_quads:
-        prefetch(dlo, ind, False)  # the chunk runs only when qmax reaches its lowest degree
     for d in range(dlo, dhi + 1):
         L.append(ind + "  " * depth + f"if (ql >= {d}) {{")
         depth += 1
         ii = ind + "  " * depth
-        if prefetch_quads and d < dhi:
-            prefetch(d + 1, ii, True)
         for (_, k, i, jj) in by_d.get(d, []):
             kq = k // 4
             if kq not in loaded:
@@ -245,7 +209,7 @@ def stage_chunk(c, chq, chb, bufexpr, bvar, ind):
             ind + "}"]
 
 
-def pipeline(so, pmax, kern, chq, chb, dload, prefetch_next, ind, prefetch_quads=0):
+def pipeline(so, pmax, kern, chq, chb, dload, prefetch_next, ind):
     """The chunks of one pair (or step): chunk j+1 staged while j is multiplied;
     after the last, prefetch_next(ind) stages the next pair's first chunk."""
     chunks = kern["chunks"]
@@ -264,7 +228,7 @@ def pipeline(so, pmax, kern, chq, chb, dload, prefetch_next, ind, prefetch_quads
         L.append(ind + "  }")
         L.append(ind + "  __syncwarp();")
         L.extend(chunk_body(so, pmax, c, kern, f"sbuf + ((base + {ci}) & 1) * {chb} + lane * {chq + 1}", dload,
-                            ind + "  ", prefetch_quads))
+                            ind + "  "))
         L.append(ind + "  __syncwarp();  // the buffer is refilled two chunks on")
         L.append(ind + "}")
     return L
@@ -404,92 +368,6 @@ def emit_cm(so, pmax, ki, kern):
     return name, dmin, 4 * (2 * chb + 2 * dq) * 16, "\n".join(L)
 
 
-def emit_tp(so, pmax, ki, kern):
-    chq = CH // 4
-    chb = 32 * (chq + 1)
-    i0 = kern["outs"][0]
-    temps = set(kern["temps"])
-    dmin = kernel_dmin(kern)
-    name = f"k_m2l_tp_s{so}_p{pmax}_k{ki}"
-    L = header_lines(kern, name, so, pmax, "TpParams", "")
-    L.append(f"  float4 *const sbuf = cm_smem + w * {2 * chb};")
-    L.append(f"  const int t = blockIdx.x * {ROWS} + threadIdx.x;")
-    L.append("  const bool act = t < P.ntgt;")
-    L.append("  const int A = act ? (P.tgt ? P.tgt[t] : t) : -1;")
-    L.append("  const int la = act ? (int)P.clevel[A] : 0;")
-    L.append("  const int k0 = act ? P.off[A] : 0;")
-    L.append("  const int n = act ? P.off[A + 1] - k0 : 0;")
-    L.append("  const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)n);")
-    for i in kern["outs"]:
-        L.append(f"  float a{i - i0} = 0.f;")
-    L.append("  const int mq = P.mstr >> 2;")
-    L.append("  // a lane's pairs (by descending order when orders are per pair): the current one (staged), the")
-    L.append("  // next (slots loaded a pair ahead, its row staged during this pair) and the list index of the one after")
-    L.append("#define TP_PAIR(jj) ((jj) < n ? (P.perm ? P.perm[k0 + (jj)] : k0 + (jj)) : -1)")
-    L.append(f"#define TP_ORD(kk) ((kk) >= 0 ? (P.ord ? min(max((int)P.ord[kk], {so + 1}), P.p) : P.p) : -1)")
-    L.append("  const int kc0 = TP_PAIR(0);")
-    L.append("  int Bc = kc0 >= 0 ? P.src[kc0] : -1, qc = TP_ORD(kc0), cc = kc0 >= 0 ? P.cls[kc0] : 0;")
-    L.append("  const int kn0 = TP_PAIR(1);")
-    L.append("  int Bn = kn0 >= 0 ? P.src[kn0] : -1, qn = TP_ORD(kn0), cn = kn0 >= 0 ? P.cls[kn0] : 0;")
-    L.append("  int k2 = TP_PAIR(2);")
-    L.append("  bool pf = false;  // the current pair's first chunk is staged")
-    L.append("  int base = 0;")
-    L.append("  for (int j = 0; j < nmax; j++) {")
-    L.append("    const int k3 = TP_PAIR(j + 3);")
-    L.append("    const int B2 = k2 >= 0 ? P.src[k2] : -1, q2 = TP_ORD(k2), c2 = k2 >= 0 ? P.cls[k2] : 0;")
-    L.append(f"    const bool on = qc >= {dmin};")
-    L.append("    // no lane has terms here: with pairs by descending order none has any further on")
-    L.append("    if (!__any_sync(0xffffffffu, on)) break;")
-    L.append("    const int ql = on ? qc : -1;")
-    L.append("    const int qmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)(on ? ql : 0));")
-    L.append("    const int B = on ? Bc : -1;")
-    L.append("    const int dl = on ? la - (int)P.clevel[B] : 0;")
-    L.append("    const float *__restrict__ Dp = P.D + (size_t)(on ? cc : 0) * P.dstr;")
-    L.append(f"    const int nch = {nch_expr(kern)};")
-    L.append("    bool pfn = false;")
-    L.append("    if (!pf) {")
-    L.extend(stage_chunk(kern["chunks"][0], chq, chb, "base", "B", "      "))
-    L.append("      cm_cp_async_commit();")
-    L.append("    }")
-    for i in kern["outs"]:
-        if i in temps:
-            L.append(f"    float t{i - i0} = 0.f;")
-
-    def prefetch_next(ind):
-        return [ind + f"const bool onn = qn >= {dmin};",
-                ind + "pfn = __any_sync(0xffffffffu, onn);",
-                ind + "if (pfn) {",
-                ind + "  const int Bnn = onn ? Bn : -1;"] + \
-            stage_chunk(kern["chunks"][0], chq, chb, "(base + nch) & 1", "Bnn", ind + "  ") + \
-            [ind + "  cm_cp_async_commit();",
-             ind + "  cm_cp_async_wait<1>();",
-             ind + "} else {",
-             ind + "  cm_cp_async_wait<0>();",
-             ind + "}"]
-
-    L.extend(pipeline(so, pmax, kern, chq, chb, lambda kq: f"__ldg((const float4 *)(Dp + {4 * kq}))",
-                      prefetch_next, "    ", TP_PREFETCH_QUADS))
-    for i in kern["outs"]:
-        if i in temps:
-            L.append(f"    a{i - i0} += t{i - i0};")
-    L.append("    base = (base + nch) & 1;")
-    L.append("    pf = pfn;")
-    L.append("    Bc = Bn;")
-    L.append("    qc = qn;")
-    L.append("    cc = cn;")
-    L.append("    Bn = B2;")
-    L.append("    qn = q2;")
-    L.append("    cn = c2;")
-    L.append("    k2 = k3;")
-    L.append("  }")
-    L.append("#undef TP_PAIR")
-    L.append("#undef TP_ORD")
-    L.append("  if (!act) return;")
-    L.extend(store_lines(kern))
-    L.append("}")
-    return name, dmin, 4 * 2 * chb * 16, "\n".join(L)
-
-
 def launcher(fname, params, so, pmax, table, grid):
     L = [f"int {fname}(const {params} &P, cudaStream_t st) {{",
          f"  if (P.p > {pmax} || P.p < {so + 1} || (P.mstr & 3) || (P.dstr & 3)) return FMM_ERR_ARG;",
@@ -510,19 +388,14 @@ def generate_family(so, pmax):
     kernels = plan(so, pmax)
     out = os.path.join(CSRC, family_file(so, pmax))
     parts = [f"// {family_file(so, pmax)} -- generated by fmmgen_gb300/gen_m2l_cm.py; do not edit.",
-             f"// FP32 M2L kernels, source order {so}, orders {so + 1}..{pmax}: class-major (k_m2l_cm_*) and",
-             "// target-major (k_m2l_tp_*) schedules of the same kernel bodies.",
+             f"// FP32 M2L kernels, source order {so}, orders {so + 1}..{pmax}, class-major schedule.",
              '#include "m2l_cm.cuh"', ""]
-    tcm, ttp = [], []
+    tcm = []
     for ki, kern in enumerate(kernels):
         name, dmin, smem, code = emit_cm(so, pmax, ki, kern)
         parts += [code, ""]
         tcm.append((name, dmin, smem))
-        name, dmin, smem, code = emit_tp(so, pmax, ki, kern)
-        parts += [code, ""]
-        ttp.append((name, dmin, smem))
-    parts += launcher(f"fmm_m2l_cm_s{so}_p{pmax}", "CmParams", so, pmax, tcm, "P.ncells") + [""]
-    parts += launcher(f"fmm_m2l_tp_s{so}_p{pmax}", "TpParams", so, pmax, ttp, "P.ntgt")
+    parts += launcher(f"fmm_m2l_cm_s{so}_p{pmax}", "CmParams", so, pmax, tcm, "P.ncells")
     with open(out, "w") as f:
         f.write("\n".join(parts) + "\n")
     return out
@@ -552,23 +425,6 @@ struct CmParams {
   int lstr, lsize;
 };
 
-// target-major schedule: a thread per target cell over its target list
-struct TpParams {
-  const int *tgt;               // [ntgt] target cells (null: cells 0 .. ntgt - 1)
-  int ntgt;
-  const int *off, *src, *cls;   // target lists: pairs of cell A are off[A] .. off[A + 1] - 1
-  const int *perm;              // pair indices of each list by descending order, or null (list order)
-  const unsigned char *ord;     // per-pair orders (list order, needs perm), or null: every pair at order p
-  int p;
-  const float *D;
-  int dstr;
-  const unsigned char *clevel;
-  const float *M;
-  int mstr;
-  float *L;
-  int lstr, lsize;
-};
-
 static __device__ __forceinline__ void cm_cp_async16(void *dst, const void *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\\n" :: "r"(d), "l"(src) : "memory");
@@ -587,14 +443,13 @@ def generate():
     for so, pmax in FAMILIES:
         outs.append(generate_family(so, pmax))
         decl.append(f"int fmm_m2l_cm_s{so}_p{pmax}(const CmParams &P, cudaStream_t st);  // orders {so + 1}..{pmax}")
-        decl.append(f"int fmm_m2l_tp_s{so}_p{pmax}(const TpParams &P, cudaStream_t st);")
     fams = sorted(FAMILIES, key=lambda f: (f[0], f[1]))
     table = ["// largest order of the families of each source order (0: none)",
              "static inline int fmm_m2l_cm_pmax(int so) {"]
     for so in sorted({f[0] for f in fams}):
         table.append(f"  if (so == {so}) return {max(pm for s_, pm in fams if s_ == so)};")
     table += ["  return 0;", "}"]
-    for kind, params in (("cm", "CmParams"), ("tp", "TpParams")):
+    for kind, params in (("cm", "CmParams"),):
         table += [f"// launch the family of source order so with the smallest largest order >= P.p (FMM_ERR_STATE: none)",
                   f"static inline int fmm_m2l_{kind}_launch(int so, const {params} &P, cudaStream_t st) {{"]
         for so, pmax in fams:

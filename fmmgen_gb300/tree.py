@@ -224,14 +224,17 @@ class Tree:
         return self
 
     # -- M2L choices and the autotuner (no counterpart in the reference) -------
-    M2L_IMPLS = {-1: "default", 0: "tensor cores", 1: "generated CUDA-core kernels", 2: "contraction engine"}
+    M2L_IMPLS = {-1: "default", 0: "default", 1: "generated CUDA-core kernels", 2: "contraction engine",
+                 3: "tensor cores, level grids", 4: "class-major CUDA-core kernels", 5: "harmonic kernels"}
 
     def set_tune(self, impl=-1, nslots=0, grouping=0, overlap=0):
-        """M2L implementation (-1 default rules, 0 tensor cores with source rows
-        gathered row by row, 1 generated CUDA-core kernels, 2 contraction
-        engine, 3 tensor cores with source rows boxed from level grids where
-        every level is complete, else as 0, 4 class-major and 5 target-major
-        CUDA-core kernels; per-pair orders run on 5 unless 2 or 4 is chosen),
+        """M2L implementation (-1 and 0 the default, as 5; 1 generated CUDA-core
+        kernels, 2 contraction engine, 3 tensor cores with source rows boxed
+        from level grids where every level is complete, 4 class-major CUDA-core
+        kernels,
+        5 kernels over harmonic coefficients, a thread per target cell;
+        per-pair orders and FP64 passes run on 5 unless 2 is chosen, or 4 for
+        orders),
         tensor-core pipeline depth
         (0: as deep as fits), cell grouping (0 by octant, 1 Morton) and
         overlap (1 / 2: tensor-core M2L and P2P side by side on the SMs, the

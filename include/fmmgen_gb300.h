@@ -238,24 +238,22 @@ int fmmgen_tree_kernel_ms(fmmgen_tree *tree, float *ms2);
 /* Work of the last tensor-core M2L (no counterpart in the reference; for
  * roofline accounting), host out4 = [class steps of 128-row tiles, tcgen05 MMA
  * instructions, executed tensor flops, 1 if its source rows were boxed from
- * level grids (else gathered row by row)]; zeros if none ran. */
+ * level grids]; zeros if none ran. */
 int fmmgen_tree_m2l_work(fmmgen_tree *tree, double *out4);
 
 /* ---- M2L choices and their autotuner (no counterpart in the reference) ----
- * impl: -1 the default rules (tensor cores for "mixed" where p <= 9 -- as
- * impl 3 --, else the generated CUDA-core kernels where the order has them:
- * impl 1, then impl 5, else the warp contraction engine), 0 tensor cores with the source rows
- * gathered row by row, 1 generated CUDA-core kernels, 2 contraction engine,
- * 3 tensor cores with the source rows boxed from dense level grids by
- * tensor-map copies where every level of the tree is complete (one system,
- * all 8^l cells of every level), else as 0, 4 class-major CUDA-core kernels
- * (a warp takes 32 target cells' pairs of one translation class per step),
- * 5 target-major CUDA-core kernels (a thread per target cell over its list);
- * 4 and 5 cover orders up to 12 for charges, 8 for dipoles (mixed passes;
- * FP64 passes always use the engine).  Per-pair M2L orders
- * (fmmgen_tree_set_m2l_orders, an order model) run in mixed passes on the
- * target-major kernels, on the class-major ones with impl 4, on the engine
- * with impl 2 or where the kernels do not cover the order.
+ * impl: -1 and 0 the default (impl 5, whatever the source order and
+ * precision; 0 is accepted for the orders of impl 3), 1 generated CUDA-core
+ * kernels, 2 contraction engine, 3 tensor cores with the source rows boxed
+ * from dense level grids by tensor-map copies where every level of the tree is
+ * complete (one system, all 8^l cells of every level), else the default,
+ * 4 class-major CUDA-core kernels (a warp takes 32 target cells' pairs of one
+ * translation class per step), 5 the kernels over harmonic coefficients (a
+ * thread per target cell over a share of its list).  4 and 5 can be chosen for
+ * orders up to 12 for charges, 8 for dipoles.  FP64 passes run 5, or the
+ * engine with impl 2.  Per-pair M2L orders (fmmgen_tree_set_m2l_orders, an
+ * order model) run on 5, on the class-major kernels with impl 4 (mixed
+ * passes), on the engine with impl 2.
  * nslots: tensor-core pipeline depth (operand slots), 0 = as many as fit.
  * grouping: order of a level's cells in M2L tiles and warps, 0 by octant
  * within the parent, 1 Morton.  overlap: 1 (2) runs the tensor-core M2L on a
