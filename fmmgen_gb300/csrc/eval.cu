@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(32 * L2P_WARPS) k_l2p(const int *leaf_cells, i
 }
 
 // P2P and the FP32 staging live in p2p.cu
-int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st, bool narrow = false);
+int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st);
 int fmm_stage_particles(DevTree *t, const double *S, cudaStream_t st);
 
 // F[caller index][outsize] = near + far, in FP64
@@ -739,7 +739,7 @@ static int m2l_p2p(DevTree *t, const PlanSet *ps, const double *S, const T *M, T
   TRY(m2l_phase<T>(t, ps, M, L, mixed, impl, mstr, lstr, dstr, t->s_hi));
   TRY(rec(t, 3, t->s_hi));
   FMM_CUDA_TRY(cudaEventRecord(t->ev_join, t->s_hi));
-  TRY(fmm_p2p_launch(t, mixed, S, st, t->tune.overlap == 2));
+  TRY(fmm_p2p_launch(t, mixed, S, st));
   FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
   return rec(t, 4, st);
 }
@@ -1003,7 +1003,7 @@ static int fused_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_c, 0));
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_s, 0));
     if (!t->tune.overlap && mixed && is_tc(impl)) FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
-    TRY(fmm_p2p_launch(t, mixed, S, st, mixed && is_tc(impl) && t->tune.overlap == 2));
+    TRY(fmm_p2p_launch(t, mixed, S, st));
   }
   FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
   TRY(rec(t, 4, st));

@@ -53,6 +53,7 @@ struct DevTree {
   DevBuf<uint32_t> perm, perm2;           // sorted position -> caller's particle index
   DevBuf<double> px, py, pz;              // sorted positions (FP64)
   DevBuf<float4> phi4, plo4, sdip;        // FP32 P2P staging: (hi offset from root centre, q), (lo, index), dipole
+  DevBuf<float4> lorg;                    // per leaf: origin of its frame in FP32, a coordinate outside the root cube
   DevBuf<float2> levf;                    // per-level half-width as an FP32 (hi, lo) pair
   // cells, level-major, Morton order within a level
   DevBuf<double> cx, cy, cz;
@@ -86,6 +87,8 @@ struct DevTree {
   cudaEvent_t ev_m = nullptr, ev_c = nullptr, ev_p = nullptr, ev_s = nullptr, ev_l = nullptr;
   int grouping_built = 0;                 // grouping m2l_order holds
   DevBuf<int> p2p_off, p2p_src;
+  DevBuf<int4> p2p_units;                 // near-field units: (cell, first target, targets <= 32, leaf)
+  int np2p_units = 0;
   // M2L translation classes: operator vectors D^(k)(d/s_target), |k| <= order
   DevBuf<int> cls_key4;                   // [nclasses][4]: dlev, dx, dy, dz
   DevBuf<double> cls_D;                   // [nclasses][Nterms(order)]

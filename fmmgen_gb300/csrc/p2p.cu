@@ -186,16 +186,23 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int *leaf_cells,
 
 // Per evaluate: positions as two-float offsets from the particle's system root
 // centre (hi in .xyz, the charge in .w; lo in .xyz, the particle's own index
-// in .w for the self test); dipole moments in FP32.
+// in .w for the self test); dipole moments in FP32; per leaf the origin of its
+// frame -- its centre's offset from the root centre, rounded to FP32: as a
+// frame any value near the centre will do, and this one is exact -- and, in .w,
+// a coordinate outside the root cube in both frames.
 __global__ void k_stage_particles(const int *leaf_cells, int nleaves, const int *pstart, const int *pcount,
-                                  const int *csys, const double *roots, const double *px, const double *py,
-                                  const double *pz, const uint32_t *perm, const double *S, int so, float4 *phi4,
-                                  float4 *plo4, float4 *sdip) {
+                                  const int *csys, const double *roots, const double *cx, const double *cy,
+                                  const double *cz, const double *px, const double *py, const double *pz,
+                                  const uint32_t *perm, const double *S, int so, float4 *phi4, float4 *plo4,
+                                  float4 *sdip, float4 *lorg) {
   int leaf = blockIdx.x;
   if (leaf >= nleaves) return;
   int c = leaf_cells[leaf];
   const double *root = roots + 4 * (size_t)csys[c];
   const double ox = root[0], oy = root[1], oz = root[2];
+  if (threadIdx.x == 0)
+    lorg[leaf] = make_float4((float)(cx[c] - ox), (float)(cy[c] - oy), (float)(cz[c] - oz),
+                             root[3] > 0 ? 3.f * (float)root[3] : 1.f);
   for (int j = threadIdx.x; j < pcount[c]; j += blockDim.x) {
     int i = pstart[c] + j;
     double dx = px[i] - ox, dy = py[i] - oy, dz = pz[i] - oz;
@@ -212,25 +219,44 @@ __global__ void k_stage_particles(const int *leaf_cells, int nleaves, const int 
 // ---------------------------------------------------------------------------
 // P2P in FP32 with compensated accumulation (mixed precision)
 // ---------------------------------------------------------------------------
-// One warp per target leaf, in chunks of up to 32 target particles.  The
-// source particles of the leaf's P2P list are taken as one stream -- the
-// concatenation of the source leaves' particle ranges, up to 32 leaves at a
-// time -- and staged in full chunks of 32, so that the per-chunk work (finding
-// each lane's source through a prefix sum of the leaves' counts, the staging
-// copy, the compensated fold) is spread over 32 sources rather than one leaf's
-// ~30.  A chunk of m targets uses f = the largest power of two with f*m <= 32
-// lanes per target, each lane taking every f-th source, so a small chunk (a
-// leaf's last few particles) does not leave most lanes idle; the f partial sums
-// of a target are combined with shuffles.
-// Positions are two-float offsets from the system's root centre: the high
-// parts of two nearby particles subtract exactly (Sterbenz) or with one
-// rounding of the difference, and the low parts carry the rest, so the
-// displacement keeps ~1e-7 relative accuracy even for very close pairs.  Each
-// chunk's contribution is summed in FP32 and folded into a Kahan-compensated
-// FP32 total; the final per-particle near + far sum is FP64 (k_finalize).
-// 1/R is the hardware approximation (relative error ~1e-7, the size of the
-// FP32 displacement's own rounding).  The potential is summed only when it is
-// an output.
+// Bound by the FP32 pipe: an add, multiply or FMA on two packed sources takes
+// it two clocks, so what counts is operations per interaction and full lanes.
+//
+// One warp (a block) takes a chunk of 32 targets of a leaf, or its last m < 32.
+// A lane holds two targets, so that a staged source read from shared memory
+// serves both; two lanes share them when m > 16, four when m > 8, else eight,
+// each taking its share of the sources.  The source particles of the leaf's P2P
+// list are one stream -- the leaves' particle ranges one after the other, up to
+// 32 leaves at a time -- staged in chunks of 64, a lane finding and storing two
+// consecutive ones (in chunks of 32, a source per lane, the staging was 40 % of
+// the instructions), the last chunk filled up with chargeless sources outside
+// the root cube, so that two sources always share an instruction.  The split is a runtime shift and the kernel has two inner
+// loops, near and far: a loop for each split, and one for chunks that may hold
+// the target itself, measured up to twice slower on adaptive trees, waiting
+// for instructions.
+//
+// Displacements: positions are two-float offsets from the system's root
+// centre; the high parts of two nearby particles subtract exactly (Sterbenz)
+// or with one rounding, and the low parts carry the rest, so the displacement
+// keeps ~1e-7 relative accuracy even for very close pairs (three operations
+// per axis).  A source leaf at least a target-leaf width away from the target
+// leaf does not need that: its particles are staged as one FP32 number per
+// axis in the target leaf's frame, where coordinates are at most ~2.5 times
+// the distance, and one subtraction gives the displacement as accurately as
+// FP32 holds it.  On a uniform tree that is 83 % of the sources; 12 instead of
+// 18 FP32 operations per interaction, and half the shared-memory reads.
+//
+// Each chunk's contribution is summed in FP32 and folded into a
+// Kahan-compensated FP32 total; the final per-particle near + far sum is FP64
+// (k_finalize).  1/R is the hardware approximation (relative error ~1e-7, the
+// size of the FP32 displacement's own rounding).  The potential is summed only
+// when it is an output.
+// Measured (one GB300, kernel alone, before and after): 10^6 uniform charges, 30
+// per leaf, field: 4.15 -> 3.1 ms (63 % of the FP32 pipe's cycles); 3x10^5, 73 per
+// leaf: 3.54 -> 2.0; 2x10^6 clustered: 16.4 -> 11.2; 2x10^6 Plummer dipoles, 18 per
+// leaf: 13.4 -> 10.9; 10^4, 20 per leaf: 0.19 -> 0.11.  Median field error against
+// FP64 over uniform, clustered and Plummer systems: 1.46-1.78e-7 before,
+// 1.46-1.60e-7 after (dipoles 2.02-2.05e-7 and 1.99-2.05e-7).
 __device__ __forceinline__ float rsqrt_approx(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -242,54 +268,28 @@ __device__ __forceinline__ void kahan_add(float &s, float &c, float v) {
   c = (t - s) - y;
   s = t;
 }
-
-template <bool SELF, bool POT>
-__device__ __forceinline__ void coulomb_one(const float4 &q, const float4 &ql, int i, float txh, float txl, float tyh,
-                                            float tyl, float tzh, float tzl, float &phi, float &ex, float &ey,
-                                            float &ez) {
-  const float dx = (txh - q.x) + (txl - ql.x);
-  const float dy = (tyh - q.y) + (tyl - ql.y);
-  const float dz = (tzh - q.z) + (tzl - ql.z);
-  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  float rinv = rsqrt_approx(r2);
-  if (SELF) rinv = __float_as_int(ql.w) == i ? 0.f : rinv;  // l2 != l1
-  const float qr = q.w * rinv;
-  const float qr3 = qr * (rinv * rinv);
-  if (POT) phi += qr;
-  ex = fmaf(qr3, dx, ex);
-  ey = fmaf(qr3, dy, ey);
-  ez = fmaf(qr3, dz, ez);
+// (s, c) += (s', c') for running sums s - c: the sum of the high parts with
+// its rounding error
+__device__ __forceinline__ void pair_add(float &s, float &c, float s2, float c2) {
+  const float t = s + s2, z = t - s;
+  const float e = (s - (t - z)) + (s2 - z);
+  s = t;
+  c = (c + c2) - e;
 }
-
-template <bool SELF>
-__device__ __forceinline__ void dipole_one(const float4 &q, const float4 &ql, const float4 &d, int i, float txh,
-                                           float txl, float tyh, float tyl, float tzh, float tzl, float &phi,
-                                           float &ex, float &ey, float &ez) {
-  const float dx = (txh - q.x) + (txl - ql.x);
-  const float dy = (tyh - q.y) + (tyl - ql.y);
-  const float dz = (tzh - q.z) + (tzl - ql.z);
-  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  float rinv = rsqrt_approx(r2);
-  if (SELF) rinv = __float_as_int(ql.w) == i ? 0.f : rinv;
-  const float r3 = rinv * rinv * rinv;
-  const float sr = fmaf(d.x, dx, fmaf(d.y, dy, d.z * dz));
-  const float r5 = 3.f * sr * r3 * rinv * rinv;
-  phi -= sr * r3;
-  ex += d.x * r3 - r5 * dx;
-  ey += d.y * r3 - r5 * dy;
-  ez += d.z * r3 - r5 * dz;
+// s - c in FP64.  The conversions are done on the integer pipe: the FP64 pipe
+// would take 20 clocks of the SM for each.
+__device__ __forceinline__ double f2d(float x) {
+  const unsigned b = __float_as_uint(x), e = (b >> 23) & 255u, m = b & 0x7fffffu;
+  const unsigned E = e == 0u ? 0u : e == 255u ? 2047u : e + 896u;
+  return __hiloint2double((int)((b & 0x80000000u) | (E << 20) | (E ? m >> 3 : 0u)), (int)(E ? m << 29 : 0u));
 }
 
 // ---- two sources per instruction (packed FP32x2) ----
-// A full chunk with one lane per target (the common case) runs two sources at a
-// time through add/sub/mul/fma.rn.f32x2: the same operations, in the same
-// precision, as coulomb_one / dipole_one for each source of the pair, with half
-// the instructions (the kernel is issue-bound).  Staged chunks are laid out for
-// this: pair k of sources (2k, 2k+1) is four 16-byte words
+// Pair k of staged sources (2k, 2k + 1) is four 16-byte words
 //   X[k] = (xh, xh', yh, yh'), Z[k] = (zh, zh', q, q'),
 //   XL[k] = (xl, xl', yl, yl'), ZL[k] = (zl, zl', index, index'),
 // and for dipoles D[k] = (mx, mx', my, my'), DZ[k] = (mz, mz', -, -)
-// (primes: source 2k + 1).
+// (primes: source 2k + 1); far sources leave XL and ZL unused.
 typedef unsigned long long u64;
 __device__ __forceinline__ u64 padd(u64 a, u64 b) {
   u64 d;
@@ -317,245 +317,247 @@ __device__ __forceinline__ u64 pk2(float a, float b) {
 __device__ __forceinline__ float plo(u64 v) { return __uint_as_float((unsigned)v); }
 __device__ __forceinline__ float phi_(u64 v) { return __uint_as_float((unsigned)(v >> 32)); }
 
-// staged chunk of one warp (32 sources)
+// staged chunk of one warp (64 sources)
 struct P2PStage {
-  ulonglong2 X[16], Z[16], XL[16], ZL[16];
+  ulonglong2 X[32], Z[32], XL[32], ZL[32];
 };
 struct P2PStageD {
-  ulonglong2 D[16], DZ[16];
+  ulonglong2 D[32], DZ[32];
 };
-__device__ __forceinline__ float *sf(ulonglong2 *a) { return (float *)a; }
-__device__ __forceinline__ const float *sf(const ulonglong2 *a) { return (const float *)a; }
-
-// the target's coordinates (hi, lo) duplicated into both halves
-struct P2PTgt {
-  u64 xh, xl, yh, yl, zh, zl;
+// One of the lane's two targets.
+struct P2PTarget {
+  int i;
+  float hx, hy, hz, lx, ly, lz;    // offset from the root centre
+  float tx, ty, tz;                // in the leaf's frame
+  float s0 = 0, s1 = 0, s2 = 0, s3 = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
 };
 
-template <bool SELF, bool POT>
-__device__ __forceinline__ void coulomb_two(const P2PStage &sg, int k, int i, const P2PTgt &t, u64 &phi, u64 &ex,
-                                            u64 &ey, u64 &ez) {
-  const ulonglong2 X = sg.X[k], Z = sg.Z[k], XL = sg.XL[k], ZL = sg.ZL[k];
-  const u64 dx = padd(psub(t.xh, X.x), psub(t.xl, XL.x));
-  const u64 dy = padd(psub(t.yh, X.y), psub(t.yl, XL.y));
-  const u64 dz = padd(psub(t.zh, Z.x), psub(t.zl, ZL.x));
-  const u64 r2 = pfma(dx, dx, pfma(dy, dy, pmul(dz, dz)));
-  float ra = rsqrt_approx(plo(r2)), rb = rsqrt_approx(phi_(r2));
-  if (SELF) {  // l2 != l1
-    ra = (int)(unsigned)ZL.y == i ? 0.f : ra;
-    rb = (int)(unsigned)(ZL.y >> 32) == i ? 0.f : rb;
-  }
-  const u64 rinv = pk2(ra, rb);
-  const u64 qr = pmul(Z.y, rinv);
-  const u64 qr3 = pmul(qr, pmul(rinv, rinv));
-  if (POT) phi = padd(phi, qr);
-  ex = pfma(qr3, dx, ex);
-  ey = pfma(qr3, dy, ey);
-  ez = pfma(qr3, dz, ez);
-}
-
-template <bool SELF>
-__device__ __forceinline__ void dipole_two(const P2PStage &sg, const P2PStageD &sd, int k, int i, const P2PTgt &t,
-                                           u64 &phi, u64 &ex, u64 &ey, u64 &ez) {
-  const ulonglong2 X = sg.X[k], Z = sg.Z[k], XL = sg.XL[k], ZL = sg.ZL[k], D = sd.D[k];
-  const u64 mz = sd.DZ[k].x;
-  const u64 dx = padd(psub(t.xh, X.x), psub(t.xl, XL.x));
-  const u64 dy = padd(psub(t.yh, X.y), psub(t.yl, XL.y));
-  const u64 dz = padd(psub(t.zh, Z.x), psub(t.zl, ZL.x));
-  const u64 r2 = pfma(dx, dx, pfma(dy, dy, pmul(dz, dz)));
-  float ra = rsqrt_approx(plo(r2)), rb = rsqrt_approx(phi_(r2));
-  if (SELF) {
-    ra = (int)(unsigned)ZL.y == i ? 0.f : ra;
-    rb = (int)(unsigned)(ZL.y >> 32) == i ? 0.f : rb;
-  }
-  const u64 rinv = pk2(ra, rb);
-  const u64 rr = pmul(rinv, rinv);
-  const u64 r3 = pmul(rr, rinv);
-  const u64 sr = pfma(D.x, dx, pfma(D.y, dy, pmul(mz, dz)));
-  const u64 r5 = pmul(pmul(pmul(pk2(3.f, 3.f), sr), r3), rr);
-  phi = psub(phi, pmul(sr, r3));
-  ex = padd(ex, psub(pmul(D.x, r3), pmul(r5, dx)));
-  ey = padd(ey, psub(pmul(D.y, r3), pmul(r5, dy)));
-  ez = padd(ez, psub(pmul(mz, r3), pmul(r5, dz)));
-}
-
-// one source of the packed layout, for partial chunks
-__device__ __forceinline__ void stage_get(const P2PStage &sg, int j, float4 &h, float4 &l) {
-  const int o = 4 * (j >> 1) + (j & 1);
-  const float *x = sf(sg.X) + o, *z = sf(sg.Z) + o, *xl = sf(sg.XL) + o, *zl = sf(sg.ZL) + o;
-  h = make_float4(x[0], x[2], z[0], z[2]);
-  l = make_float4(xl[0], xl[2], zl[0], zl[2]);
-}
-__device__ __forceinline__ float4 stage_getd(const P2PStageD &sd, int j) {
-  const int o = 4 * (j >> 1) + (j & 1);
-  const float *d = sf(sd.D) + o, *dz = sf(sd.DZ) + o;
-  return make_float4(d[0], d[2], dz[0], 0.f);
-}
-
-// Sources first, first + step, ... < cnt of the staged chunk.
-template <bool SELF, bool POT, int SO>
-__device__ __forceinline__ void p2p_chunk(const P2PStage &sg, const P2PStageD &sd, int first, int cnt, int step,
-                                          int i, const P2PTgt &t, float txh, float txl, float tyh, float tyl,
-                                          float tzh, float tzl, float &phi, float &ex, float &ey, float &ez) {
-  if (step == 1 && cnt == 32) {
-    u64 p2 = 0, x2 = 0, y2 = 0, z2 = 0;
-#pragma unroll 4
-    for (int k = 0; k < 16; k++) {
-      if (SO == 0)
-        coulomb_two<SELF, POT>(sg, k, i, t, p2, x2, y2, z2);
-      else
-        dipole_two<SELF>(sg, sd, k, i, t, p2, x2, y2, z2);
+// The lane's targets on the staged pairs slice, slice + (1 << lf), ...: nb blocks
+// of two.
+template <bool NEAR, bool POT, int SO>
+__device__ __forceinline__ void p2p_pairs(const P2PStage &sg, const P2PStageD &sd, int slice, int lf, int nb,
+                                          P2PTarget (&g)[2]) {
+  u64 ph[2] = {}, ex[2] = {}, ey[2] = {}, ez[2] = {};
+  u64 hx[2], hy[2], hz[2], lx[2], ly[2], lz[2];
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    if (NEAR) {
+      hx[t] = pk2(g[t].hx, g[t].hx); hy[t] = pk2(g[t].hy, g[t].hy); hz[t] = pk2(g[t].hz, g[t].hz);
+      lx[t] = pk2(g[t].lx, g[t].lx); ly[t] = pk2(g[t].ly, g[t].ly); lz[t] = pk2(g[t].lz, g[t].lz);
+    } else {
+      hx[t] = pk2(g[t].tx, g[t].tx); hy[t] = pk2(g[t].ty, g[t].ty); hz[t] = pk2(g[t].tz, g[t].tz);
     }
-    if (POT || SO) phi += plo(p2) + phi_(p2);
-    ex += plo(x2) + phi_(x2);
-    ey += plo(y2) + phi_(y2);
-    ez += plo(z2) + phi_(z2);
-    return;
   }
-#pragma unroll 4
-  for (int jj = first; jj < cnt; jj += step) {
-    float4 h, l;
-    stage_get(sg, jj, h, l);
-    if (SO == 0)
-      coulomb_one<SELF, POT>(h, l, i, txh, txl, tyh, tyl, tzh, tzl, phi, ex, ey, ez);
-    else
-      dipole_one<SELF>(h, l, stage_getd(sd, jj), i, txh, txl, tyh, tyl, tzh, tzl, phi, ex, ey, ez);
+  int k = slice;
+#pragma unroll 1
+  for (int b = 0; b < nb; b++)
+#pragma unroll
+    for (int u = 0; u < 2; u++, k += 1 << lf) {
+      const ulonglong2 X = sg.X[k], Z = sg.Z[k];
+      ulonglong2 XL, ZL, D;
+      u64 mz;
+      if (NEAR) {
+        XL = sg.XL[k];
+        ZL = sg.ZL[k];
+      }
+      if (SO) {
+        D = sd.D[k];
+        mz = sd.DZ[k].x;
+      }
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        u64 dx = psub(hx[t], X.x), dy = psub(hy[t], X.y), dz = psub(hz[t], Z.x);
+        if (NEAR) {
+          dx = padd(dx, psub(lx[t], XL.x));
+          dy = padd(dy, psub(ly[t], XL.y));
+          dz = padd(dz, psub(lz[t], ZL.x));
+        }
+        const u64 r2 = pfma(dx, dx, pfma(dy, dy, pmul(dz, dz)));
+        float ra = rsqrt_approx(plo(r2)), rb = rsqrt_approx(phi_(r2));
+        if (NEAR) {  // l2 != l1
+          ra = (int)(unsigned)ZL.y == g[t].i ? 0.f : ra;
+          rb = (int)(unsigned)(ZL.y >> 32) == g[t].i ? 0.f : rb;
+        }
+        const u64 rinv = pk2(ra, rb);
+        const u64 rr = pmul(rinv, rinv);
+        if (SO == 0) {
+          const u64 qr = pmul(Z.y, rinv);
+          const u64 qr3 = pmul(qr, rr);
+          if (POT) ph[t] = padd(ph[t], qr);
+          ex[t] = pfma(qr3, dx, ex[t]);
+          ey[t] = pfma(qr3, dy, ey[t]);
+          ez[t] = pfma(qr3, dz, ez[t]);
+        } else {
+          const u64 r3 = pmul(rr, rinv);
+          const u64 v = pmul(pfma(D.x, dx, pfma(D.y, dy, pmul(mz, dz))), r3);
+          if (POT) ph[t] = psub(ph[t], v);
+          const u64 r5 = pmul(pmul(pk2(-3.f, -3.f), rr), v);
+          ex[t] = padd(ex[t], pfma(D.x, r3, pmul(r5, dx)));
+          ey[t] = padd(ey[t], pfma(D.y, r3, pmul(r5, dy)));
+          ez[t] = padd(ez[t], pfma(mz, r3, pmul(r5, dz)));
+        }
+      }
+    }
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    if (POT) kahan_add(g[t].s0, g[t].c0, plo(ph[t]) + phi_(ph[t]));
+    kahan_add(g[t].s1, g[t].c1, plo(ex[t]) + phi_(ex[t]));
+    kahan_add(g[t].s2, g[t].c2, plo(ey[t]) + phi_(ey[t]));
+    kahan_add(g[t].s3, g[t].c3, plo(ez[t]) + phi_(ez[t]));
   }
 }
 
-// The near field of target leaf A by one warp (sg, sd: its staging area).
+struct P2PArgs {
+  const int4 *units;               // (cell, first target, targets, leaf)
+  const int *pstart, *pcount, *off, *src;
+  const int *ix, *iy, *iz;
+  const unsigned char *clevel;
+  const float4 *phi4, *plo4, *sdip, *lorg;
+  double *Fnear;
+};
+
+// The near field of the targets [tb, tb + m) of leaf cell A by one warp (sg, sd:
+// its staging area).
 template <bool POT, int SO>
-__device__ __forceinline__ void p2p_leaf(int A, const int *pstart, const int *pcount, const int *off_,
-                                         const int *src, const float4 *phi4, const float4 *plo4,
-                                         const float4 *sdip, P2PStage &sg, P2PStageD &sd, double *Fnear) {
-  const unsigned FULL = 0xffffffffu;
+__device__ __forceinline__ void p2p_targets(const P2PArgs &P, int A, const float4 org, int tb, int m, P2PStage &sg,
+                                            P2PStageD &sd) {
+  constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int a0 = pstart[A], na = pcount[A];
-  const int k0 = off_[A], k1 = off_[A + 1];
-  const int sk = 4 * (lane >> 1) + (lane & 1);  // this lane's slot when it stages source `lane` of a chunk
-  for (int tb = 0; tb < na; tb += 32) {
-    const int m = min(32, na - tb);
-    int lf = 0;  // f = 2^lf lanes per target
-    while ((2 << lf) * m <= 32) lf++;
-    const int f = 1 << lf;
-    const int tl = lane >> lf, slice = lane & (f - 1);
-    const bool ok = tl < m;
-    const int i = a0 + tb + (ok ? tl : 0);
-    const float4 th = phi4[i], tlo = plo4[i];
-    const P2PTgt tg = {pk2(th.x, th.x), pk2(tlo.x, tlo.x), pk2(th.y, th.y),
-                       pk2(tlo.y, tlo.y), pk2(th.z, th.z), pk2(tlo.z, tlo.z)};
-    float s0 = 0, s1 = 0, s2 = 0, s3 = 0, c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-    for (int kb = k0; kb < k1; kb += 32) {
-      // up to 32 source leaves: lane q holds leaf kb + q's particle range and
-      // the exclusive prefix of the counts (its offset in the stream)
-      const int nbat = min(32, k1 - kb);
-      int B = -1, start = 0, cnt = 0;
-      if (lane < nbat) {
-        B = src[kb + lane];
-        start = pstart[B];
-        cnt = pcount[B];
-      }
-      int incl = cnt;
+  const int a0 = P.pstart[A];
+  const int k0 = P.off[A], k1 = P.off[A + 1];
+  const int la = P.clevel[A], ax = P.ix[A], ay = P.iy[A], az = P.iz[A];
+  const int lf = m > 16 ? 1 : m > 8 ? 2 : 3, half = 32 >> lf;  // targets tl and tl + half
+  const int tl = lane >> lf, slice = lane - (tl << lf);
+  P2PTarget g[2];
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    const int tt = tl + t * half;
+    g[t].i = a0 + tb + (tt < m ? tt : 0);
+    const float4 h = P.phi4[g[t].i], l = P.plo4[g[t].i];
+    g[t].hx = h.x; g[t].hy = h.y; g[t].hz = h.z;
+    g[t].lx = l.x; g[t].ly = l.y; g[t].lz = l.z;
+    g[t].tx = (h.x - org.x) + l.x; g[t].ty = (h.y - org.y) + l.y; g[t].tz = (h.z - org.z) + l.z;
+  }
+  for (int kb = k0; kb < k1; kb += 32) {
+    // up to 32 source leaves: lane q holds leaf kb + q's particle range
+    const int nbat = min(32, k1 - kb);
+    int B = -1, start = 0, cnt = 0;
+    bool far = false;
+    if (lane < nbat) {
+      B = P.src[kb + lane];
+      start = P.pstart[B];
+      cnt = P.pcount[B];
+      // gap between the two cells along each axis, in cells of the finer level
+      const int lb = P.clevel[B], lm = max(la, lb), sa = lm - la, sb = lm - lb;
+      const int gx = max((P.ix[B] << sb) - ((ax + 1) << sa), (ax << sa) - ((P.ix[B] + 1) << sb));
+      const int gy = max((P.iy[B] << sb) - ((ay + 1) << sa), (ay << sa) - ((P.iy[B] + 1) << sb));
+      const int gz = max((P.iz[B] << sb) - ((az + 1) << sa), (az << sa) - ((P.iz[B] + 1) << sb));
+      far = max(gx, max(gy, gz)) >= 1 << sa;  // a target-leaf width
+    }
+#pragma unroll 1
+    for (int near = 1; near >= 0; near--) {  // the near leaves' stream, then the far ones'
+      const int mine = far == (near == 0) ? cnt : 0;
+      int incl = mine;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int v = __shfl_up_sync(FULL, incl, d);
         if (lane >= d) incl += v;
       }
-      const int excl = incl - cnt;
+      const int excl = incl - mine;
       const int total = __shfl_sync(FULL, incl, 31);
-      // the target leaf's own range in the stream (self pairs skip i == j)
-      const unsigned selfq = __ballot_sync(FULL, B == A);
-      const int self_lo = selfq ? __shfl_sync(FULL, excl, __ffs(selfq) - 1) : -1;
-      for (int cb = 0; cb < total; cb += 32) {
-        // the lane's source: the last leaf q whose stream offset is <= s
-        const int s = cb + lane;
+      const int shift = start - excl;  // stream place -> particle
+      const unsigned after = __ballot_sync(FULL, mine > 0) & (0xfffffffeu << lane);
+      const int next = __shfl_sync(FULL, start, after ? __ffs(after) - 1 : lane);  // of the next leaf that holds any
+#pragma unroll 1
+      for (int cb = 0; cb < total; cb += 64) {
+        // the lane's sources: s lies in the last leaf q whose stream offset is <= s
+        const int s = cb + 2 * lane;
         int q = 0;
 #pragma unroll
         for (int stp = 16; stp; stp >>= 1) {
-          const int cand = q + stp;
-          const int v = __shfl_sync(FULL, excl, cand & 31);
-          if (cand < nbat && v <= s) q = cand;
+          const int v = __shfl_sync(FULL, excl, q + stp);
+          if (v <= s) q += stp;
         }
-        const int jb = __shfl_sync(FULL, start, q), je = __shfl_sync(FULL, excl, q);
-        __syncwarp();
+        const int j0 = s + __shfl_sync(FULL, shift, q), end = __shfl_sync(FULL, incl, q);
+        const int jn = __shfl_sync(FULL, next, q);
+        const int j1 = s + 1 < end ? j0 + 1 : jn;
+        float4 h0 = make_float4(org.w, org.w, org.w, 0.f), h1 = h0;
+        float4 l0 = make_float4(0.f, 0.f, 0.f, __int_as_float(-1)), l1 = l0;
+        float4 d0 = make_float4(0.f, 0.f, 0.f, 0.f), d1 = d0;
         if (s < total) {
-          const int j = jb + (s - je);
-          const float4 h = phi4[j], l = plo4[j];
-          sf(sg.X)[sk] = h.x; sf(sg.X)[sk + 2] = h.y;
-          sf(sg.Z)[sk] = h.z; sf(sg.Z)[sk + 2] = h.w;
-          sf(sg.XL)[sk] = l.x; sf(sg.XL)[sk + 2] = l.y;
-          sf(sg.ZL)[sk] = l.z; sf(sg.ZL)[sk + 2] = l.w;
-          if (SO) {
-            const float4 d = sdip[j];
-            sf(sd.D)[sk] = d.x; sf(sd.D)[sk + 2] = d.y;
-            sf(sd.DZ)[sk] = d.z;
-          }
+          h0 = P.phi4[j0];
+          l0 = P.plo4[j0];
+          if (SO) d0 = P.sdip[j0];
+        }
+        if (s + 1 < total) {
+          h1 = P.phi4[j1];
+          l1 = P.plo4[j1];
+          if (SO) d1 = P.sdip[j1];
         }
         __syncwarp();
-        const int n = min(32, total - cb);
-        const bool self = self_lo >= 0 && self_lo < cb + n && self_lo + na > cb;
-        float phi = 0, ex = 0, ey = 0, ez = 0;
-        if (self)
-          p2p_chunk<true, POT, SO>(sg, sd, slice, n, f, i, tg, th.x, tlo.x, th.y, tlo.y, th.z, tlo.z, phi, ex, ey,
-                                   ez);
-        else
-          p2p_chunk<false, POT, SO>(sg, sd, slice, n, f, i, tg, th.x, tlo.x, th.y, tlo.y, th.z, tlo.z, phi, ex, ey,
-                                    ez);
-        if (POT) kahan_add(s0, c0, phi);
-        kahan_add(s1, c1, ex); kahan_add(s2, c2, ey); kahan_add(s3, c3, ez);
+        if (near) {
+          sg.XL[lane] = make_ulonglong2(pk2(l0.x, l1.x), pk2(l0.y, l1.y));
+          sg.ZL[lane] = make_ulonglong2(pk2(l0.z, l1.z), pk2(l0.w, l1.w));
+        } else {  // into the target leaf's frame
+          h0.x = (h0.x - org.x) + l0.x; h1.x = (h1.x - org.x) + l1.x;
+          h0.y = (h0.y - org.y) + l0.y; h1.y = (h1.y - org.y) + l1.y;
+          h0.z = (h0.z - org.z) + l0.z; h1.z = (h1.z - org.z) + l1.z;
+        }
+        sg.X[lane] = make_ulonglong2(pk2(h0.x, h1.x), pk2(h0.y, h1.y));
+        sg.Z[lane] = make_ulonglong2(pk2(h0.z, h1.z), pk2(h0.w, h1.w));
+        if (SO) {
+          sd.D[lane] = make_ulonglong2(pk2(d0.x, d1.x), pk2(d0.y, d1.y));
+          sd.DZ[lane].x = pk2(d0.z, d1.z);
+        }
+        __syncwarp();
+        // blocks of 2 << lf pairs that hold the chunk's sources
+        const int nb = (min(64, total - cb) + (4 << lf) - 1) >> (2 + lf);
+        if (near) p2p_pairs<true, POT, SO>(sg, sd, slice, lf, nb, g);
+        else p2p_pairs<false, POT, SO>(sg, sd, slice, lf, nb, g);
       }
     }
-    // combine the f lanes of each target in FP64
-    double r0 = (double)s0 - (double)c0, r1 = (double)s1 - (double)c1;
-    double r2 = (double)s2 - (double)c2, r3 = (double)s3 - (double)c3;
-    for (int o = 1; o < f; o <<= 1) {
-      r0 += __shfl_xor_sync(FULL, r0, o);
-      r1 += __shfl_xor_sync(FULL, r1, o);
-      r2 += __shfl_xor_sync(FULL, r2, o);
-      r3 += __shfl_xor_sync(FULL, r3, o);
+  }
+  // the lanes of each target
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    P2PTarget &r = g[t];
+    for (int o = 1; o < 1 << lf; o <<= 1) {
+      if (POT) pair_add(r.s0, r.c0, __shfl_xor_sync(FULL, r.s0, o), __shfl_xor_sync(FULL, r.c0, o));
+      pair_add(r.s1, r.c1, __shfl_xor_sync(FULL, r.s1, o), __shfl_xor_sync(FULL, r.c1, o));
+      pair_add(r.s2, r.c2, __shfl_xor_sync(FULL, r.s2, o), __shfl_xor_sync(FULL, r.c2, o));
+      pair_add(r.s3, r.c3, __shfl_xor_sync(FULL, r.s3, o), __shfl_xor_sync(FULL, r.c3, o));
     }
-    if (ok && slice == 0) {
-      Fnear[4 * (size_t)i] = r0;
-      Fnear[4 * (size_t)i + 1] = r1;
-      Fnear[4 * (size_t)i + 2] = r2;
-      Fnear[4 * (size_t)i + 3] = r3;
+    if (slice == t && tl + t * half < m) {
+      double *F = P.Fnear + 4 * (size_t)r.i;
+      F[0] = f2d(r.s0) - f2d(r.c0);
+      F[1] = f2d(r.s1) - f2d(r.c1);
+      F[2] = f2d(r.s2) - f2d(r.c2);
+      F[3] = f2d(r.s3) - f2d(r.c3);
     }
   }
 }
 
-template <bool POT, int WARPS, int SO>
-__global__ void __launch_bounds__(32 * WARPS) k_p2p32(const int *leaf_cells, int nleaves, const int *pstart,
-                                                      const int *pcount, const int *off_, const int *src,
-                                                      const float4 *phi4, const float4 *plo4, const float4 *sdip,
-                                                      double *Fnear) {
-  __shared__ P2PStage sg[WARPS];
-  __shared__ P2PStageD sd[SO ? WARPS : 1];
-  const int w = threadIdx.x >> 5;
-  const int leaf = blockIdx.x * WARPS + w;
-  if (leaf < nleaves)
-    p2p_leaf<POT, SO>(leaf_cells[leaf], pstart, pcount, off_, src, phi4, plo4, sdip, sg[w], sd[SO ? w : 0], Fnear);
+template <bool POT, int SO>
+__global__ void __launch_bounds__(32, 24) k_p2p32(const P2PArgs P) {
+  __shared__ P2PStage sg;
+  __shared__ P2PStageD sd;
+  const int4 u = P.units[blockIdx.x];
+  p2p_targets<POT, SO>(P, u.x, P.lorg[u.w], u.y, u.z, sg, sd);
 }
 
 // ---------------------------------------------------------------------------
 // launchers used by eval.cu
 // ---------------------------------------------------------------------------
-int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st, bool narrow) {
+int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st) {
   const int nl = t->nleaves, so = t->so;
   if (mixed && so <= 1) {  // quadrupole sources take the FP64 kernel in every precision
-    // narrow blocks (2 warps) when running beside the tensor-core M2L: they
-    // fit in the registers its CTA leaves free
-    const bool pot = t->pass_potential || so;
-    const int wp = narrow ? 2 : P2P_WARPS;
-    decltype(&k_p2p32<true, 2, 0>) k;
-    if (so)
-      k = narrow ? k_p2p32<true, 2, 1> : k_p2p32<true, P2P_WARPS, 1>;
-    else
-      k = narrow ? (pot ? k_p2p32<true, 2, 0> : k_p2p32<false, 2, 0>)
-                 : (pot ? k_p2p32<true, P2P_WARPS, 0> : k_p2p32<false, P2P_WARPS, 0>);
-    const unsigned grid = fmm_blocks(nl, wp);
+    const bool pot = t->pass_potential;
+    decltype(&k_p2p32<true, 0>) k = so ? (pot ? k_p2p32<true, 1> : k_p2p32<false, 1>)
+                                       : (pot ? k_p2p32<true, 0> : k_p2p32<false, 0>);
+    const P2PArgs P = {t->p2p_units.p, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->ix.p, t->iy.p,
+                       t->iz.p, t->clevel.p, t->phi4.p, t->plo4.p, t->sdip.p, t->lorg.p, t->Fnear.p};
     if (int rc = fmm_mark_kernel(t, 2, st)) return rc;
-    fmm_note_launch(), k<<<grid, 32 * wp, 0, st>>>(t->leaf_cells.p, nl, t->pstart.p, t->pcount.p, t->p2p_off.p,
-                                                   t->p2p_src.p, t->phi4.p, t->plo4.p, t->sdip.p, t->Fnear.p);
+    fmm_note_launch(), k<<<t->np2p_units, 32, 0, st>>>(P);
   } else {
     // a leaf holds fewer than ncrit particles (a root leaf fewer than N): its full chunks of 32, then three groups
     const bool pot = t->pass_potential;
@@ -575,9 +577,10 @@ int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st, boo
 
 int fmm_stage_particles(DevTree *t, const double *S, cudaStream_t st) {
   if (t->so > 1) return FMM_OK;  // the FP64 P2P reads the sources directly
+  if (int rc = fmm_reserve(t->lorg, t->nleaves)) return rc;
   fmm_note_launch(), k_stage_particles<<<t->nleaves, 128, 0, st>>>(
-      t->leaf_cells.p, t->nleaves, t->pstart.p, t->pcount.p, t->csys.p, t->roots.p, t->px.p, t->py.p, t->pz.p,
-      t->perm.p, S, t->so, t->phi4.p, t->plo4.p, t->sdip.p);
+      t->leaf_cells.p, t->nleaves, t->pstart.p, t->pcount.p, t->csys.p, t->roots.p, t->cx.p, t->cy.p, t->cz.p,
+      t->px.p, t->py.p, t->pz.p, t->perm.p, S, t->so, t->phi4.p, t->plo4.p, t->sdip.p, t->lorg.p);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
 }

@@ -283,12 +283,28 @@ __global__ void k_leaf_flags(int ncells, long ncrit, const int *pcount, uint32_t
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < ncells) flag[c] = pcount[c] < ncrit ? 1u : 0u;
 }
+// Leaves in cell order, and the near field's units: each leaf's targets in chunks
+// of 32, (cell, first target, targets, leaf), in the order the warps arrive (the
+// units do not depend on one another).
 __global__ void k_leaf_compact(int ncells, long ncrit, const int *pcount, const uint32_t *off, int *leaf_cells,
-                               int *cell_leaf) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  if (pcount[c] < ncrit) { leaf_cells[off[c]] = c; cell_leaf[c] = (int)off[c]; }
-  else cell_leaf[c] = -1;
+                               int *cell_leaf, int4 *units, uint32_t *nunits) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int cnt = c < ncells ? pcount[c] : 0;
+  const bool leaf = c < ncells && cnt < ncrit;
+  const int ord = leaf ? (int)off[c] : -1;
+  if (leaf) leaf_cells[ord] = c;
+  if (c < ncells) cell_leaf[c] = ord;
+  const int n = leaf ? (cnt + 31) >> 5 : 0;
+  int incl = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  uint32_t base = 0;
+  if (lane == 31 && incl > 0) base = atomicAdd(nunits, (uint32_t)incl);
+  base = __shfl_sync(0xffffffffu, base, 31) + (uint32_t)(incl - n);
+  for (int k = 0; k < n; k++) units[base + k] = make_int4(c, 32 * k, min(32, cnt - 32 * k), ord);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,8 +673,8 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
   }
   t->build_serial++;
   TRY(rec(t, 0, st));
-  TRY(fmm_reserve(t->d_eflags, 4));
-  FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, sizeof(uint32_t), st));
+  TRY(fmm_reserve(t->d_eflags, 4));  // error flags, near-field units
+  FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, 2 * sizeof(uint32_t), st));
   TRY(fmm_reserve(t->sys_off, (size_t)nsys + 1));
   FMM_CUDA_TRY(cudaMemcpyAsync(t->sys_off.p, t->sys_off_h.data(), sizeof(long) * (nsys + 1),
                                cudaMemcpyHostToDevice, st));
@@ -833,16 +849,18 @@ static int build_cells(DevTree *t, cudaStream_t st, int nlev, bool *deeper) {
   uint32_t *stmp = total + 1;
   fmm_note_launch(), k_leaf_flags<<<fmm_blocks(nc, 256), 256, 0, st>>>(nc, t->ncrit, t->pcount.p, flag);
   TRY(fmm_scan<uint32_t>(flag, flag, nc, total, stmp, st));
-  fmm_note_launch(), k_leaf_compact<<<fmm_blocks(nc, 256), 256, 0, st>>>(nc, t->ncrit, t->pcount.p, flag, t->leaf_cells.p,
-                                                      t->cell_leaf.p);
+  TRY(fmm_reserve(t->p2p_units, (size_t)nc + (size_t)(N / 32) + 1));
+  fmm_note_launch(), k_leaf_compact<<<fmm_blocks(nc, 256), 256, 0, st>>>(
+      nc, t->ncrit, t->pcount.p, flag, t->leaf_cells.p, t->cell_leaf.p, t->p2p_units.p, t->d_eflags.p + 1);
   FMM_CUDA_TRY(cudaGetLastError());
   FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned + 1, t->d_eflags.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned + 1, t->d_eflags.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   FMM_CUDA_TRY(cudaStreamSynchronize(st));
   t->nleaves = (int)t->h_pinned[0];
+  t->np2p_units = (int)t->h_pinned[2];
   if (t->h_pinned[1] & FMM_EFLAG_KEYS) {
     *deeper = true;
-    FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, sizeof(uint32_t), st));
+    FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, 2 * sizeof(uint32_t), st));
     return FMM_OK;
   }
   TRY(fmm_reserve(t->cmargin, nc));
@@ -1141,7 +1159,8 @@ void fmm_tree_destroy(DevTree *t) {
   t->gstream = nullptr;
   fmm_release(t->keys); fmm_release(t->keys2); fmm_release(t->perm); fmm_release(t->perm2);
   fmm_release(t->px); fmm_release(t->py); fmm_release(t->pz);
-  fmm_release(t->phi4); fmm_release(t->plo4); fmm_release(t->sdip); fmm_release(t->levf);
+  fmm_release(t->phi4); fmm_release(t->plo4); fmm_release(t->sdip); fmm_release(t->lorg); fmm_release(t->p2p_units);
+  fmm_release(t->levf);
   fmm_release(t->cx); fmm_release(t->cy); fmm_release(t->cz); fmm_release(t->cid);
   fmm_release(t->ix); fmm_release(t->iy); fmm_release(t->iz);
   fmm_release(t->pstart); fmm_release(t->pcount); fmm_release(t->parent); fmm_release(t->child_first);
