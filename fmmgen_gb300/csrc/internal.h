@@ -25,6 +25,11 @@ struct PlanSet {
 };
 const PlanSet *fmm_get_plans(int order, int so);  // cached per device
 
+// Barnes-Hut: the weights of one harmonic derivative in the potential and the three field components (bh.cu)
+struct __align__(16) BhWeight {
+  double v, x, y, z;
+};
+
 struct DevTree {
   // configuration
   long N = 0, ncrit = 0;
@@ -120,6 +125,7 @@ struct DevTree {
   DevBuf<unsigned char> cm_otab;          // per class step: each tile row's per-pair M2L order
   DevBuf<int> cm_woff, cm_wstep;          // per (tile, warp of 32 rows): its steps with a pair
   uint64_t cm_wserial = ~0ull, cm_wversion = ~0ull;  // ... of this schedule (build, cell order)
+  DevBuf<BhWeight> bhW;                   // Barnes-Hut: weights of each cell's harmonic derivatives (bh.cu)
   DevBuf<char> hM, hL, hD;                // harmonic M2L: folded multipoles, outputs, operators (m2l_h.cu)
   DevBuf<int> tp_perm;                    // per target list: pair indices by descending per-pair order
   DevBuf<int> tp_tgt;                     // targets by list length (of this build and cell order); with per-pair
@@ -227,6 +233,8 @@ bool fmm_m2l_cm_supported(int p, int so);
 int fmm_m2l_h(DevTree *t, const float *M, int mstr, float *L, int lstr, const unsigned char *ord, cudaStream_t st);
 int fmm_m2l_h(DevTree *t, const double *M, int mstr, double *L, int lstr, const unsigned char *ord, cudaStream_t st);
 bool fmm_m2l_h_supported(int p, int so);
+int fmm_h_fold(DevTree *t, const double *M, int mstr, double *Mh, int hstr, cudaStream_t st);  // every cell's multipole
+int fmm_bh_walk(DevTree *t, const double *S, double *F, int potential, int field, cudaStream_t st);  // (bh.cu)
 // targets of the harmonic M2L (tp_tgt): by list length, longest first; with per-pair orders by their high-order pairs,
 // and each list by descending order (tp_perm)
 int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st);

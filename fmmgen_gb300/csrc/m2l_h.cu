@@ -138,3 +138,9 @@ int fmm_m2l_h(DevTree *t, const float *M, int mstr, float *L, int lstr, const un
 int fmm_m2l_h(DevTree *t, const double *M, int mstr, double *L, int lstr, const unsigned char *ord, cudaStream_t st) {
   return run<double>(t, M, mstr, L, lstr, ord, st);
 }
+int fmm_h_fold(DevTree *t, const double *M, int mstr, double *Mh, int hstr, cudaStream_t st) {
+  fmm_note_launch(), k_h_fold<double><<<grid_of((long)t->ncells * h_terms(t->order)), H_BLOCK, 0, st>>>(
+      t->ncells, t->order, t->so, M, mstr, Mh, hstr);
+  FMM_CUDA_TRY(cudaGetLastError());
+  return FMM_OK;
+}

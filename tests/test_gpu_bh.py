@@ -95,3 +95,20 @@ def test_m2p_operator(fg, oracle_lib):
             mod.M2P(*d[0], np.ascontiguousarray(M[0]), Fs, p)
             getattr(mod, f"M2P{p}")(*d[0], np.ascontiguousarray(M[0]), Fs)  # += semantics: twice
             assert np.allclose(Fs, 2 * F[0], rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("so,p", [(0, 1), (0, 2), (0, 5), (0, 8), (0, 12), (1, 2), (1, 7), (2, 3), (2, 6)])
+@pytest.mark.parametrize("n,ncrit,theta", [(1, 8, 0.5), (31, 4, 0.5), (700, 4, 0.3), (1503, 40, 0.6)])
+def test_bh_orders_and_queues(fg, oracle_lib, n, ncrit, theta, so, p):
+    """Every order's kernel family edges, a warp's last particles, and walks that fill the queues of accepted cells
+    (64) and opened leaves (32) several times over."""
+    rng = np.random.default_rng(100 * p + n)
+    pos = rng.uniform(0, 1, (n, 3)) ** 2
+    S = rng.uniform(-1, 1, (n, {0: 1, 1: 3, 2: 6}[so]))
+    F = fg.build_tree(pos, S, n, ncrit, p, theta, source_order=so).compute_field_bh().cpu().numpy()
+    Fo = oracle_lib.OracleTree(pos, S, ncrit, p, theta, so).evaluate_bh()
+    if n == 1:
+        assert (F == 0).all()
+        return
+    assert rel(F[:, 0], Fo[:, 0]) < 1e-11
+    assert rel(F[:, 1:], Fo[:, 1:]) < 1e-11
