@@ -32,7 +32,7 @@
 #include "internal.h"
 
 size_t fmm_seqsum_scratch(long N);
-int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, cudaStream_t st);
+int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, bool tables, cudaStream_t st);
 __global__ void k_root_absmax(const double *__restrict__ pos, long N, const double *sums, unsigned long long *mx);
 __global__ void k_root_final(const double *sums, const unsigned long long *mx, long N, double *root, double *lev,
                              float2 *levf);
@@ -82,7 +82,7 @@ extern "C" int fmmgen_root_box_noalloc(const double *pos, long N, double *root4,
   void *ss = b + 1024;
   // the maxima are combined with atomicMax and must start at zero
   FMM_CUDA_TRY(cudaMemsetAsync(mx, 0, 3 * sizeof(unsigned long long), st));
-  rc = fmm_seqsum3(pos, N, sums, ss, st);
+  rc = fmm_seqsum3(pos, N, sums, ss, false, st);  // the static scratch has no room for the tables
   if (rc) return rc;
   unsigned nbm = std::min<unsigned>(fmm_blocks(N, 256), 152 * 8);
   fmm_note_launch(), k_root_absmax<<<nbm, 256, 0, st>>>(pos, N, sums, mx);

@@ -17,10 +17,29 @@
 //  valid while every intermediate S stays in [2^52, 2^53) (or its negative
 //  mirror).  Chunks are analysed in parallel (integer arithmetic on the
 //  mantissa bits, no FP64 pipe), with the binade guessed from an ordinary
-//  parallel prefix sum; a single thread then chains the chunk maps, checks
-//  each map's validity against the exact S, and falls back to plain sequential
-//  FP64 adds for any chunk that leaves its binade or was guessed wrong (the
-//  first chunk always does).  The result equals the sequential loop exactly.
+//  parallel prefix sum.
+//
+//  A chunk that leaves its binade has no such map, but the prefix sum tells
+//  where: the guess is off by rounding errors (~1e-12 of the terms), the running
+//  sum passes the powers of two at distances of the size of the terms.  Take two
+//  starts that differ by d, a multiple of 2^5 ulps of the start, and let no
+//  result within the chunk lie above the start's binade by more than four.  Then d
+//  is a multiple of twice every result's ulp, and if no result comes closer to a
+//  power of two than |d|, every exact sum of the two runs is rounded to the same
+//  grid, with the same parity: the results differ by exactly d.  So 32 runs of
+//  plain FP64 adds, one for each value of the start's last five bits (a lane
+//  each), are a table of the chunk for every start near the guess; the closest
+//  approach to a power of two is kept beside it (k_ss_tables).
+//
+//  One warp then chains the chunks, checks each map's or table's validity against
+//  the exact sum, and falls back to element scans with plain FP64 adds where
+//  neither holds (the first chunk; sums passing zero).  The result equals the
+//  sequential loop exactly.  A forest's systems are chained side by side.
+//
+//  Measured (one GB300): 2x10^6 centred positions (Plummer), whose sums leave
+//  their binade in 1,740 of 7,813 chunks per axis: 19.1 -> 2.4 ms (those chunks took
+//  26,000 clocks each as element scans); 10^6 positions in the unit cube: 0.31
+//  -> 0.30 ms; 512 systems of 1,000 to 65,536: 7.1 -> 0.9 ms (a thread per sum).
 #include "internal.h"
 
 #define SS_C 256  // elements per chunk
@@ -33,26 +52,64 @@ struct ChunkMap {
   int ok;                // 0: no map, run the chunk sequentially
 };
 
+// The systems' elements and chunks: system s holds elements [sys_off[s],
+// sys_off[s + 1]) and chunks [chunk_off[s], chunk_off[s + 1]); one system has
+// neither array.
+struct SsArgs {
+  const double *pos;
+  long N, nchunks;
+  int nsys;
+  const long *sys_off;
+  const int *chunk_off;
+  __device__ __forceinline__ void chunks(int s, long &k0, long &k1) const {
+    k0 = nsys > 1 ? chunk_off[s] : 0;
+    k1 = nsys > 1 ? chunk_off[s + 1] : nchunks;
+  }
+  // elements [i0, i1) of chunk k
+  __device__ __forceinline__ void range(long k, long &i0, long &i1) const {
+    long end = N;
+    i0 = k * SS_C;
+    if (nsys > 1) {
+      int lo = 0, hi = nsys - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (chunk_off[mid] <= k) lo = mid; else hi = mid - 1;
+      }
+      i0 = sys_off[lo] + (k - chunk_off[lo]) * SS_C;
+      end = sys_off[lo + 1];
+    }
+    i1 = min(end, i0 + SS_C);
+  }
+};
+
 // approximate chunk sums (FP64, any order)
-__global__ void k_ss_chunksum(const double *__restrict__ pos, long N, long nchunks, double *csum) {
+__global__ void k_ss_chunksum(const SsArgs A, double *csum) {
+  const long nchunks = A.nchunks;
   long k = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   int a = blockIdx.y, lane = threadIdx.x & 31;
   if (k >= nchunks) return;
+  long i0, i1;
+  A.range(k, i0, i1);
   double s = 0;
   for (int j = 0; j < SS_PER_LANE; j++) {
-    long i = k * SS_C + lane * SS_PER_LANE + j;
-    if (i < N) s += pos[3 * i + a];
+    long i = i0 + lane * SS_PER_LANE + j;
+    if (i < i1) s += A.pos[3 * i + a];
   }
   for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
   if (lane == 0) csum[a * nchunks + k] = s;
 }
 
-// exclusive prefix of the chunk sums (approximate start values), one block per axis
-__global__ void k_ss_prefix(const double *csum, long nchunks, double *start) {
+// exclusive prefix of a system's chunk sums (approximate start values), one block
+// per axis and system
+__global__ void k_ss_prefix(const SsArgs A, const double *csum, double *start) {
   __shared__ double wsum[32];
-  const int a = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5, nt = blockDim.x;
-  long per = (nchunks + nt - 1) / nt;
-  long b0 = t * per, b1 = min(nchunks, b0 + per);
+  const long nchunks = A.nchunks;
+  long k0, k1;
+  const int a = blockIdx.x % 3;
+  A.chunks(blockIdx.x / 3, k0, k1);
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5, nt = blockDim.x;
+  long per = (k1 - k0 + nt - 1) / nt;
+  long b0 = min(k1, k0 + t * per), b1 = min(k1, b0 + per);
   double s = 0;
   for (long k = b0; k < b1; k++) s += csum[a * nchunks + k];
   double inc = s;
@@ -153,10 +210,13 @@ __device__ __forceinline__ Map2 elem_map(const Elem &el) {
   return m;
 }
 
-__global__ void k_ss_maps(const double *__restrict__ pos, long N, long nchunks, const double *start, ChunkMap *maps) {
+__global__ void k_ss_maps(const SsArgs A, const double *start, ChunkMap *maps) {
+  const long nchunks = A.nchunks;
   long k = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   int a = blockIdx.y, lane = threadIdx.x & 31;
   if (k >= nchunks) return;
+  long i0, i1;
+  A.range(k, i0, i1);
   double s0 = start[a * nchunks + k];
   ChunkMap cm{0, 0, 0, 0, 0, 0};
   if (s0 == 0.0 || !isfinite(s0)) {
@@ -168,9 +228,9 @@ __global__ void k_ss_maps(const double *__restrict__ pos, long N, long nchunks, 
   long long run = 0, lmin = 0, lmax = 0;
   int bad = 0;
   for (int j = 0; j < SS_PER_LANE; j++) {
-    long i = k * SS_C + lane * SS_PER_LANE + j;
-    if (i >= N) break;
-    Elem el = elem_in_ulps(pos[3 * i + a], e);
+    long i = i0 + lane * SS_PER_LANE + j;
+    if (i >= i1) break;
+    Elem el = elem_in_ulps(A.pos[3 * i + a], e);
     bad |= el.bad;
     acc = compose(acc, elem_map(el));
     run += el.inc;
@@ -232,6 +292,62 @@ __device__ __forceinline__ bool ss_from_double(double s, int &e, long long &S) {
   return true;
 }
 
+// Tables of the chunks whose map will not hold for the guessed start: for each
+// value r of its last SS_TBITS bits the sum after the chunk, then the closest any
+// of the runs' results came to a power of two, in ulps of the start (0: no table).
+#define SS_TBITS 5
+#define SS_TAB ((1 << SS_TBITS) + 1)
+__global__ void k_ss_tables(const SsArgs A, const double *start, const ChunkMap *maps, double *tab) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const long nchunks = A.nchunks;
+  const long k = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int a = blockIdx.y, lane = threadIdx.x & 31;
+  if (k >= nchunks) return;
+  const long at = a * nchunks + k;
+  double *t = tab + at * SS_TAB;
+  const double s0 = start[at];
+  const ChunkMap m = maps[at];
+  int e0 = 0;
+  long long S0 = 0;
+  bool want = ss_from_double(s0, e0, S0);
+  if (want && m.ok) {  // the map holds with room to spare: no table
+    const long long LO = 1ll << 52, HI = 1ll << 53, room = 1ll << 24;
+    want = !(S0 > 0 ? (S0 + m.pmin >= LO + room && S0 + m.pmax < HI - room)
+                    : (S0 + m.pmax <= -LO - room && S0 + m.pmin > -HI + room));
+  }
+  if (!want) {
+    if (lane == 0) t[SS_TAB - 1] = 0.0;
+    return;
+  }
+  long i0, i1;
+  A.range(k, i0, i1);
+  const int n = (int)(i1 - i0);
+  double x[SS_PER_LANE];
+#pragma unroll
+  for (int j = 0; j < SS_PER_LANE; j++) x[j] = lane + 32 * j < n ? A.pos[3 * (i0 + lane + 32 * j) + a] : 0.0;
+  const unsigned long long mask = (1ull << SS_TBITS) - 1, b0 = (unsigned long long)__double_as_longlong(s0);
+  double s = __longlong_as_double((long long)((b0 & ~mask) | (unsigned)lane));
+  const int ex0 = (int)((b0 >> 52) & 0x7ff);
+  float room = 3e38f;
+#pragma unroll
+  for (int j = 0; j < SS_PER_LANE; j++) {
+    const int cnt = min(32, n - 32 * j);
+    for (int c = 0; c < cnt; c++) {
+      s = __dadd_rn(s, __shfl_sync(FULL, x[j], c));
+      const unsigned long long b = (unsigned long long)__double_as_longlong(s);
+      const int ex = (int)((b >> 52) & 0x7ff), d = ex - ex0;
+      const unsigned long long f = b & ((1ull << 52) - 1);
+      // distance to the nearer power of two, four ulps short of it
+      const float near = __ull2float_rd(min(f, (1ull << 52) - f)) - 4.f;
+      const bool good = ex > 0 && ex < 0x7ff && d <= SS_TBITS - 1 && d > -64;
+      room = fminf(room, good ? near * __int_as_float((d + 127) << 23) : 0.f);
+    }
+  }
+  for (int d = 16; d; d >>= 1) room = fminf(room, __shfl_xor_sync(FULL, room, d));
+  t[lane] = s;
+  if (lane == 0) t[SS_TAB - 1] = (double)fmaxf(room, 0.f);
+}
+
 // Chunk maps compose: chunk a then chunk b (same binade) is again
 //   S -> S + B[S mod 2],  B[p] = A_a[p] + A_b[(p + A_a[p]) mod 2]
 // (the parity after a is that of p + A_a[p]), valid while every intermediate
@@ -270,19 +386,28 @@ __device__ __forceinline__ ChunkMap cm_shfl_up(const ChunkMap &m, int d) {
   return o;
 }
 
-// Chains the chunk maps in order, exactly: one warp per axis (each on its own
-// SM), 32 chunks at a time.  The state (s, or S in ulps of binade e) is kept identical in every
+// Chains the chunk maps in order, exactly: one warp per axis and system, 32
+// chunks at a time.  The state (s, or S in ulps of binade e) is kept identical in every
 // lane.  From the current chunk j of a block, the lanes compose the maps of
 // chunks j..lane (a warp scan); the longest run of composites that is valid
-// for the exact S is applied in one step.  A chunk that no composite covers
-// (its map is missing or invalid for the exact state) is run 32 elements at a
-// time: the lanes scan the element maps from the exact S, a ballot finds the
+// for the exact S is applied in one step.  A chunk with a table takes that when
+// the state is close enough to its guess.  A chunk that neither covers is run 32
+// elements at a time: the lanes scan the element maps from the exact S, a ballot finds the
 // first element whose result leaves the binade, and only that element takes a
 // plain sequential FP64 add.
-__global__ void k_ss_chain(const double *__restrict__ pos, long N, long nchunks, const ChunkMap *maps, double *out) {
+__global__ void k_ss_chain(const SsArgs A, const double *start, const ChunkMap *maps, const double *tab, double *out) {
   __shared__ double sx[1][SS_C];
   const unsigned FULL = 0xffffffffu;
-  const int a = blockIdx.x, lane = threadIdx.x & 31;  // one axis per block, so per SM
+  const int a = blockIdx.x % 3, sys = blockIdx.x / 3, lane = threadIdx.x & 31;  // one axis of one system per block
+  const double *__restrict__ pos = A.pos;
+  long kb, ke;
+  A.chunks(sys, kb, ke);
+  const long nchunks = ke - kb, all = A.nchunks;
+  maps += a * all + kb;
+  start += a * all + kb;
+  if (tab) tab += (a * all + kb) * SS_TAB;
+  const long e0 = A.nsys > 1 ? A.sys_off[sys] : 0, N = (A.nsys > 1 ? A.sys_off[sys + 1] : A.N) - e0;
+  pos += 3 * e0;
   const long long LO = 1ll << 52, HI = 1ll << 53;
   double s = 0.0;
   bool imode = false;
@@ -292,13 +417,53 @@ __global__ void k_ss_chain(const double *__restrict__ pos, long N, long nchunks,
   // (such chunks come in runs: their loads overlap the previous one's work)
   long pref_k = -1;
   double pr[SS_PER_LANE];
-  ChunkMap nxt = lane < nchunks ? maps[a * nchunks + lane] : cm_identity();
+  ChunkMap nxt = lane < nchunks ? maps[lane] : cm_identity();
+  double nguess = lane < nchunks ? start[lane] : 0.0;
+  double nroom = tab && lane < nchunks ? tab[lane * SS_TAB + SS_TAB - 1] : 0.0;
   for (long k0 = 0; k0 < nchunks; k0 += 32) {
     const ChunkMap mo = nxt;  // this lane's chunk k0 + lane
-    if (k0 + 32 + lane < nchunks) nxt = maps[a * nchunks + k0 + 32 + lane];  // the next block's, ahead
+    const double guess = nguess, room = nroom;  // its guessed start; its table's room (0: none)
+    const long kn = k0 + 32 + lane;
+    if (kn < nchunks) {  // the next block's, ahead
+      nxt = maps[kn];
+      nguess = start[kn];
+      nroom = tab ? tab[kn * SS_TAB + SS_TAB - 1] : 0.0;
+    }
     const int nb = (int)min(32L, nchunks - k0);
+    // the block's chunks with a table; the first one's rows are requested now, each next one's with its turn
+    unsigned tabs = __ballot_sync(FULL, lane < nb && room > 0.0);
+    double after = tabs ? tab[(k0 + __ffs(tabs) - 1) * SS_TAB + lane] : 0.0;
     int j = 0;
     while (j < nb) {
+      const long k = k0 + j;
+      while (tabs && __ffs(tabs) - 1 < j) {  // passed by
+        tabs &= tabs - 1;
+        after = tabs ? tab[(k0 + __ffs(tabs) - 1) * SS_TAB + lane] : 0.0;
+      }
+      if (tabs && __ffs(tabs) - 1 == j) {  // ---- chunk j's table ----
+        const double row = after;
+        tabs &= tabs - 1;
+        after = tabs ? tab[(k0 + __ffs(tabs) - 1) * SS_TAB + lane] : 0.0;
+        const unsigned long long cur =
+            (unsigned long long)__double_as_longlong(imode ? ss_to_double(S, e) : s);
+        const unsigned long long g = (unsigned long long)__double_as_longlong(__shfl_sync(FULL, guess, j));
+        const unsigned long long mask = (1ull << SS_TBITS) - 1;
+        // distance to the run with the same last bits, in ulps of the start (a multiple of 32)
+        const long long d = (long long)(cur & ~mask) - (long long)(g & ~mask);
+        // sign and binade of the guess, and near enough to it
+        if ((cur >> 52) == (g >> 52) && (float)(d < 0 ? -d : d) < (float)__shfl_sync(FULL, room, j) * 0.999999f) {
+          const unsigned long long r =
+              (unsigned long long)__double_as_longlong(__shfl_sync(FULL, row, (int)(cur & mask)));
+          // the same distance in ulps of the result, whose magnitude grows with it where the signs agree
+          const int sh = (int)((g >> 52) & 0x7ff) - (int)((r >> 52) & 0x7ff);
+          const long long dr = sh >= 0 ? d << sh : d >> -sh;  // exact
+          s = __longlong_as_double((long long)(((g ^ r) >> 63) ? r - (unsigned long long)dr
+                                                               : r + (unsigned long long)dr));
+          imode = false;
+          j++;
+          continue;
+        }
+      }
       // the state in the binade of chunk j's map, when it has one
       const int ej = __shfl_sync(FULL, mo.e, j), okj = __shfl_sync(FULL, mo.ok, j);
       if (okj && (!imode || e != ej)) {
@@ -333,7 +498,6 @@ __global__ void k_ss_chain(const double *__restrict__ pos, long N, long nchunks,
         }
       }
       // ---- warp-parallel exact fallback over chunk k ----
-      const long k = k0 + j;
       long i0 = k * SS_C;
       int n = (int)(min(N, (k + 1) * SS_C) - i0);
       __syncwarp();
@@ -397,26 +561,46 @@ __global__ void k_ss_chain(const double *__restrict__ pos, long N, long nchunks,
   }
   if (lane == 0) {
     if (imode) s = ss_to_double(S, e);
-    out[a] = s;
+    out[3 * (long)sys + a] = s;
   }
 }
 
-// out[0..2] = the three sequential sums; scratch must hold fmm_seqsum_scratch(N) bytes
+// Scratch of fmm_seqsum3, without and with the tables.
 size_t fmm_seqsum_scratch(long N) {
   long nch = (N + SS_C - 1) / SS_C;
   return (size_t)nch * 3 * (2 * sizeof(double) + sizeof(ChunkMap)) + 256;
 }
+long fmm_seqsum_chunks(long n) { return (n + SS_C - 1) / SS_C; }
+size_t fmm_seqsum_scratch_tables(long chunks) {
+  return (size_t)chunks * 3 * (2 * sizeof(double) + sizeof(ChunkMap) + SS_TAB * sizeof(double)) + 256;
+}
 
-int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, cudaStream_t st) {
-  long nch = (N + SS_C - 1) / SS_C;
+static int seqsum_run(const SsArgs &A, double *out, void *scratch, bool tables, cudaStream_t st) {
+  const long nch = A.nchunks;
   double *csum = (double *)scratch;
   double *start = csum + 3 * nch;
   ChunkMap *maps = (ChunkMap *)(start + 3 * nch);
-  dim3 g((unsigned)((nch + 3) / 4), 3);
-  fmm_note_launch(), k_ss_chunksum<<<g, 128, 0, st>>>(pos, N, nch, csum);
-  fmm_note_launch(), k_ss_prefix<<<3, 1024, 0, st>>>(csum, nch, start);
-  fmm_note_launch(), k_ss_maps<<<g, 128, 0, st>>>(pos, N, nch, start, maps);
-  fmm_note_launch(), k_ss_chain<<<3, 32, 0, st>>>(pos, N, nch, maps, out);
+  double *tab = tables ? (double *)(maps + 3 * nch) : nullptr;
+  const dim3 g((unsigned)((nch + 3) / 4), 3);
+  const unsigned per = 3u * (unsigned)A.nsys;
+  fmm_note_launch(), k_ss_chunksum<<<g, 128, 0, st>>>(A, csum);
+  fmm_note_launch(), k_ss_prefix<<<per, A.nsys > 1 ? 128 : 1024, 0, st>>>(A, csum, start);
+  fmm_note_launch(), k_ss_maps<<<g, 128, 0, st>>>(A, start, maps);
+  if (tables) fmm_note_launch(), k_ss_tables<<<g, 128, 0, st>>>(A, start, maps, tab);
+  fmm_note_launch(), k_ss_chain<<<per, 32, 0, st>>>(A, start, maps, tab, out);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
+}
+
+// out[0..2] = the three sequential sums; scratch must hold fmm_seqsum_scratch(N)
+// bytes, or with `tables` fmm_seqsum_scratch_tables(fmm_seqsum_chunks(N))
+int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, bool tables, cudaStream_t st) {
+  return seqsum_run({pos, N, fmm_seqsum_chunks(N), 1, nullptr, nullptr}, out, scratch, tables, st);
+}
+
+// out[3 s .. 3 s + 2] = the sums of system s, whose chunks are [chunk_off[s], chunk_off[s + 1]) (device arrays);
+// scratch as with tables
+int fmm_seqsum3_systems(const double *pos, const long *sys_off, const int *chunk_off, int nsys, long chunks,
+                        double *out, void *scratch, cudaStream_t st) {
+  return seqsum_run({pos, 0, chunks, nsys, sys_off, chunk_off}, out, scratch, true, st);
 }

@@ -28,8 +28,11 @@
 // ---------------------------------------------------------------------------
 // The three sequential sums come from fmm_seqsum3 (seqsum.cu), bit-identical to
 // the reference's loop; the maxima are order-independent.
-size_t fmm_seqsum_scratch(long N);
-int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, cudaStream_t st);
+long fmm_seqsum_chunks(long n);
+size_t fmm_seqsum_scratch_tables(long chunks);
+int fmm_seqsum3_systems(const double *pos, const long *sys_off, const int *chunk_off, int nsys, long chunks,
+                        double *out, void *scratch, cudaStream_t st);
+int fmm_seqsum3(const double *pos, long N, double *out, void *scratch, bool tables, cudaStream_t st);
 
 __global__ void k_root_absmax(const double *__restrict__ pos, long N, const double *sums,
                               unsigned long long *mx) {
@@ -160,16 +163,6 @@ __global__ void k_init_roots(int nsys, const double *roots, const long *sys_off,
 __global__ void k_fill_psys(const long *sys_off, int *psys) {
   const int s = blockIdx.x;
   for (long i = sys_off[s] + threadIdx.x; i < sys_off[s + 1]; i += blockDim.x) psys[i] = s;
-}
-// The reference's three sequential FP64 sums, one thread per (system, axis).
-__global__ void k_seg_sums(const double *pos, const long *sys_off, int nsys, double *sums) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * nsys) return;
-  const int s = t / 3, ax = t - 3 * s;
-  double acc = 0.0;
-  const long e = sys_off[s + 1];
-  for (long i = sys_off[s]; i < e; i++) acc = __dadd_rn(acc, pos[3 * i + ax]);
-  sums[t] = acc;
 }
 // max |x - mean| per system and axis (order-independent), one block per system
 __global__ void k_seg_absmax(const double *pos, const long *sys_off, const double *sums, unsigned long long *mx) {
@@ -685,22 +678,27 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
   if (nsys == 1) {
     // one system: the exact sequential mean through fmm_seqsum3 (parallel)
     FMM_CUDA_TRY(cudaMemsetAsync(dr, 0, sizeof(double) * 16, st));
-    TRY(tmp_reserve(t, fmm_seqsum_scratch(N)));
-    TRY(fmm_seqsum3(pos, N, dr, t->tmp.p, st));
+    TRY(tmp_reserve(t, fmm_seqsum_scratch_tables(fmm_seqsum_chunks(N))));
+    TRY(fmm_seqsum3(pos, N, dr, t->tmp.p, true, st));
     unsigned nbm = std::min<unsigned>(fmm_blocks(N, 256), 152 * 8);
     fmm_note_launch(), k_root_absmax<<<nbm, 256, 0, st>>>(pos, N, dr, (unsigned long long *)(dr + 3));
     TRY(fmm_reserve(t->levf, FMM_MAXLEVEL + 1));
     fmm_note_launch(), k_root_final<<<1, 1, 0, st>>>(dr, (const unsigned long long *)(dr + 3), N, t->roots.p,
                                                      dr + 16, t->levf.p);
   } else {
-    // a forest: each system's sums by one thread (systems run side by side)
+    // a forest: each system's exact sequential means, side by side
     TRY(fmm_reserve(t->psys, N));
     fmm_note_launch(), k_fill_psys<<<nsys, 256, 0, st>>>(t->sys_off.p, t->psys.p);
-    TRY(tmp_reserve(t, sizeof(double) * 6 * (size_t)nsys + 64));
+    std::vector<int> co(nsys + 1, 0);
+    for (int k = 0; k < nsys; k++) co[k + 1] = co[k] + (int)fmm_seqsum_chunks(sys_off[k + 1] - sys_off[k]);
+    const size_t head = (sizeof(double) * 6 * (size_t)nsys + sizeof(int) * (nsys + 1) + 255) & ~(size_t)255;
+    TRY(tmp_reserve(t, head + fmm_seqsum_scratch_tables(co[nsys])));
     double *sums = (double *)t->tmp.p;
+    int *chunk_off = (int *)(sums + 6 * (size_t)nsys);
+    FMM_CUDA_TRY(cudaMemcpyAsync(chunk_off, co.data(), sizeof(int) * (nsys + 1), cudaMemcpyHostToDevice, st));
     unsigned long long *mx = (unsigned long long *)(sums + 3 * (size_t)nsys);
     FMM_CUDA_TRY(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) * 3 * nsys, st));
-    fmm_note_launch(), k_seg_sums<<<fmm_blocks(3 * (size_t)nsys, 128), 128, 0, st>>>(pos, t->sys_off.p, nsys, sums);
+    TRY(fmm_seqsum3_systems(pos, t->sys_off.p, chunk_off, nsys, co[nsys], sums, t->tmp.p + head, st));
     fmm_note_launch(), k_seg_absmax<<<nsys, 256, 0, st>>>(pos, t->sys_off.p, sums, mx);
     fmm_note_launch(), k_seg_root_final<<<fmm_blocks(nsys, 128), 128, 0, st>>>(nsys, t->sys_off.p, sums, mx,
                                                                                 t->roots.p);
