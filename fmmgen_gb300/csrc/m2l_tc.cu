@@ -1416,21 +1416,68 @@ int fmm_m2l_cm(DevTree *t, const float *M, int mstr, float *L, int lstr, const u
   return rc ? rc : fmm_mark_kernel(t, 1, st);
 }
 
-// key per target in processing order: its list length, longest first
-__global__ void k_h_lengths(const int *off, const int *order, int nc, unsigned *key, unsigned *val) {
+// The targets by list length, longest first: a histogram over the lengths (the
+// last bin: all longer ones), its prefix, and each target to its bin's next
+// place.  Targets of one length keep their processing order only roughly, as the
+// warps arrive; a target's sums do not depend on its neighbours.
+constexpr int H_BINS = 4096;
+__device__ __forceinline__ int h_bin(int len) { return H_BINS - 1 - min(len, H_BINS - 1); }
+__global__ void k_h_hist(const int *off, int nc, unsigned *bins) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nc) atomicAdd(&bins[h_bin(off[c + 1] - off[c])], 1u);
+}
+__global__ void __launch_bounds__(1024) k_h_prefix(unsigned *bins) {  // exclusive, in place
+  __shared__ unsigned wsum[32];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  constexpr int PER = H_BINS / 1024;
+  unsigned v[PER], s = 0;
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    v[k] = bins[PER * t + k];
+    s += v[k];
+  }
+  unsigned incl = s;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const unsigned o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) wsum[w] = incl;
+  __syncthreads();
+  unsigned base = incl - s;
+  for (int k = 0; k < w; k++) base += wsum[k];
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    bins[PER * t + k] = base;
+    base += v[k];
+  }
+}
+__global__ void k_h_targets(const int *off, const int *order, int nc, unsigned *bins, int *tgt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nc) return;
-  const int A = order[i];
-  key[i] = 65535u - (unsigned)min(off[A + 1] - off[A], 65535);
-  val[i] = (unsigned)A;
+  const int c = order[i];
+  tgt[atomicAdd(&bins[h_bin(off[c + 1] - off[c])], 1u)] = c;
 }
 
 int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st) {
   const int p = t->order, so = t->so, nc = t->ncells;
   if (p - so > 32) return FMM_ERR_STATE;
-  if (!ord && t->tgt_serial == t->build_serial && t->tgt_version == t->order_version) return FMM_OK;
+  if (!ord) {
+    if (t->tgt_serial == t->build_serial && t->tgt_version == t->order_version) return FMM_OK;
+    if (fmm_reserve(t->tp_tgt, nc) || fmm_reserve(t->tmp, H_BINS * sizeof(unsigned))) return FMM_ERR_CUDA;
+    unsigned *bins = (unsigned *)t->tmp.p;
+    FMM_CUDA_TRY(cudaMemsetAsync(bins, 0, H_BINS * sizeof(unsigned), st));
+    fmm_note_launch(), k_h_hist<<<fmm_blocks(nc, 256), 256, 0, st>>>(t->m2l_off.p, nc, bins);
+    fmm_note_launch(), k_h_prefix<<<1, 1024, 0, st>>>(bins);
+    fmm_note_launch(), k_h_targets<<<fmm_blocks(nc, 256), 256, 0, st>>>(t->m2l_off.p, t->m2l_order.p, nc, bins,
+                                                                        t->tp_tgt.p);
+    FMM_CUDA_TRY(cudaGetLastError());
+    t->tgt_serial = t->build_serial;
+    t->tgt_version = t->order_version;
+    return FMM_OK;
+  }
   const size_t nbh = fmm_rs_nblocks(nc), hist_n = 256 * nbh;
-  if (fmm_reserve(t->tp_tgt, nc) || (ord && fmm_reserve(t->tp_perm, (size_t)t->nm2l)) ||
+  if (fmm_reserve(t->tp_tgt, nc) || fmm_reserve(t->tp_perm, (size_t)t->nm2l) ||
       fmm_reserve(t->tmp, (size_t)nc * 12 + hist_n * 4 + fmm_scan_tmp_elems<uint32_t>(hist_n) * 4 + 256))
     return FMM_ERR_CUDA;
   char *q = t->tmp.p;
@@ -1439,14 +1486,9 @@ int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st) {
   uint32_t *v2 = (uint32_t *)q; q += (size_t)nc * 4;
   uint32_t *hist = (uint32_t *)q; q += hist_n * 4;
   uint32_t *stmp = (uint32_t *)q;
-  if (ord)
-    fmm_note_launch(), k_tp_perm<<<fmm_blocks((size_t)nc * 32, 256), 256, 0, st>>>(
-        t->m2l_off.p, ord, t->m2l_order.p, t->clevel.p, nc, so + 1, p, t->tp_perm.p, k1, (unsigned *)t->tp_tgt.p);
-  else
-    fmm_note_launch(), k_h_lengths<<<fmm_blocks(nc, 256), 256, 0, st>>>(t->m2l_off.p, t->m2l_order.p, nc, k1,
-                                                                        (unsigned *)t->tp_tgt.p);
+  t->tgt_serial = ~0ull;
+  fmm_note_launch(), k_tp_perm<<<fmm_blocks((size_t)nc * 32, 256), 256, 0, st>>>(
+      t->m2l_off.p, ord, t->m2l_order.p, t->clevel.p, nc, so + 1, p, t->tp_perm.p, k1, (unsigned *)t->tp_tgt.p);
   FMM_CUDA_TRY(cudaGetLastError());
-  t->tgt_serial = ord ? ~0ull : t->build_serial;
-  t->tgt_version = t->order_version;
-  return fmm_radix_sort<unsigned>(k1, (uint32_t *)t->tp_tgt.p, k2, v2, nc, 0, ord ? 32 : 16, hist, stmp, st);
+  return fmm_radix_sort<unsigned>(k1, (uint32_t *)t->tp_tgt.p, k2, v2, nc, 0, 32, hist, stmp, st);
 }

@@ -151,3 +151,19 @@ def test_handle_reuse(fg, oracle_lib):
     t2 = fg.build_tree(torch.tensor(b, device="cuda"), torch.tensor(q[:12000], device="cuda"), 12000, 64, 4, 0.5)
     assert (t.ncells, t.nm2l, t.np2p) == (t2.ncells, t2.nm2l, t2.np2p)
     assert all(np.array_equal(x, y) for x, y in zip(t.lists(), t2.lists()))
+
+
+@pytest.mark.parametrize("n,ncrit,theta,spread", [(65, 64, 0.5, 1), (900, 2, 0.5, 1), (4000, 3, 0.3, 1.5), (20000, 32, 0.5, 1),
+                                                  (20000, 16, 0.5, 1.5)])
+def test_lists_by_class(fg, oracle_lib, n, ncrit, theta, spread):
+    """The M2L lists, placed through atomics and ranked by class: the oracle's pairs, in the same order in every build
+    (few and many classes, targets of one pair and of hundreds), and the same bits from them."""
+    rng = np.random.default_rng(n + ncrit)
+    pos = (rng.uniform(-1, 1, (n, 3)) * rng.uniform(0, 1, (n, 1)) ** spread).copy()
+    S = rng.uniform(-1, 1, (n, 1))
+    t, _ = oracle_check(fg, oracle_lib, pos, S, ncrit, 4, theta)
+    lists, F = t.lists(), {k: t.compute_field_fmm(precision=k) for k in ("mixed", "fp64")}
+    for _ in range(3):
+        t.rebuild(torch.tensor(pos, device="cuda"))
+        assert all(np.array_equal(a, b) for a, b in zip(t.lists(), lists))
+        assert all(torch.equal(t.compute_field_fmm(precision=k), F[k]) for k in F)
