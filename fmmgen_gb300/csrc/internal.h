@@ -94,6 +94,14 @@ struct DevTree {
   DevBuf<int> p2p_off, p2p_src;
   DevBuf<int4> p2p_units;                 // near-field units: (cell, first target, targets <= 32, leaf)
   int np2p_units = 0;
+  // FP64 near field, each pair once (p2p.cu): per list entry its owner's place and the place to gather from
+  DevBuf<int> sym_own, sym_get;
+  DevBuf<uint32_t> sym_place;
+  DevBuf<int4> sym_units;
+  DevBuf<unsigned long long> sym_totals;
+  DevBuf<double> sym_shares;
+  long sym_places = 0, sym_nunits = 0;
+  uint64_t sym_serial = ~0ull;
   // M2L translation classes: operator vectors D^(k)(d/s_target), |k| <= order
   DevBuf<int> cls_key4;                   // [nclasses][4]: dlev, dx, dy, dz
   DevBuf<double> cls_D;                   // [nclasses][Nterms(order)]

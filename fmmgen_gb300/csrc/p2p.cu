@@ -183,6 +183,340 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int *leaf_cells,
 }
 
 // ---------------------------------------------------------------------------
+// P2P in FP64, each pair of particles once (charges and dipoles)
+// ---------------------------------------------------------------------------
+// Two leaves that list each other need the displacement, the distance and its
+// reciprocal powers of a pair of particles only once: 22.6 FP64 operations for
+// both directions instead of 2 x 17.6 (dipoles 37.6 instead of 2 x 25.6).  One
+// leaf of every such pair owns it (which one alternates with the cells'
+// parities, so that each leaf owns about half of its list): the sources' side is
+// added up in shared memory and left in a buffer, 32 bytes per particle of the
+// other leaf.  A unit of work is 32 entries of a leaf's list and one warp (a warp
+// per leaf made a tail of the densest ones: a single warp gets a quarter of its
+// SM's FP64 rate at most); it leaves its targets' sums in the buffer too, and
+// k_p2p64_gather adds a leaf's shares up in list order, so that every pass gives
+// the same bits, wherever in the buffer the shares lie.  In a step, the 32 lanes
+// are at 32 different staged sources, so that each adds to its own; a warp
+// barrier orders the steps.
+// An entry whose reverse is not listed (the walk gives symmetric lists; nothing
+// here relies on it) and the leaf itself go one way.  The buffer is at most
+// P64_SHARES; systems that would need more take k_p2p64.
+// Measured (one GB300): 10^6 charges: 158 -> 114 ms, the 86,400 dipoles 10.2 -> 8.8 ms.
+constexpr size_t P64_SHARES = (size_t)4 << 30;
+
+__device__ __forceinline__ bool p64_owns(int A, int B) { return ((A ^ B) & 1) ? A < B : A > B; }
+
+// Places in the buffer (in particles): for each leaf the sums of its units, one
+// after the other, then what its owned entries leave for their sources, place[k];
+// and the units (cell, leaf, batch of 32 entries).  totals: units, places (64 bits).
+__global__ void k_sym_places(const int *leaf_cells, int nleaves, const int *pcount, const int *off, const int *src,
+                             uint32_t *place, uint32_t *leaf_place, int4 *units, unsigned long long *totals) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int leaf = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (leaf >= nleaves) return;
+  const int A = leaf_cells[leaf], k0 = off[A], k1 = off[A + 1], nb = (k1 - k0 + 31) >> 5, na = pcount[A];
+  unsigned sum = 0;
+  for (int k = k0 + lane; k < k1; k += 32) {
+    const int B = src[k];
+    if (A != B && p64_owns(A, B)) sum += (unsigned)pcount[B];
+  }
+  for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+  unsigned long long at = 0, ub = 0;
+  if (lane == 0) {
+    at = atomicAdd(&totals[1], (unsigned long long)sum + (unsigned long long)na * nb);
+    ub = atomicAdd(&totals[0], (unsigned long long)nb);
+    leaf_place[leaf] = (uint32_t)at;
+  }
+  uint32_t run = __shfl_sync(FULL, (uint32_t)at, 0) + (uint32_t)(na * nb);
+  ub = __shfl_sync(FULL, ub, 0);
+  for (int b = lane; b < nb; b += 32) units[ub + b] = make_int4(A, leaf, b, 0);
+  for (int kb = k0; kb < k1; kb += 32) {
+    const int k = kb + lane, B = k < k1 ? src[k] : A;
+    const int n = A != B && p64_owns(A, B) ? pcount[B] : 0;
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(FULL, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (k < k1) place[k] = run + (uint32_t)(incl - n);
+    run += (uint32_t)__shfl_sync(FULL, incl, 31);
+  }
+}
+// own[k]: place of the shares entry k's target leaves for its source, -1: one way,
+// -2: the source owns the pair, and leaves the target's shares at get[k] (else -1).
+// One warp per unit.
+__global__ void k_sym_pairs(const int4 *units, const unsigned long long *totals, const int *off, const int *src,
+                            const uint32_t *place, int *own, int *get) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned long long u = blockIdx.x * 8ull + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (u >= totals[0]) return;
+  const int A = units[u].x, k = off[A] + 32 * units[u].z + lane;
+  const bool in = k < off[A + 1];
+  const int B = in ? src[k] : A;
+  int o = -1, g = -1;
+  const bool mine = A != B && p64_owns(A, B), seek = A != B && !mine;
+  if (mine) o = (int)place[k];
+  const int q0 = seek ? off[B] : 0, q1 = seek ? off[B + 1] : 0;
+  for (unsigned left = __ballot_sync(FULL, seek); left; left &= left - 1) {  // A's place in each such B's list
+    const int l = __ffs(left) - 1;
+    const int b0 = __shfl_sync(FULL, q0, l), b1 = __shfl_sync(FULL, q1, l);
+    int at = -1;
+    for (int q = b0; q < b1 && at < 0; q += 128) {
+      int v[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) v[r] = q + 32 * r + lane < b1 ? src[q + 32 * r + lane] : -1;
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const unsigned hit = __ballot_sync(FULL, v[r] == A);
+        if (hit && at < 0) at = q + 32 * r + __ffs(hit) - 1;
+      }
+    }
+    if (lane == l && at >= 0) {
+      o = -2;
+      g = (int)place[at];
+    }
+  }
+  if (in) {
+    own[k] = o;
+    get[k] = g;
+  }
+}
+
+// A pair of particles both ways: source jj (components sq[.][jj]) on the target
+// (si), and the target on the source, into acc[.][aj].  (dx, dy, dz) = target - source.
+template <int SO, bool POT, int STRIDE>
+__device__ __forceinline__ void p64_both(double dx, double dy, double dz, const double (*sq)[P64_CHUNK], int jj,
+                                         const double *si, double &phi, double &ex, double &ey, double &ez,
+                                         double (*acc)[STRIDE], int aj) {
+  constexpr int LAST = p64_nq(SO) - 1;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  const double rinv = rsqrt(r2), rr = rinv * rinv, r3 = rr * rinv;
+  if (SO == 0) {
+    const double qj = sq[0][jj], bj = qj * r3, bi = si[0] * r3;
+    if (POT) phi += qj * rinv;
+    ex += bj * dx;
+    ey += bj * dy;
+    ez += bj * dz;
+    if (POT) acc[0][aj] += si[0] * rinv;
+    acc[1][aj] -= bi * dx;
+    acc[2][aj] -= bi * dy;
+    acc[3][aj] -= bi * dz;
+  } else {
+    const double mx = sq[0][jj], my = sq[LAST > 1 ? 1 : 0][jj], mz = sq[LAST][jj], t3 = 3.0 * rr;
+    const double uj = (mx * dx + my * dy + mz * dz) * r3, wj = t3 * uj;
+    const double sx = si[0], sy = si[LAST > 1 ? 1 : 0], sz = si[LAST];
+    const double ui = (sx * dx + sy * dy + sz * dz) * r3, wi = t3 * ui;
+    if (POT) phi -= uj;
+    ex += mx * r3 - wj * dx;
+    ey += my * r3 - wj * dy;
+    ez += mz * r3 - wj * dz;
+    if (POT) acc[0][aj] += ui;  // seen from the source the displacement is -d
+    acc[1][aj] += sx * r3 - wi * dx;
+    acc[2][aj] += sy * r3 - wi * dy;
+    acc[3][aj] += sz * r3 - wi * dz;
+  }
+}
+
+struct P64Args {
+  const int4 *units;
+  const int *leaf_cells, *pstart, *pcount, *off, *src;
+  const double *px, *py, *pz;
+  const uint32_t *perm;
+  const double *S;
+  const int *own, *get;
+  const uint32_t *leaf_place;
+  double *shares;  // [places][4]
+  double *Fnear;
+};
+
+template <int SO, bool POT>
+__global__ void __launch_bounds__(32) k_p2p64_sym(const P64Args P) {
+  constexpr int NQ = p64_nq(SO);
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ double sp[3][P64_CHUNK], sq[NQ][P64_CHUNK], acc[4][32];
+  const int lane = threadIdx.x;
+  const int4 unit = P.units[blockIdx.x];
+  const int A = unit.x, a0 = P.pstart[A], na = P.pcount[A];
+  double *const mine_out = P.shares + 4 * ((size_t)P.leaf_place[unit.y] + (size_t)na * unit.z);
+  // up to 32 source leaves: lane q holds entry q's particle range and owner
+  const int k0 = P.off[A] + 32 * unit.z, nbat = min(32, P.off[A + 1] - k0);
+  int B = -1, start = 0, cnt = 0, own = -2;
+  if (lane < nbat) {
+    B = P.src[k0 + lane];
+    start = P.pstart[B];
+    cnt = P.pcount[B];
+    own = P.own[k0 + lane];
+  }
+  for (int tb = 0; tb < na;) {
+    // the next group of targets: 32 with a lane each, 16 with two, 8 with four, ...
+    // (25 to 31, or 13 to 15, idle a few lanes rather than go over the sources again)
+    const int rem = na - tb, lf = rem > 24 ? 0 : rem > 12 ? 1 : rem > 4 ? 2 : rem > 2 ? 3 : 4;
+    const int m = min(rem, 32 >> lf);
+    const int f = 1 << lf, steps = 32 >> lf;
+    const int tl = lane >> lf, slice = lane & (f - 1);
+    const bool ok = tl < m;
+    const int i = a0 + tb + (ok ? tl : 0);
+    const double xi = P.px[i], yi = P.py[i], zi = P.pz[i];
+    double si[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; k++) si[k] = P.S[NQ * (size_t)P.perm[i] + k];
+    double phi = 0, ex = 0, ey = 0, ez = 0;
+#pragma unroll 1
+    for (int both = 1; both >= 0; both--) {  // the owned leaves' particles, then those that go one way
+      const int mine = (both ? own >= 0 : own == -1) ? cnt : 0;
+      int incl = mine;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, d);
+        if (lane >= d) incl += v;
+      }
+      const int excl = incl - mine;
+      const int total = __shfl_sync(FULL, incl, 31);
+      const unsigned selfq = both ? 0u : __ballot_sync(FULL, B == A);
+      const int self_lo = selfq ? __shfl_sync(FULL, excl, __ffs(selfq) - 1) : -1;
+      for (int cb = 0; cb < total; cb += 32) {
+        const int n = min(32, total - cb), s = cb + lane;
+        int q = 0;
+#pragma unroll
+        for (int stp = 16; stp; stp >>= 1) {
+          const int v = __shfl_sync(FULL, excl, q + stp);
+          if (v <= s) q += stp;
+        }
+        const int at = s - __shfl_sync(FULL, excl, q);  // the source's place in its leaf
+        const int j = __shfl_sync(FULL, start, q) + at, base = __shfl_sync(FULL, own, q);
+        double *share = P.shares + 4 * ((size_t)(both ? base : 0) + at);
+        __syncwarp();
+        if (s < total) {
+          const size_t o = P.perm[j];
+          sp[0][lane] = P.px[j];
+          sp[1][lane] = P.py[j];
+          sp[2][lane] = P.pz[j];
+#pragma unroll
+          for (int k = 0; k < NQ; k++) sq[k][lane] = P.S[NQ * o + k];
+          if (both)  // this leaf's earlier groups have left their part
+#pragma unroll
+            for (int c = 0; c < 4; c++) acc[c][lane] = tb > 0 ? share[c] : 0.0;
+        }
+        __syncwarp();
+        if (!both) {
+          const int me = self_lo >= 0 ? self_lo + tb + tl - cb : -1;
+          if (ok)
+            for (int jj = slice; jj < n; jj += f)
+              p64_one<SO, true, POT>(xi - sp[0][jj], yi - sp[1][jj], zi - sp[2][jj], sq, jj, jj == me, phi, ex, ey, ez);
+          continue;
+        }
+        for (int st = 0; st < steps; st++) {
+          const int jj = (slice * steps + st + tl) & 31;
+          if (ok && jj < n) {
+            const double dx = xi - sp[0][jj], dy = yi - sp[1][jj], dz = zi - sp[2][jj];
+            p64_both<SO, POT, 32>(dx, dy, dz, sq, jj, si, phi, ex, ey, ez, acc, jj);
+          }
+          __syncwarp();
+        }
+        if (s < total)
+#pragma unroll
+          for (int c = POT ? 0 : 1; c < 4; c++) share[c] = acc[c][lane];
+      }
+    }
+    __syncwarp();
+    for (int o = 1; o < f; o <<= 1) {
+      phi += __shfl_xor_sync(FULL, phi, o);
+      ex += __shfl_xor_sync(FULL, ex, o);
+      ey += __shfl_xor_sync(FULL, ey, o);
+      ez += __shfl_xor_sync(FULL, ez, o);
+    }
+    if (ok && slice == 0) {
+      double *v = mine_out + 4 * (size_t)(tb + tl);
+      v[0] = phi;
+      v[1] = ex;
+      v[2] = ey;
+      v[3] = ez;
+    }
+    tb += m;
+  }
+}
+
+// A leaf's sums: each of its units' and, after it, the shares that the owners of
+// the unit's other pairs left, in list order.
+template <bool POT>
+__global__ void __launch_bounds__(128) k_p2p64_gather(const P64Args P, int nleaves) {
+  const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (leaf >= nleaves) return;
+  const int A = P.leaf_cells[leaf];
+  const int a0 = P.pstart[A], na = P.pcount[A], k0 = P.off[A], k1 = P.off[A + 1];
+  const double *own = P.shares + 4 * (size_t)P.leaf_place[leaf];
+  for (int tb = 0; tb < na; tb += 32) {
+    const int at = tb + lane;
+    double v[4] = {0, 0, 0, 0};
+    for (int kb = k0; kb < k1; kb += 32) {
+      if (at < na)
+#pragma unroll
+        for (int c = 0; c < 4; c++) v[c] += own[4 * ((size_t)na * ((kb - k0) >> 5) + at) + c];
+      const int g = kb + lane < k1 ? P.get[kb + lane] : -1;
+      unsigned has = __ballot_sync(0xffffffffu, g >= 0);
+      while (has) {
+        const int base = __shfl_sync(0xffffffffu, g, __ffs(has) - 1);
+        has &= has - 1;
+        if (at < na)
+#pragma unroll
+          for (int c = POT ? 0 : 1; c < 4; c++) v[c] += P.shares[4 * ((size_t)base + at) + c];
+      }
+    }
+    if (at < na)
+#pragma unroll
+      for (int c = 0; c < 4; c++) P.Fnear[4 * (size_t)(a0 + at) + c] = v[c];
+  }
+}
+
+// The owners and places of this build's pairs and room for the shares; *places:
+// particles in the buffer, or -1 where the pairs are to be done one way: more
+// shares than P64_SHARES, no memory to spare for them, or a capture of a build
+// whose pairs are not laid out yet.  Reads the totals back, once per build.
+static int p64_pairs(DevTree *t, long *places, cudaStream_t st) {
+  const int nl = t->nleaves;
+  *places = -1;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  FMM_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+  if (t->sym_serial != t->build_serial) {
+    if (cap != cudaStreamCaptureStatusNone) return FMM_OK;
+    const size_t n = (size_t)std::max(t->np2p, 1L), nu = (size_t)nl + n / 32;
+    if (fmm_reserve(t->sym_own, n) || fmm_reserve(t->sym_get, n) || fmm_reserve(t->sym_place, n + (size_t)nl) ||
+        fmm_reserve(t->sym_units, nu) || fmm_reserve(t->sym_totals, 2)) {
+      cudaGetLastError();
+      return FMM_OK;
+    }
+    FMM_CUDA_TRY(cudaMemsetAsync(t->sym_totals.p, 0, 2 * sizeof(unsigned long long), st));
+    fmm_note_launch(), k_sym_places<<<fmm_blocks(nl, 8), 256, 0, st>>>(
+        t->leaf_cells.p, nl, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->sym_place.p, t->sym_place.p + n,
+        t->sym_units.p, t->sym_totals.p);
+    fmm_note_launch(), k_sym_pairs<<<fmm_blocks(nu, 8), 256, 0, st>>>(t->sym_units.p, t->sym_totals.p, t->p2p_off.p,
+                                                                      t->p2p_src.p, t->sym_place.p, t->sym_own.p,
+                                                                      t->sym_get.p);
+    FMM_CUDA_TRY(cudaGetLastError());
+    unsigned long long v[2] = {0, 0};
+    FMM_CUDA_TRY(cudaMemcpyAsync(v, t->sym_totals.p, sizeof(v), cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    t->sym_nunits = (long)v[0];
+    t->sym_places = (long)v[1];
+    t->sym_serial = t->build_serial;
+  }
+  const size_t room = 4 * (size_t)std::max(t->sym_places, 1L);
+  if (room * sizeof(double) > P64_SHARES) return FMM_OK;
+  if (room > t->sym_shares.cap) {
+    size_t avail = 0, all = 0;  // an eighth of what is free at most: the rest of the pass needs its buffers too
+    if (cap != cudaStreamCaptureStatusNone || cudaMemGetInfo(&avail, &all) != cudaSuccess ||
+        room * sizeof(double) > avail / 8 || fmm_reserve(t->sym_shares, room)) {
+      cudaGetLastError();
+      return FMM_OK;
+    }
+  }
+  *places = t->sym_places;
+  return FMM_OK;
+}
+
+// ---------------------------------------------------------------------------
 
 // Per evaluate: positions as two-float offsets from the particle's system root
 // centre (hi in .xyz, the charge in .w; lo in .xyz, the particle's own index
@@ -558,9 +892,28 @@ int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st) {
                        t->iz.p, t->clevel.p, t->phi4.p, t->plo4.p, t->sdip.p, t->lorg.p, t->Fnear.p};
     if (int rc = fmm_mark_kernel(t, 2, st)) return rc;
     fmm_note_launch(), k<<<t->np2p_units, 32, 0, st>>>(P);
+    FMM_CUDA_TRY(cudaGetLastError());
+    return fmm_mark_kernel(t, 3, st);
+  }
+  const bool pot = t->pass_potential;
+  long places = -1;
+  if (so <= 1)
+    if (int rc = p64_pairs(t, &places, st)) return rc;
+  if (places >= 0) {
+    const P64Args P = {t->sym_units.p, t->leaf_cells.p, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p,
+                       t->py.p, t->pz.p, t->perm.p, S, t->sym_own.p, t->sym_get.p,
+                       t->sym_place.p + std::max(t->np2p, 1L), t->sym_shares.p, t->Fnear.p};
+    decltype(&k_p2p64_sym<0, true>) k = so == 0 ? (pot ? k_p2p64_sym<0, true> : k_p2p64_sym<0, false>)
+                                                : (pot ? k_p2p64_sym<1, true> : k_p2p64_sym<1, false>);
+    if (int rc = fmm_mark_kernel(t, 2, st)) return rc;
+    if (t->sym_nunits > 0) fmm_note_launch(), k<<<(unsigned)t->sym_nunits, 32, 0, st>>>(P);
+    const unsigned grid = fmm_blocks(nl, 4);
+    if (pot)
+      fmm_note_launch(), k_p2p64_gather<true><<<grid, 128, 0, st>>>(P, nl);
+    else
+      fmm_note_launch(), k_p2p64_gather<false><<<grid, 128, 0, st>>>(P, nl);
   } else {
     // a leaf holds fewer than ncrit particles (a root leaf fewer than N): its full chunks of 32, then three groups
-    const bool pot = t->pass_potential;
     const int nchunk = (int)(std::min(t->ncrit - 1, t->N) / 32);
     const int nlb = (int)fmm_blocks(nl, P2P_WARPS);
     decltype(&k_p2p64<0, true>) k = so == 0   ? (pot ? k_p2p64<0, true> : k_p2p64<0, false>)

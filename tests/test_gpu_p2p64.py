@@ -75,3 +75,26 @@ def test_direct(fg, n, nt, so):
     close(fg.direct(P, Q, targets=tt, source_order=so).cpu().numpy(), ref, mag, n)
     close(fg.direct(P, Q, targets=tt, source_order=so, field=False).cpu().numpy(), ref[:, :1], mag[:, :1], n)
     close(fg.direct(P, Q, targets=tt, source_order=so, potential=False).cpu().numpy(), ref[:, 1:], mag[:, 1:], n)
+
+
+@pytest.mark.parametrize("so", [0, 1])
+@pytest.mark.parametrize("n,ncrit,kind", [(300, 10, "uniform"), (900, 40, "plummer"), (1500, 70, "uniform"),
+                                          (2500, 130, "plummer"), (1200, 3, "uniform")])
+def test_pairs_once(fg, n, ncrit, kind, so):
+    """Trees of leaves of every group size, each pair of leaves worked off once by its owner: with theta so small that
+    no pair of cells is well separated the FMM is the pairwise sum; the same bits in every pass, and for the field
+    alone."""
+    pos, S = system(n, so, n + so)
+    if kind == "plummer":
+        pos = (pos - 0.5) * np.random.default_rng(n).uniform(0.01, 1, (n, 1)) ** 3
+    t = fg.build_tree(torch.tensor(pos, device="cuda"), torch.tensor(S, device="cuda"), n, ncrit, 4, 1e-3,
+                      source_order=so)
+    assert t.nleaves > 8 and t.nm2l == 0
+    ref, mag = pairwise(pos, S, so)
+    F = t.compute_field_fmm(precision="fp64")
+    close(F.cpu().numpy(), ref, mag, n)
+    assert torch.equal(t.compute_field_fmm(precision="fp64"), F)
+    assert torch.equal(t.compute_field_fmm(precision="fp64", potential=False), F[:, 1:])
+    fresh = fg.build_tree(torch.tensor(pos, device="cuda"), torch.tensor(S, device="cuda"), n, ncrit, 4, 1e-3,
+                          source_order=so)
+    assert torch.equal(fresh.rebuild_compute(precision="fp64"), F)
