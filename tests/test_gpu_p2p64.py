@@ -65,7 +65,7 @@ def test_one_leaf(fg, n, so):
 
 @pytest.mark.parametrize("so", [0, 1, 2])
 @pytest.mark.parametrize("n,nt", [(1, 1), (63, 2), (64, 5), (65, 31), (513, 32), (2000, 33), (2000, None), (9000, 3),
-                                  (9000, 700)])
+                                  (9000, 700), (4095, None), (4096, None), (4097, None), (4640, None), (5200, None)])
 def test_direct(fg, n, nt, so):
     pos, S = system(n, so, n + so)
     tg = None if nt is None else np.random.default_rng(3).integers(0, n, nt)
