@@ -248,7 +248,6 @@ __global__ void k_sym_places(const int *leaf_cells, int nleaves, const int *pcou
 // One warp per unit.
 __global__ void k_sym_pairs(const int4 *units, const unsigned long long *totals, const int *off, const int *src,
                             const uint32_t *place, int *own, int *get) {
-  constexpr unsigned FULL = 0xffffffffu;
   const unsigned long long u = blockIdx.x * 8ull + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (u >= totals[0]) return;
@@ -258,24 +257,17 @@ __global__ void k_sym_pairs(const int4 *units, const unsigned long long *totals,
   int o = -1, g = -1;
   const bool mine = A != B && p64_owns(A, B), seek = A != B && !mine;
   if (mine) o = (int)place[k];
-  const int q0 = seek ? off[B] : 0, q1 = seek ? off[B + 1] : 0;
-  for (unsigned left = __ballot_sync(FULL, seek); left; left &= left - 1) {  // A's place in each such B's list
-    const int l = __ffs(left) - 1;
-    const int b0 = __shfl_sync(FULL, q0, l), b1 = __shfl_sync(FULL, q1, l);
-    int at = -1;
-    for (int q = b0; q < b1 && at < 0; q += 128) {
-      int v[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) v[r] = q + 32 * r + lane < b1 ? src[q + 32 * r + lane] : -1;
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        const unsigned hit = __ballot_sync(FULL, v[r] == A);
-        if (hit && at < 0) at = q + 32 * r + __ffs(hit) - 1;
-      }
+  if (seek) {  // A's place in B's list, which is sorted
+    const int end = off[B + 1];
+    int lo = off[B], hi = end;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (src[mid] < A) lo = mid + 1;
+      else hi = mid;
     }
-    if (lane == l && at >= 0) {
+    if (lo < end && src[lo] == A) {
       o = -2;
-      g = (int)place[at];
+      g = (int)place[lo];
     }
   }
   if (in) {

@@ -167,3 +167,20 @@ def test_lists_by_class(fg, oracle_lib, n, ncrit, theta, spread):
         t.rebuild(torch.tensor(pos, device="cuda"))
         assert all(np.array_equal(a, b) for a, b in zip(t.lists(), lists))
         assert all(torch.equal(t.compute_field_fmm(precision=k), F[k]) for k in F)
+
+
+@pytest.mark.parametrize("n,ncrit,lo,hi", [(1, 2, 1, 2), (110, 3, 2, 129), (160, 2, 129, 257), (700, 2, 257, 1025),
+                                           (2000, 2, 1025, 4000)])
+def test_p2p_lists_sorted(fg, oracle_lib, n, ncrit, lo, hi):
+    """The near-field lists at the lengths at which their sort changes: with theta so small that no pair of cells is
+    separated every leaf's list is all leaves, in cell order; and the interaction count of all of them."""
+    rng = np.random.default_rng(n)
+    pos, S = rng.uniform(-1, 1, (n, 3)), rng.uniform(-1, 1, (n, 1))
+    t, _ = oracle_check(fg, oracle_lib, pos, S, ncrit, 4, 1e-3)
+    assert lo <= t.nleaves < hi
+    _, p2p = t.lists()
+    c = t.cells()
+    leaves = c["id"][c["count"] < ncrit]
+    assert np.array_equal(p2p.reshape(t.nleaves, t.nleaves, 2)[:, :, 0], np.repeat(leaves[:, None], t.nleaves, 1))
+    assert np.array_equal(p2p.reshape(t.nleaves, t.nleaves, 2)[:, :, 1], np.repeat(leaves[None], t.nleaves, 0))
+    assert t.p2p_interactions == n * (n - 1)
