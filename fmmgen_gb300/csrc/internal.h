@@ -66,7 +66,7 @@ struct DevTree {
   DevBuf<int> ix, iy, iz;                 // integer cell coordinates at the cell's level
   DevBuf<double> cr, crmax;               // half-width and rmax = sqrt(3 r r) (the reference's FP64 values)
   DevBuf<float2> crf;                     // half-width as an FP32 (hi, lo) pair
-  DevBuf<float> cmargin;                  // walk: relative MAC band decided in FP64 for pairs this cell refines
+  DevBuf<int4> wcell;                     // the walk's record of a cell (tree.cu), [2]
   DevBuf<int> csys;                       // system of the cell (forests of independent systems)
   DevBuf<int> pstart, pcount, parent, child_first;
   DevBuf<unsigned char> child_mask, clevel;
@@ -119,8 +119,9 @@ struct DevTree {
   DevBuf<int> fa, fb, fa2, fb2;           // traversal frontiers
   DevBuf<int> m2l_tgt_raw, m2l_src_raw;   // walk output in frontier order (kept between builds)
   DevBuf<int> p2p_tgt_raw, p2p_src_raw;
-  uint32_t *h_pinned = nullptr;           // 64 pinned host bytes for count readbacks
+  uint32_t *h_pinned = nullptr;           // 256 pinned host bytes for count readbacks
 #define FMM_PINNED_SCRATCH 8              // h_pinned word 8: the tensor-core schedule's step count
+#define FMM_PINNED_WALK 16                // h_pinned words 16..40: the walk's counters
 #define FMM_PINNED_TCERR 12               // h_pinned words 12..15: last tensor-core M2L error flags, class steps
   // tensor-core M2L operands (m2l_tc.cu)
   DevBuf<unsigned char> tc_T;             // split, swizzled operator records per class
@@ -145,7 +146,7 @@ struct DevTree {
   uint64_t sched_serial = ~0ull, sched_version = ~0ull;  // ... of this build and cell order
   uint64_t order_version = 0;             // incremented whenever m2l_order is rewritten
   int tc_order = -1, tc_so = -1;          // ... and to this expansion order and source order
-  DevBuf<unsigned char> wdec;             // decision of each frontier pair
+  DevBuf<unsigned char> d_walk;           // the walk's counters (tree.cu)
   DevBuf<char> tmp;                       // scan / sort / misc scratch
   DevBuf<uint32_t> d_eflags;
   DevBuf<double> d_root;                  // sums / maxima for the root box

@@ -305,11 +305,8 @@ __global__ void k_leaf_compact(int ncells, long ncrit, const int *pcount, const 
 // ---------------------------------------------------------------------------
 #define WALK_BS 256
 struct WalkCells {
+  const int4 *cell;  // per cell, one 32-byte sector: (ix, iy, iz, level + 256 children's mask), (first child, margin)
   const double *cx, *cy, *cz, *crmax;
-  const unsigned char *mask, *clevel;
-  const int *child_first;
-  const int *ix, *iy, *iz;
-  const float *margin;  // per cell: relative band around the MAC boundary decided in FP64
   float theta2;
 };
 
@@ -321,16 +318,17 @@ struct WalkCells {
 // `margin` of 1 -- where the rounding of the FP64 centres can matter -- is the
 // reference's own FP64 expression evaluated, with the same roundings.
 // Returns 0 = M2L, 1 = P2P, 2 = split A, 3 = split B.
-__device__ __forceinline__ int walk_decide(const WalkCells &W, int A, int B, double theta) {
-  const int la = W.clevel[A], lb = W.clevel[B], L = max(la, lb);
+__device__ __forceinline__ int walk_decide(const WalkCells &W, int A, int B, const int4 &a, const int4 &b, double theta) {
+  const int la = a.w & 255, lb = b.w & 255, L = max(la, lb);
   const int sa = L - la, sb = L - lb;
-  const long long gx = ((long long)(2 * W.ix[A] + 1) << sa) - ((long long)(2 * W.ix[B] + 1) << sb);
-  const long long gy = ((long long)(2 * W.iy[A] + 1) << sa) - ((long long)(2 * W.iy[B] + 1) << sb);
-  const long long gz = ((long long)(2 * W.iz[A] + 1) << sa) - ((long long)(2 * W.iz[B] + 1) << sb);
-  const long long n2 = gx * gx + gy * gy + gz * gz;
-  const long long base = (1ll << sa) + (1ll << sb);
-  const float rho = (float)n2 * W.theta2 / (3.f * (float)(base * base));
-  const float m = W.margin[la >= lb ? A : B];  // the band of the finer cell's level
+  // (coordinates below 2^23 are exact in FP32, and the margin holds the rounding of the rest)
+  const float gx = (float)(((2 * a.x + 1) << sa) - ((2 * b.x + 1) << sb));
+  const float gy = (float)(((2 * a.y + 1) << sa) - ((2 * b.y + 1) << sb));
+  const float gz = (float)(((2 * a.z + 1) << sa) - ((2 * b.z + 1) << sb));
+  const float base = (float)((1 << sa) + (1 << sb));
+  const float rho = (gx * gx + gy * gy + gz * gz) * W.theta2 / (3.f * base * base);
+  // the finer cell's band around the boundary
+  const float m = __int_as_float(W.cell[2 * (la >= lb ? A : B) + 1].y);
   bool mac;
   if (rho > 1.f + m) mac = true;
   else if (rho < 1.f - m) mac = false;
@@ -343,92 +341,138 @@ __device__ __forceinline__ int walk_decide(const WalkCells &W, int A, int B, dou
     mac = __dmul_rn(R, theta) > __dadd_rn(ra, rb);
   }
   if (mac) return 0;
-  bool leafa = W.mask[A] == 0, leafb = W.mask[B] == 0;
+  const bool leafa = (a.w >> 8) == 0, leafb = (b.w >> 8) == 0;
   if (leafa && leafb) return 1;  // the nleaf >= ncrit leaf-leaf branch is unreachable
   if (leafb || (la <= lb && !leafa)) return 2;  // rmax_A >= rmax_B  <=>  lA <= lB
   return 3;
 }
 
-// margin of each cell, for pairs in which it is the finer cell: FP32 evaluation
+// The walk's record of each cell.  Its margin, for pairs in which it is the finer cell: FP32 evaluation
 // error plus a bound on how far FP64 centre rounding can move R relative to the
 // cell half-width (from its system's root cube)
-__global__ void k_cell_margins(int nc, const int *csys, const double *roots, const double *cr, double theta,
-                               float *margin) {
+__global__ void k_walk_cells(int nc, const int *csys, const double *roots, const double *cr, double theta,
+                             const int *ix, const int *iy, const int *iz, const unsigned char *clevel,
+                             const unsigned char *mask, const int *child_first, int4 *cell) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
   const double *rt = roots + 4 * csys[c];
   const double cmax = fmax(fmax(fabs(rt[0]), fabs(rt[1])), fabs(rt[2])) + rt[3];
   const double s = cr[c];
   const double m = 1e-5 + 64.0 * ldexp(1.0, -52) * cmax / s * fmax(1.0, theta);
-  margin[c] = s > 0 && m < 0.01 ? (float)m : 1e30f;  // 1e30: always decide in FP64
+  const float margin = s > 0 && m < 0.01 ? (float)m : 1e30f;  // 1e30: always decide in FP64
+  cell[2 * c] = make_int4(ix[c], iy[c], iz[c], clevel[c] | (int)mask[c] << 8);
+  cell[2 * c + 1] = make_int4(child_first[c], __float_as_int(margin), 0, 0);
 }
 
-__global__ void k_root_pairs(int nsys, int *fa, int *fb) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nsys) fa[s] = fb[s] = s;
+// One level of the walk per launch: every frontier pair gives an M2L pair, a P2P
+// pair, or the split cell's children as pairs of the next frontier.  A block
+// counts the outputs of WALK_TILE pairs, takes their places with one atomic of each
+// kind and writes them, so the order within the lists and the frontier is that in
+// which the blocks arrive; what is built from them does not depend on it (the P2P
+// lists are sorted, the M2L lists ranked by class).  The sizes stay on the device,
+// so WALK_BATCH levels are launched before the host looks at them.  A level whose
+// outputs exceed a buffer writes only what fits and the levels after it do
+// nothing; the host then grows the buffer and starts again with that level, whose
+// frontier is still there.  A level's time is its blocks' chain of loads, barriers
+// and atomics (2 or 4 pairs a thread: the same).  Counting, scanning and writing in
+// three kernels, with the host waiting at every level, against this: a step of 10^4
+// charges 924 -> 803 us, of 10^6 7.94 -> 7.82 ms, of 2x10^6 Plummer dipoles (19 levels)
+// 23.2 -> 22.75 ms, of 512 systems 44.8 -> 44.3 ms.
+constexpr int WALK_BATCH = 8, WALK_IPT = 2, WALK_TILE = WALK_BS * WALK_IPT;
+struct WalkState {
+  uint32_t nf[WALK_BATCH + 1];                // frontier pairs of each level of the batch
+  uint32_t m2l[WALK_BATCH], p2p[WALK_BATCH];  // its outputs
+};
+struct WalkOut {
+  int *m2l_src, *m2l_tgt, *p2p_tgt, *p2p_src;
+  size_t cap_m2l, cap_p2p, cap_f[2];          // cap_f: the frontier written by the batch's even and odd levels
+  size_t m2l, p2p;                            // pairs written before this batch
+};
+// the batch's first frontier; of the whole walk: each system's (root, root) pair
+__global__ void k_walk_begin(WalkState *S, uint32_t nf, bool first, int *fa, int *fb) {
+  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (first && s < nf) fa[s] = fb[s] = (int)s;
+  if (s <= WALK_BATCH) S->nf[s] = s == 0 ? nf : 0;
+  if (s < WALK_BATCH) S->m2l[s] = S->p2p[s] = 0;
 }
-
-// Output slots of a decided pair: one M2L pair, one P2P pair, or the split
-// cell's children as new frontier pairs.
-__device__ __forceinline__ U3 walk_slots(const WalkCells &W, int A, int B, int d) {
-  U3 c{0u, 0u, 0u};
-  if (d == 0) c.x = 1;
-  else if (d == 1) c.y = 1;
-  else c.z = __popc((unsigned)W.mask[d == 2 ? A : B]);
-  return c;
-}
-
-// Decisions of the frontier pairs, and each block's slot totals (the per-pair
-// slots are recomputed by k_walk_write, so only the block totals are scanned).
-__global__ void __launch_bounds__(WALK_BS) k_walk_count(WalkCells W, const int *fa, const int *fb, uint32_t nf,
-                                                        double theta, U3 *bsum, unsigned char *dec) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  U3 c{0u, 0u, 0u};
-  if (i < nf) {
-    const int A = fa[i], B = fb[i];
-    const int d = walk_decide(W, A, B, theta);
-    dec[i] = (unsigned char)d;
-    c = walk_slots(W, A, B, d);
+__global__ void __launch_bounds__(WALK_BS) k_walk(WalkCells W, double theta, int lev, WalkState *S, WalkOut O,
+                                                  const int *fa, const int *fb, int *na, int *nb) {
+  __shared__ uint32_t s_at[3];
+  __shared__ uint64_t s_w[WALK_BS / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t nf = S->nf[lev];
+  size_t m0 = O.m2l, p0 = O.p2p;
+  bool over = false;
+  for (int j = 0; j < lev; j++) {
+    m0 += S->m2l[j];
+    p0 += S->p2p[j];
+    over |= S->nf[j + 1] > ((j & 1) ? O.cap_f[1] : O.cap_f[0]);
   }
-  U3 tot;
-  block_exclusive<U3>(c, &tot);
-  if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
-}
-
-// Writes each pair's outputs at its block's offset (boff, the scanned block
-// totals) plus its rank in the block: the walk order of the sequential scan.
-__global__ void __launch_bounds__(WALK_BS) k_walk_write(WalkCells W, const int *fa, const int *fb, uint32_t nf,
-                                                        const unsigned char *dec, const U3 *boff, U3 base,
-                                                        int *m2l_src, int *m2l_tgt, int *p2p_tgt, int *p2p_src,
-                                                        int *na, int *nb) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  int A = 0, B = 0, d = 0;
-  U3 c{0u, 0u, 0u};
-  if (i < nf) {
-    A = fa[i];
-    B = fb[i];
-    d = dec[i];
-    c = walk_slots(W, A, B, d);
-  }
-  U3 tot;
-  const U3 o = boff[blockIdx.x] + block_exclusive<U3>(c, &tot);
-  if (i >= nf) return;
-  if (d == 0) {
-    m2l_src[base.x + o.x] = B;
-    m2l_tgt[base.x + o.x] = A;
-  } else if (d == 1) {
-    p2p_tgt[base.y + o.y] = A;
-    p2p_src[base.y + o.y] = B;
-  } else {
-    int P = d == 2 ? A : B;
-    unsigned m = W.mask[P];
-    int ch = W.child_first[P];
-    uint32_t k = o.z;
-    for (int oc = 0; oc < 8; oc++) {
-      if (!(m & (1u << oc))) continue;
-      if (d == 2) { na[k] = ch; nb[k] = B; }
-      else { na[k] = A; nb[k] = ch; }
-      ch++; k++;
+  if (over || m0 > O.cap_m2l || p0 > O.cap_p2p) return;
+  const size_t capz = (lev & 1) ? O.cap_f[1] : O.cap_f[0];
+  for (size_t t0 = (size_t)blockIdx.x * WALK_TILE; t0 < nf; t0 += (size_t)gridDim.x * WALK_TILE) {
+    int A[WALK_IPT], B[WALK_IPT], d[WALK_IPT], nch[WALK_IPT];
+    uint64_t c = 0;  // outputs of the three kinds, 21 bits each
+#pragma unroll
+    for (int q = 0; q < WALK_IPT; q++) {
+      const size_t i = t0 + q * WALK_BS + threadIdx.x;
+      d[q] = -1;
+      if (i < nf) {
+        A[q] = fa[i];
+        B[q] = fb[i];
+        const int4 a = W.cell[2 * A[q]], b = W.cell[2 * B[q]];
+        d[q] = walk_decide(W, A[q], B[q], a, b, theta);
+        nch[q] = __popc((unsigned)(d[q] == 2 ? a.w : b.w) >> 8);
+        c += d[q] == 0 ? 1ull : d[q] == 1 ? 1ull << 21 : (uint64_t)nch[q] << 42;
+      }
+    }
+    uint64_t e = c;  // exclusive over the block
+#pragma unroll
+    for (int sh = 1; sh < 32; sh <<= 1) {
+      const uint64_t v = __shfl_up_sync(0xffffffffu, e, sh);
+      if (lane >= sh) e += v;
+    }
+    if (lane == 31) s_w[w] = e;
+    __syncthreads();
+    e -= c;
+    uint64_t tot = 0;
+#pragma unroll
+    for (int k = 0; k < WALK_BS / 32; k++) {
+      const uint64_t v = s_w[k];
+      tot += v;
+      if (k < w) e += v;
+    }
+    if (threadIdx.x < 3) {
+      const uint32_t n = (uint32_t)(tot >> (21 * threadIdx.x)) & 0x1fffffu;
+      uint32_t *at = threadIdx.x == 0 ? &S->m2l[lev] : threadIdx.x == 1 ? &S->p2p[lev] : &S->nf[lev + 1];
+      s_at[threadIdx.x] = n ? atomicAdd(at, n) : 0;
+    }
+    __syncthreads();
+    size_t x = m0 + s_at[0] + ((uint32_t)e & 0x1fffffu), y = p0 + s_at[1] + ((uint32_t)(e >> 21) & 0x1fffffu);
+    size_t z = (size_t)s_at[2] + (uint32_t)(e >> 42);
+#pragma unroll
+    for (int q = 0; q < WALK_IPT; q++) {
+      if (d[q] < 0) continue;
+      if (d[q] == 0) {
+        if (x < O.cap_m2l) {
+          O.m2l_src[x] = B[q];
+          O.m2l_tgt[x] = A[q];
+        }
+        x++;
+      } else if (d[q] == 1) {
+        if (y < O.cap_p2p) {
+          O.p2p_tgt[y] = A[q];
+          O.p2p_src[y] = B[q];
+        }
+        y++;
+      } else {
+        const int ch = W.cell[2 * (d[q] == 2 ? A[q] : B[q]) + 1].x;
+        for (int k = 0; k < nch[q]; k++, z++)
+          if (z < capz) {
+            na[z] = d[q] == 2 ? ch + k : A[q];
+            nb[z] = d[q] == 2 ? B[q] : ch + k;
+          }
+      }
     }
   }
 }
@@ -468,14 +512,13 @@ __global__ void k_csr_from_sorted(const K *keys, long n, int cbits, int nc, int 
 // the distinct keys in that order.
 #define CLS_EMPTY 0xffffffffffffffffull
 #define CLS_LIM (1LL << 18)
-__device__ __forceinline__ uint64_t pair_key(const int *ix, const int *iy, const int *iz, const unsigned char *clevel,
-                                             int A, int B) {
-  const int la = clevel[A], lb = clevel[B];
+__device__ __forceinline__ uint64_t pair_key(const int4 a, const int4 b) {  // the walk's records of A and B
+  const int la = a.w & 255, lb = b.w & 255;
   const int L = la > lb ? la : lb;
   const int sa = L - la, sb = L - lb;
-  const long long dx = ((2LL * ix[A] + 1) << sa) - ((2LL * ix[B] + 1) << sb);
-  const long long dy = ((2LL * iy[A] + 1) << sa) - ((2LL * iy[B] + 1) << sb);
-  const long long dz = ((2LL * iz[A] + 1) << sa) - ((2LL * iz[B] + 1) << sb);
+  const long long dx = ((2LL * a.x + 1) << sa) - ((2LL * b.x + 1) << sb);
+  const long long dy = ((2LL * a.y + 1) << sa) - ((2LL * b.y + 1) << sb);
+  const long long dz = ((2LL * a.z + 1) << sa) - ((2LL * b.z + 1) << sb);
   if (llabs(dx) >= CLS_LIM || llabs(dy) >= CLS_LIM || llabs(dz) >= CLS_LIM) return CLS_EMPTY;
   return ((uint64_t)(lb - la + 64) << 57) | ((uint64_t)(dx + CLS_LIM) << 38) | ((uint64_t)(dy + CLS_LIM) << 19) |
          (uint64_t)(dz + CLS_LIM);
@@ -508,12 +551,11 @@ __device__ __forceinline__ long key_find(const uint64_t *tab, uint32_t mask, uin
 
 // Class key of every pair, inserted into the table; stat[0] counts distinct
 // keys, stat[1] flags a table that filled up.
-__global__ void k_class_keys(const int *src, const int *tgt, long n, const int *ix, const int *iy, const int *iz,
-                             const unsigned char *clevel, uint64_t *keys, uint64_t *tab, uint32_t mask,
-                             uint32_t *stat, uint32_t *eflags) {
+__global__ void k_class_keys(const int *src, const int *tgt, long n, const int4 *cell, uint64_t *keys, uint64_t *tab,
+                             uint32_t mask, uint32_t *stat, uint32_t *eflags) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint64_t k = pair_key(ix, iy, iz, clevel, tgt[i], src[i]);
+  const uint64_t k = pair_key(cell[2 * tgt[i]], cell[2 * src[i]]);
   keys[i] = k;
   if (k == CLS_EMPTY) {
     atomicOr(eflags, FMM_EFLAG_RANGE);
@@ -679,8 +721,8 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
     t->ev_ready = true;
   }
   if (!t->h_pinned) {
-    FMM_CUDA_TRY(cudaMallocHost((void **)&t->h_pinned, 64));
-    memset(t->h_pinned, 0, 64);
+    FMM_CUDA_TRY(cudaMallocHost((void **)&t->h_pinned, 256));
+    memset(t->h_pinned, 0, 256);
   }
   t->build_serial++;
   TRY(rec(t, 0, st));
@@ -879,9 +921,10 @@ static int build_cells(DevTree *t, cudaStream_t st, int nlev, bool *deeper) {
     FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, 2 * sizeof(uint32_t), st));
     return FMM_OK;
   }
-  TRY(fmm_reserve(t->cmargin, nc));
-  fmm_note_launch(), k_cell_margins<<<fmm_blocks(nc, 256), 256, 0, st>>>(nc, t->csys.p, t->roots.p, t->cr.p,
-                                                                          t->theta, t->cmargin.p);
+  TRY(fmm_reserve(t->wcell, 2 * (size_t)nc));
+  fmm_note_launch(), k_walk_cells<<<fmm_blocks(nc, 256), 256, 0, st>>>(
+      nc, t->csys.p, t->roots.p, t->cr.p, t->theta, t->ix.p, t->iy.p, t->iz.p, t->clevel.p, t->child_mask.p,
+      t->child_first.p, t->wcell.p);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
 }
@@ -1077,59 +1120,78 @@ static int p2p_lists(DevTree *t, cudaStream_t st) {
   return FMM_OK;
 }
 
+// blocks that fill the SMs, eight of 256 threads each
+constexpr size_t WALK_GRID = 152 * 8;
 static int build_lists(DevTree *t, cudaStream_t st) {
-  int nc = t->ncells;
-  WalkCells W{t->cx.p, t->cy.p, t->cz.p, t->crmax.p, t->child_mask.p, t->clevel.p, t->child_first.p,
-              t->ix.p, t->iy.p, t->iz.p, t->cmargin.p, (float)(t->theta * t->theta)};
-  // raw lists in walk order; the buffers keep their capacity between builds,
-  // so a rebuild of a similar tree allocates nothing
+  const int nc = t->ncells;
+  const WalkCells W{t->wcell.p, t->cx.p, t->cy.p, t->cz.p, t->crmax.p, (float)(t->theta * t->theta)};
+  // raw lists in the walk's order; the buffers keep their capacity between
+  // builds, so a rebuild of a similar tree allocates nothing.  At first: what
+  // uniform and clustered trees need (a list of up to ~480 M2L and 140 P2P
+  // sources a cell), or less where that is more than an eighth of the free memory
   DevBuf<int> &m2l_src_raw = t->m2l_src_raw, &m2l_tgt_raw = t->m2l_tgt_raw;
   DevBuf<int> &p2p_tgt_raw = t->p2p_tgt_raw, &p2p_src_raw = t->p2p_src_raw;
-  size_t cap_pairs = (size_t)nc * 64 + 1024 + t->nsys;
-  TRY(fmm_reserve(t->fa, cap_pairs)); TRY(fmm_reserve(t->fb, cap_pairs));
-  TRY(fmm_reserve(t->fa2, cap_pairs)); TRY(fmm_reserve(t->fb2, cap_pairs));
-  TRY(fmm_reserve(m2l_src_raw, cap_pairs)); TRY(fmm_reserve(m2l_tgt_raw, cap_pairs));
-  TRY(fmm_reserve(p2p_tgt_raw, cap_pairs)); TRY(fmm_reserve(p2p_src_raw, cap_pairs));
-  int rc = FMM_OK;
-  long nm2l = 0, np2p = 0;
-  // the walk starts from each system's (root, root) pair
-  uint32_t nf = (uint32_t)t->nsys;
-  U3 *h_tot = (U3 *)t->h_pinned;
-  fmm_note_launch(), k_root_pairs<<<fmm_blocks(nf, 256), 256, 0, st>>>((int)nf, t->fa.p, t->fb.p);
-  FMM_CUDA_TRY(cudaGetLastError());
-  while (nf > 0) {
-    const unsigned nblk = fmm_blocks(nf, WALK_BS);
-    size_t need = (size_t)nblk * sizeof(U3) + fmm_scan_tmp_elems<U3>(nblk) * sizeof(U3) + 2 * sizeof(U3);
-    if ((rc = tmp_reserve(t, need))) break;
-    U3 *cnt = (U3 *)t->tmp.p;  // per block: slot totals, then their exclusive scan
-    U3 *tot = cnt + nblk;
-    U3 *stmp = tot + 1;
-    if ((rc = fmm_reserve(t->wdec, nf))) break;
-    fmm_note_launch(), k_walk_count<<<nblk, WALK_BS, 0, st>>>(W, t->fa.p, t->fb.p, nf, t->theta, cnt, t->wdec.p);
-    if ((rc = fmm_scan<U3>(cnt, cnt, nblk, tot, stmp, st))) break;
-    cudaMemcpyAsync(h_tot, tot, sizeof(U3), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) { rc = FMM_ERR_CUDA; break; }
-    U3 T = *h_tot;
-    if ((rc = grow_keep(m2l_src_raw, nm2l + T.x, nm2l, st)) || (rc = grow_keep(m2l_tgt_raw, nm2l + T.x, nm2l, st)) ||
-        (rc = grow_keep(p2p_tgt_raw, np2p + T.y, np2p, st)) || (rc = grow_keep(p2p_src_raw, np2p + T.y, np2p, st)) ||
-        (rc = fmm_reserve(t->fa2, T.z + 1)) || (rc = fmm_reserve(t->fb2, T.z + 1)))
-      break;
-    U3 base{(uint32_t)nm2l, (uint32_t)np2p, 0u};
-    fmm_note_launch(), k_walk_write<<<nblk, WALK_BS, 0, st>>>(W, t->fa.p, t->fb.p, nf, t->wdec.p, cnt, base,
-                                                     m2l_src_raw.p, m2l_tgt_raw.p, p2p_tgt_raw.p, p2p_src_raw.p,
-                                                     t->fa2.p, t->fb2.p);
-    if (cudaGetLastError() != cudaSuccess) { rc = FMM_ERR_CUDA; break; }
-    nm2l += T.x;
-    np2p += T.y;
-    nf = T.z;
-    std::swap(t->fa, t->fa2);
-    std::swap(t->fb, t->fb2);
+  DevBuf<int> *fr[2][2] = {{&t->fa, &t->fb}, {&t->fa2, &t->fb2}};
+  TRY(fmm_reserve(t->d_walk, sizeof(WalkState)));
+  WalkState *S = (WalkState *)t->d_walk.p, *H = (WalkState *)(t->h_pinned + FMM_PINNED_WALK);
+  const size_t all = (size_t)nc * nc;
+  auto room = [&](size_t m2l, size_t p2p, size_t f) {
+    const size_t cm = std::min(m2l * nc, all) + 1024 + t->nsys, cp = std::min(p2p * nc, all) + 1024 + t->nsys,
+                 cf = std::min(f * nc, all) + 1024 + t->nsys;
+    for (auto &b : fr)
+      if (fmm_reserve(*b[0], cf) || fmm_reserve(*b[1], cf)) return FMM_ERR_CUDA;
+    return fmm_reserve(m2l_src_raw, cm) || fmm_reserve(m2l_tgt_raw, cm) || fmm_reserve(p2p_tgt_raw, cp) ||
+                   fmm_reserve(p2p_src_raw, cp)
+               ? FMM_ERR_CUDA
+               : FMM_OK;
+  };
+  size_t avail = ~(size_t)0, total = 0;
+  if (m2l_src_raw.cap < std::min((size_t)480 * nc, all) && cudaMemGetInfo(&avail, &total) != cudaSuccess) avail = 0;
+  if (avail / 8 < (size_t)nc * 4 * (2 * 480 + 2 * 160 + 4 * 320) || room(480, 160, 320)) {
+    cudaGetLastError();
+    TRY(room(64, 64, 64));
   }
-  if (rc) return rc;
+  size_t nm2l = 0, np2p = 0;
+  uint32_t nf = (uint32_t)t->nsys;
+  int cur = 0;  // the frontier to read
+  for (bool first = true; nf > 0; first = false) {
+    fmm_note_launch(), k_walk_begin<<<fmm_blocks(first ? std::max(nf, 32u) : 32, 256), 256, 0, st>>>(
+        S, nf, first, fr[cur][0]->p, fr[cur][1]->p);
+    auto cap2 = [](const DevBuf<int> &a, const DevBuf<int> &b) { return std::min(a.cap, b.cap); };
+    const WalkOut O = {m2l_src_raw.p, m2l_tgt_raw.p, p2p_tgt_raw.p, p2p_src_raw.p, cap2(m2l_src_raw, m2l_tgt_raw),
+                       cap2(p2p_tgt_raw, p2p_src_raw),
+                       {cap2(*fr[cur ^ 1][0], *fr[cur ^ 1][1]), cap2(*fr[cur][0], *fr[cur][1])}, nm2l, np2p};
+    size_t most = nf;  // pairs the level can have
+    for (int l = 0; l < WALK_BATCH; l++) {
+      const int rd = cur ^ (l & 1);
+      const size_t nb = std::min<size_t>((most + WALK_TILE - 1) / WALK_TILE, WALK_GRID);
+      fmm_note_launch(), k_walk<<<(unsigned)nb, WALK_BS, 0, st>>>(W, t->theta, l, S, O, fr[rd][0]->p, fr[rd][1]->p,
+                                                                  fr[rd ^ 1][0]->p, fr[rd ^ 1][1]->p);
+      most = std::min(8 * most, (size_t)1 << 32);
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+    FMM_CUDA_TRY(cudaMemcpyAsync(H, S, sizeof(WalkState), cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    int l = 0;
+    for (; l < WALK_BATCH && H->nf[l] > 0; l++) {
+      const size_t m1 = nm2l + H->m2l[l], p1 = np2p + H->p2p[l];
+      const size_t f1 = H->nf[l + 1];
+      if (m1 > O.cap_m2l || p1 > O.cap_p2p || f1 > O.cap_f[l & 1]) {  // grow, and again from this level
+        TRY(grow_keep(m2l_src_raw, m1, nm2l, st)); TRY(grow_keep(m2l_tgt_raw, m1, nm2l, st));
+        TRY(grow_keep(p2p_tgt_raw, p1, np2p, st)); TRY(grow_keep(p2p_src_raw, p1, np2p, st));
+        for (DevBuf<int> *b : fr[cur ^ 1 ^ (l & 1)]) TRY(fmm_reserve(*b, f1 + f1 / 2));
+        break;
+      }
+      nm2l = m1;
+      np2p = p1;
+    }
+    nf = H->nf[l];
+    cur ^= l & 1;
+  }
   // the M2L pairs stay in walk order here: build_classes groups them by
   // (target, class) once the classes are known
-  t->nm2l = nm2l;
-  t->np2p = np2p;
+  t->nm2l = (long)nm2l;
+  t->np2p = (long)np2p;
   return p2p_lists(t, st);
 }
 
@@ -1179,9 +1241,8 @@ static int build_classes(DevTree *t, cudaStream_t st) {
     TRY(fmm_reserve(t->cls_hkeys, hsize));
     FMM_CUDA_TRY(cudaMemsetAsync(t->cls_hkeys.p, 0xff, sizeof(uint64_t) * hsize, st));  // all CLS_EMPTY
     FMM_CUDA_TRY(cudaMemsetAsync(stat, 0, 4 * sizeof(uint32_t), st));
-    fmm_note_launch(), k_class_keys<<<fmm_blocks(n, 256), 256, 0, st>>>(src, tgt, n, t->ix.p, t->iy.p, t->iz.p,
-                                                                        t->clevel.p, keys, t->cls_hkeys.p,
-                                                                        hsize - 1, stat, t->d_eflags.p);
+    fmm_note_launch(), k_class_keys<<<fmm_blocks(n, 256), 256, 0, st>>>(src, tgt, n, t->wcell.p, keys,
+                                                                        t->cls_hkeys.p, hsize - 1, stat, t->d_eflags.p);
     FMM_CUDA_TRY(cudaGetLastError());
     FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned, stat, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     FMM_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1413,12 +1474,12 @@ void fmm_tree_destroy(DevTree *t) {
   t->cm_wserial = ~0ull;
   t->sched_serial = ~0ull;
   t->tc_serial = ~0ull;
-  fmm_release(t->wdec);
+  fmm_release(t->d_walk);
   fmm_release(t->d_p2pcount);
   fmm_release(t->m2l_ord); fmm_release(t->mnorm); fmm_release(t->feat); fmm_release(t->tscale); fmm_release(t->tpart);
   fmm_release(t->sys_pairs);
   fmm_release(t->ltgt);
-  fmm_release(t->cr); fmm_release(t->crmax); fmm_release(t->crf); fmm_release(t->cmargin); fmm_release(t->csys);
+  fmm_release(t->cr); fmm_release(t->crmax); fmm_release(t->crf); fmm_release(t->wcell); fmm_release(t->csys);
   fmm_release(t->sys_off); fmm_release(t->psys); fmm_release(t->roots);
   fmm_release(t->tmp); fmm_release(t->d_eflags); fmm_release(t->d_root);
   if (t->h_pinned) cudaFreeHost(t->h_pinned);
