@@ -119,9 +119,10 @@ struct DevTree {
   DevBuf<int> fa, fb, fa2, fb2;           // traversal frontiers
   DevBuf<int> m2l_tgt_raw, m2l_src_raw;   // walk output in frontier order (kept between builds)
   DevBuf<int> p2p_tgt_raw, p2p_src_raw;
-  uint32_t *h_pinned = nullptr;           // 256 pinned host bytes for count readbacks
+  uint32_t *h_pinned = nullptr;           // pinned host words for count readbacks
+#define FMM_PINNED_WORDS 64
 #define FMM_PINNED_SCRATCH 8              // h_pinned word 8: the tensor-core schedule's step count
-#define FMM_PINNED_WALK 16                // h_pinned words 16..40: the walk's counters
+#define FMM_PINNED_WALK 16                // h_pinned words 16..63: the cells', then the walk's counters
 #define FMM_PINNED_TCERR 12               // h_pinned words 12..15: last tensor-core M2L error flags, class steps
   // tensor-core M2L operands (m2l_tc.cu)
   DevBuf<unsigned char> tc_T;             // split, swizzled operator records per class

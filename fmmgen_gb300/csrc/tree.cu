@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <cooperative_groups.h>
 #include "internal.h"
 #include "prims.cuh"
 #include "deriv.cuh"
@@ -215,89 +216,192 @@ __global__ void k_apply_order(const uint32_t *idx, long N, const uint64_t *kin, 
   pout[i] = pin[idx[i]];
 }
 
-// One warp per cell of the level: lane o (1..7) finds where digit o starts in
-// the cell's sorted keys, so the eight child ranges come from seven searches
-// side by side; bnd[9 (c - lo) + o] = first particle of child o (bnd[.. + 8] = end).
-__global__ void k_count_children(int lo, int hi, int level, int nlev, long ncrit, const uint64_t *keys,
-                                 const int *pstart, const int *pcount, unsigned char *child_mask, uint32_t *cnt,
-                                 int *bnd, uint32_t *eflags) {
-  const int c = lo + (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (c >= hi) return;
-  const int s = pstart[c], e = s + pcount[c];
-  const bool split = pcount[c] >= ncrit && level < nlev;
-  int b = lane == 0 ? s : e;
-  if (split && lane >= 1 && lane <= 7) b = lower_digit(keys, s, e, level + 1, lane);
-  if (lane <= 8) bnd[9 * (c - lo) + lane] = b;
-  // child o holds [bnd[o], bnd[o + 1])
-  const int nb = __shfl_down_sync(0xffffffffu, b, 1);
-  const unsigned mask = __ballot_sync(0xffffffffu, split && lane < 8 && nb > b) & 0xffu;
-  if (lane == 0) {
-    if (pcount[c] >= ncrit && level >= nlev)  // no digits below: give up, or ask for all levels
-      atomicOr(eflags, nlev >= FMM_MAXLEVEL ? FMM_EFLAG_DEPTH : FMM_EFLAG_KEYS);
-    child_mask[c] = (unsigned char)mask;
-    cnt[c - lo] = (uint32_t)__popc(mask);
-  }
+// The walk's margin of a cell, for pairs in which it is the finer cell: FP32
+// evaluation error plus a bound on how far FP64 centre rounding can move R relative
+// to the cell half-width s (rt: its system's root cube)
+__device__ __forceinline__ float cell_margin(const double *rt, double s, double theta) {
+  const double cmax = fmax(fmax(fabs(rt[0]), fabs(rt[1])), fabs(rt[2])) + rt[3];
+  const double m = 1e-5 + 64.0 * ldexp(1.0, -52) * cmax / s * fmax(1.0, theta);
+  return s > 0 && m < 0.01 ? (float)m : 1e30f;  // 1e30: always decide in FP64
 }
 
-// One warp per cell: lane o writes child o, when it exists.
-__global__ void k_write_children(int lo, int hi, int level, const uint32_t *off, const int *bnd, double *cx,
-                                 double *cy, double *cz, uint64_t *cid, int *ix, int *iy, int *iz, int *pstart,
-                                 int *pcount, int *parent, int *child_first, const unsigned char *child_mask_in,
-                                 unsigned char *child_mask, unsigned char *clevel, double *cr, double *crmax,
-                                 float2 *crf, int *csys) {
-  const int c = lo + (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), o = threadIdx.x & 31;
-  if (c >= hi) return;
-  const unsigned mask = child_mask_in[c];
-  const int first = hi + (int)off[c - lo];
-  if (o == 0) child_first[c] = mask ? first : -1;
-  if (o >= 8 || !((mask >> o) & 1u)) return;
-  const int j = first + __popc(mask & ((1u << o) - 1u));
-  const double r = __ddiv_rn(cr[c], 2.0);  // child half-width = parent r / 2.0 (example/tree.cpp:95)
-  const int b = bnd[9 * (c - lo) + o], nb = bnd[9 * (c - lo) + o + 1];
-  // add_child (example/tree.cpp:95-98)
-  cx[j] = __dadd_rn(cx[c], (o & 1) ? r : -r);
-  cy[j] = __dadd_rn(cy[c], (o & 2) ? r : -r);
-  cz[j] = __dadd_rn(cz[c], (o & 4) ? r : -r);
-  cid[j] = (cid[c] << 3) | (uint64_t)o;
-  ix[j] = 2 * ix[c] + (o & 1);
-  iy[j] = 2 * iy[c] + ((o >> 1) & 1);
-  iz[j] = 2 * iz[c] + (o >> 2);
-  pstart[j] = b;
-  pcount[j] = nb - b;
-  parent[j] = c;
-  child_first[j] = -1;
-  child_mask[j] = 0;
-  clevel[j] = (unsigned char)(level + 1);
-  set_radius(j, r, cr, crmax, crf);
-  csys[j] = csys[c];
+// All levels of cells, then the leaves, in one cooperative launch: a grid-wide
+// barrier stands between the steps of a level, so the host waits once for the
+// whole tree instead of once a level.  A block takes a contiguous range of a
+// level's cells, eight lanes a cell:
+// - lane o (1..7) finds where digit o starts in the cell's sorted keys, so the
+//   eight child ranges come from seven searches side by side;
+// - after the barrier, the children's places are the counts of the blocks before,
+//   added up by every block, and a scan within the block, which keeps the cells of
+//   a level in parent order; lane o writes child o.
+// When a level does not fit the arrays the kernel stops there; the host grows them
+// and starts again at that level.  At the end: the leaves in cell order, the near
+// field's units (each leaf's targets in chunks of 32: cell, first target, targets,
+// leaf) and the walk's records of the cells.
+// With the waits, two kernels and a scan a level, from the roots to the leaves: 10^4
+// charges, 4 levels: 155 -> 50 us; 10^6, 5 levels: 245 -> 85 us.
+struct CellArrays {
+  double *cx, *cy, *cz;
+  uint64_t *cid;
+  int *ix, *iy, *iz, *pstart, *pcount, *parent, *child_first;
+  unsigned char *mask, *clevel;
+  double *cr, *crmax;
+  float2 *crf;
+  int *csys, *leaf_cells, *cell_leaf;
+  int4 *walk;  // the walk's record, [2]
+  int4 *units;
+  int *bnd;  // [8] per cell of a level: first particle of each child
+  size_t cap;
+};
+struct CellState {
+  double root[4];                     // system 0's
+  int lo, hi, level;                  // the last level's cells
+  int full;                           // cells that the next level would have needed
+  uint32_t nleaves, nunits, eflags, pad;
+  int off[FMM_MAXLEVEL + 3];          // first cell of each level reached in this launch
+};
+constexpr int CELL_BS = 1024, CELL_GROUPS = CELL_BS / 8;
+
+// sum over the block; over the blocks before this one, and over all
+__device__ __forceinline__ uint64_t block_sum(uint64_t v) {
+  uint64_t tot;
+  block_exclusive<uint64_t>(v, &tot);
+  return tot;
+}
+__device__ __forceinline__ uint64_t blocks_before(const uint64_t *gsum, uint64_t *total) {
+  uint64_t pre = 0, all = 0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+    const uint64_t v = __ldcg(&gsum[i]);
+    all += v;
+    if (i < blockIdx.x) pre += v;
+  }
+  *total = block_sum(all);
+  return block_sum(pre);
 }
 
-__global__ void k_leaf_flags(int ncells, long ncrit, const int *pcount, uint32_t *flag) {
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < ncells) flag[c] = pcount[c] < ncrit ? 1u : 0u;
-}
-// Leaves in cell order, and the near field's units: each leaf's targets in chunks
-// of 32, (cell, first target, targets, leaf), in the order the warps arrive (the
-// units do not depend on one another).
-__global__ void k_leaf_compact(int ncells, long ncrit, const int *pcount, const uint32_t *off, int *leaf_cells,
-                               int *cell_leaf, int4 *units, uint32_t *nunits) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  const int cnt = c < ncells ? pcount[c] : 0;
-  const bool leaf = c < ncells && cnt < ncrit;
-  const int ord = leaf ? (int)off[c] : -1;
-  if (leaf) leaf_cells[ord] = c;
-  if (c < ncells) cell_leaf[c] = ord;
-  const int n = leaf ? (cnt + 31) >> 5 : 0;
-  int incl = n;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
+__global__ void __launch_bounds__(CELL_BS) k_build_cells(CellArrays C, CellState *S, int lo, int hi, int level,
+                                                         int nlev, long ncrit, const uint64_t *keys,
+                                                         const double *roots, double theta, uint64_t *gsum,
+                                                         uint32_t *eflags) {
+  cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+  const int g = threadIdx.x >> 3, o = threadIdx.x & 7;
+  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+  int full = 0;
+  for (;;) {
+    const int n = hi - lo, chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int c0 = lo + (int)min((long)n, (long)blockIdx.x * chunk), c1 = min(hi, c0 + chunk);
+    uint64_t mine = 0;
+    for (int cb = c0; cb < c1; cb += CELL_GROUPS) {
+      const int c = cb + g;
+      int b = 0, e = 0;
+      bool split = false;
+      if (c < c1) {
+        const int cnt = C.pcount[c];
+        b = C.pstart[c];
+        e = b + cnt;
+        split = cnt >= ncrit && level < nlev;
+        if (o == 0 && cnt >= ncrit && level >= nlev)  // no digits below: give up, or ask for all levels
+          atomicOr(eflags, nlev >= FMM_MAXLEVEL ? FMM_EFLAG_DEPTH : FMM_EFLAG_KEYS);
+        if (split && o) b = lower_digit(keys, b, e, level + 1, o);
+        C.bnd[8 * (size_t)(c - lo) + o] = b;
+      }
+      int nb = __shfl_down_sync(0xffffffffu, b, 1, 8);  // child o holds [b, nb)
+      if (o == 7) nb = e;
+      const unsigned m = (__ballot_sync(0xffffffffu, split && nb > b) >> (threadIdx.x & 24)) & 0xffu;
+      if (c < c1 && o == 0) {
+        C.mask[c] = (unsigned char)m;
+        mine += __popc(m);
+      }
+    }
+    mine = block_sum(mine);
+    if (threadIdx.x == 0) gsum[blockIdx.x] = mine;
+    grid.sync();
+    uint64_t total;
+    int run = hi + (int)blocks_before(gsum, &total);
+    if (total == 0) break;
+    if ((size_t)hi + total > C.cap) {
+      full = hi + (int)total;
+      break;
+    }
+    for (int cb = c0; cb < c1; cb += CELL_GROUPS) {
+      const int c = cb + g;
+      const unsigned m = c < c1 ? C.mask[c] : 0u;
+      uint32_t tot;
+      uint32_t at = block_exclusive<uint32_t>(o == 0 ? __popc(m) : 0, &tot);
+      if (o) at -= __popc(m);
+      if (c < c1 && o == 0) C.child_first[c] = m ? run + (int)at : -1;
+      if ((m >> o) & 1u) {
+        const int j = run + (int)at + __popc(m & ((1u << o) - 1u));
+        const double r = __ddiv_rn(C.cr[c], 2.0);  // child half-width = parent r / 2.0 (example/tree.cpp:95)
+        const int b = C.bnd[8 * (size_t)(c - lo) + o];
+        const int nb = o < 7 ? C.bnd[8 * (size_t)(c - lo) + o + 1] : C.pstart[c] + C.pcount[c];
+        // add_child (example/tree.cpp:95-98)
+        C.cx[j] = __dadd_rn(C.cx[c], (o & 1) ? r : -r);
+        C.cy[j] = __dadd_rn(C.cy[c], (o & 2) ? r : -r);
+        C.cz[j] = __dadd_rn(C.cz[c], (o & 4) ? r : -r);
+        C.cid[j] = (C.cid[c] << 3) | (uint64_t)o;
+        C.ix[j] = 2 * C.ix[c] + (o & 1);
+        C.iy[j] = 2 * C.iy[c] + ((o >> 1) & 1);
+        C.iz[j] = 2 * C.iz[c] + (o >> 2);
+        C.pstart[j] = b;
+        C.pcount[j] = nb - b;
+        C.parent[j] = c;
+        C.child_first[j] = -1;
+        C.mask[j] = 0;
+        C.clevel[j] = (unsigned char)(level + 1);
+        set_radius(j, r, C.cr, C.crmax, C.crf);
+        C.csys[j] = C.csys[c];
+      }
+      run += (int)tot;
+    }
+    lo = hi;
+    hi += (int)total;
+    level++;
+    if (first) S->off[level + 1] = hi;
+    grid.sync();
   }
-  uint32_t base = 0;
-  if (lane == 31 && incl > 0) base = atomicAdd(nunits, (uint32_t)incl);
-  base = __shfl_sync(0xffffffffu, base, 31) + (uint32_t)(incl - n);
-  for (int k = 0; k < n; k++) units[base + k] = make_int4(c, 32 * k, min(32, cnt - 32 * k), ord);
+  if (first) {
+    for (int k = 0; k < 4; k++) S->root[k] = roots[k];
+    S->lo = lo;
+    S->hi = hi;
+    S->level = level;
+    S->full = full;
+    S->eflags = __ldcg(eflags);  // every block's cells are counted
+  }
+  if (full) return;
+  // leaves and units: counted together, the units in the high half
+  const int chunk = (hi + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int c0 = (int)min((long)hi, (long)blockIdx.x * chunk), c1 = min(hi, c0 + chunk);
+  uint64_t mine = 0;
+  for (int c = c0 + (int)threadIdx.x; c < c1; c += CELL_BS) {
+    const int cnt = C.pcount[c];
+    if (cnt < ncrit) mine += 1ull | (uint64_t)((cnt + 31) >> 5) << 32;
+  }
+  mine = block_sum(mine);
+  if (threadIdx.x == 0) gsum[gridDim.x + blockIdx.x] = mine;
+  grid.sync();
+  uint64_t total;
+  uint64_t run = blocks_before(gsum + gridDim.x, &total);
+  if (first) {
+    S->nleaves = (uint32_t)total;
+    S->nunits = (uint32_t)(total >> 32);
+  }
+  for (int cb = c0; cb < c1; cb += CELL_BS) {
+    const int c = cb + (int)threadIdx.x, cnt = c < c1 ? C.pcount[c] : 0;
+    const bool leaf = c < c1 && cnt < ncrit;
+    uint64_t tot;
+    const uint64_t at = run + block_exclusive<uint64_t>(leaf ? 1ull | (uint64_t)((cnt + 31) >> 5) << 32 : 0ull, &tot);
+    run += tot;
+    if (c >= c1) continue;
+    const int ord = leaf ? (int)(uint32_t)at : -1;
+    C.cell_leaf[c] = ord;
+    const float margin = cell_margin(roots + 4 * (size_t)C.csys[c], C.cr[c], theta);
+    C.walk[2 * c] = make_int4(C.ix[c], C.iy[c], C.iz[c], C.clevel[c] | (int)C.mask[c] << 8);
+    C.walk[2 * c + 1] = make_int4(C.child_first[c], __float_as_int(margin), 0, 0);
+    if (!leaf) continue;
+    C.leaf_cells[ord] = c;
+    for (int k = 0; 32 * k < cnt; k++) C.units[(at >> 32) + k] = make_int4(c, 32 * k, min(32, cnt - 32 * k), ord);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -345,23 +449,6 @@ __device__ __forceinline__ int walk_decide(const WalkCells &W, int A, int B, con
   if (leafa && leafb) return 1;  // the nleaf >= ncrit leaf-leaf branch is unreachable
   if (leafb || (la <= lb && !leafa)) return 2;  // rmax_A >= rmax_B  <=>  lA <= lB
   return 3;
-}
-
-// The walk's record of each cell.  Its margin, for pairs in which it is the finer cell: FP32 evaluation
-// error plus a bound on how far FP64 centre rounding can move R relative to the
-// cell half-width (from its system's root cube)
-__global__ void k_walk_cells(int nc, const int *csys, const double *roots, const double *cr, double theta,
-                             const int *ix, const int *iy, const int *iz, const unsigned char *clevel,
-                             const unsigned char *mask, const int *child_first, int4 *cell) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const double *rt = roots + 4 * csys[c];
-  const double cmax = fmax(fmax(fabs(rt[0]), fabs(rt[1])), fabs(rt[2])) + rt[3];
-  const double s = cr[c];
-  const double m = 1e-5 + 64.0 * ldexp(1.0, -52) * cmax / s * fmax(1.0, theta);
-  const float margin = s > 0 && m < 0.01 ? (float)m : 1e30f;  // 1e30: always decide in FP64
-  cell[2 * c] = make_int4(ix[c], iy[c], iz[c], clevel[c] | (int)mask[c] << 8);
-  cell[2 * c + 1] = make_int4(child_first[c], __float_as_int(margin), 0, 0);
 }
 
 // One level of the walk per launch: every frontier pair gives an M2L pair, a P2P
@@ -721,13 +808,13 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
     t->ev_ready = true;
   }
   if (!t->h_pinned) {
-    FMM_CUDA_TRY(cudaMallocHost((void **)&t->h_pinned, 256));
-    memset(t->h_pinned, 0, 256);
+    FMM_CUDA_TRY(cudaMallocHost((void **)&t->h_pinned, 4 * FMM_PINNED_WORDS));
+    memset(t->h_pinned, 0, 4 * FMM_PINNED_WORDS);
   }
   t->build_serial++;
   TRY(rec(t, 0, st));
-  TRY(fmm_reserve(t->d_eflags, 4));  // error flags, near-field units
-  FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, 2 * sizeof(uint32_t), st));
+  TRY(fmm_reserve(t->d_eflags, 4));
+  FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, sizeof(uint32_t), st));
   TRY(fmm_reserve(t->sys_off, (size_t)nsys + 1));
   FMM_CUDA_TRY(cudaMemcpyAsync(t->sys_off.p, t->sys_off_h.data(), sizeof(long) * (nsys + 1),
                                cudaMemcpyHostToDevice, st));
@@ -798,7 +885,6 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
     fmm_note_launch(), k_gather_pos<<<fmm_blocks(N, 256), 256, 0, st>>>(pos, t->perm.p, N, t->px.p, t->py.p,
                                                                          t->pz.p);
     FMM_CUDA_TRY(cudaGetLastError());
-    FMM_CUDA_TRY(cudaMemcpyAsync(&t->root, t->roots.p, sizeof(RootBox), cudaMemcpyDeviceToHost, st));  // system 0
     TRY(rec(t, 2, st));
     bool deeper = false;
     TRY(build_cells(t, st, nlev, &deeper));
@@ -850,82 +936,61 @@ static int build_cells(DevTree *t, cudaStream_t st, int nlev, bool *deeper) {
       t->pcount.p, t->parent.p, t->child_first.p, t->child_mask.p, t->clevel.p, t->cr.p, t->crmax.p, t->crf.p,
       t->csys.p);
   FMM_CUDA_TRY(cudaGetLastError());
+  int sms = 0, level = 0, lo = 0, hi = nsys;
+  FMM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t->dev));
+  // 16 cells a block at least: a grid of all SMs has the slower barrier
+  const unsigned nblk = (unsigned)std::min<size_t>(sms, (cap - 1024) / 16 + 1);
+  const size_t head = ((sizeof(CellState) + 255) & ~(size_t)255) + 16 * (size_t)nblk;
+  CellState *H = (CellState *)(t->h_pinned + FMM_PINNED_WALK);
+  static_assert(sizeof(CellState) <= 4 * (FMM_PINNED_WORDS - FMM_PINNED_WALK), "pinned words");
   t->level_off.assign(1, 0);
   t->level_off.push_back(nsys);
-  int lo = 0, hi = nsys, level = 0;
-  uint32_t *h_total = t->h_pinned;
-  int rc = FMM_OK;
-  while (true) {
-    int n = hi - lo;
-    const size_t nscan = (size_t)n + 1 + fmm_scan_tmp_elems<uint32_t>(n) + 16;
-    size_t need = nscan * 4 + (size_t)n * 9 * 4;
-    if ((rc = tmp_reserve(t, need))) break;
-    uint32_t *cnt = (uint32_t *)t->tmp.p;
-    uint32_t *total = cnt + n;
-    uint32_t *stmp = total + 1;
-    int *bnd = (int *)(cnt + nscan);  // child boundaries of each cell of the level
-    fmm_note_launch(), k_count_children<<<fmm_blocks((size_t)n * 32, 128), 128, 0, st>>>(
-        lo, hi, level, nlev, t->ncrit, t->keys.p, t->pstart.p, t->pcount.p, t->child_mask.p, cnt, bnd,
-        t->d_eflags.p);
-    if ((rc = fmm_scan<uint32_t>(cnt, cnt, n, total, stmp, st))) break;
-    cudaMemcpyAsync(h_total, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) { rc = FMM_ERR_CUDA; break; }
-    uint32_t nnew = *h_total;
-    if (nnew == 0) break;
-    size_t need_cells = (size_t)hi + nnew;
-    size_t used = hi;
-    if ((rc = grow_keep(t->cx, need_cells, used, st)) || (rc = grow_keep(t->cy, need_cells, used, st)) ||
-        (rc = grow_keep(t->cz, need_cells, used, st)) || (rc = grow_keep(t->cid, need_cells, used, st)) ||
-        (rc = grow_keep(t->ix, need_cells, used, st)) || (rc = grow_keep(t->iy, need_cells, used, st)) ||
-        (rc = grow_keep(t->iz, need_cells, used, st)) || (rc = grow_keep(t->pstart, need_cells, used, st)) ||
-        (rc = grow_keep(t->pcount, need_cells, used, st)) || (rc = grow_keep(t->parent, need_cells, used, st)) ||
-        (rc = grow_keep(t->child_first, need_cells, used, st)) ||
-        (rc = grow_keep(t->child_mask, need_cells, used, st)) || (rc = grow_keep(t->clevel, need_cells, used, st)) ||
-        (rc = grow_keep(t->cr, need_cells, used, st)) || (rc = grow_keep(t->crmax, need_cells, used, st)) ||
-        (rc = grow_keep(t->crf, need_cells, used, st)) || (rc = grow_keep(t->csys, need_cells, used, st)))
-      break;
-    fmm_note_launch(), k_write_children<<<fmm_blocks((size_t)n * 32, 128), 128, 0, st>>>(
-        lo, hi, level, cnt, bnd, t->cx.p, t->cy.p, t->cz.p, t->cid.p, t->ix.p, t->iy.p, t->iz.p, t->pstart.p,
-        t->pcount.p, t->parent.p, t->child_first.p, t->child_mask.p, t->child_mask.p, t->clevel.p, t->cr.p,
-        t->crmax.p, t->crf.p, t->csys.p);
-    if (cudaGetLastError() != cudaSuccess) { rc = FMM_ERR_CUDA; break; }
-    lo = hi;
-    hi = hi + (int)nnew;
-    level++;
-    t->level_off.push_back(hi);
+  for (;;) {
+    size_t room = std::min({t->cx.cap, t->cy.cap, t->cz.cap, t->cid.cap, t->ix.cap, t->iy.cap, t->iz.cap, t->pstart.cap,
+                            t->pcount.cap, t->parent.cap, t->child_first.cap, t->child_mask.cap, t->clevel.cap,
+                            t->cr.cap, t->crmax.cap, t->crf.cap, t->csys.cap});
+    TRY(fmm_reserve(t->leaf_cells, room)); TRY(fmm_reserve(t->cell_leaf, room)); TRY(fmm_reserve(t->wcell, 2 * room));
+    TRY(fmm_reserve(t->p2p_units, room + (size_t)(N / 32) + 1));
+    TRY(tmp_reserve(t, head + 32 * room));
+    CellState *S = (CellState *)t->tmp.p;
+    uint64_t *gsum = (uint64_t *)(t->tmp.p + head) - 2 * (size_t)nblk;
+    CellArrays C = {t->cx.p, t->cy.p, t->cz.p, t->cid.p, t->ix.p, t->iy.p, t->iz.p, t->pstart.p, t->pcount.p,
+                    t->parent.p, t->child_first.p, t->child_mask.p, t->clevel.p, t->cr.p, t->crmax.p, t->crf.p,
+                    t->csys.p, t->leaf_cells.p, t->cell_leaf.p, t->wcell.p, t->p2p_units.p, (int *)(t->tmp.p + head),
+                    room};
+    const uint64_t *keys = t->keys.p;
+    const double *roots = t->roots.p;
+    uint32_t *eflags = t->d_eflags.p;
+    void *args[] = {&C, &S, &lo, &hi, &level, &nlev, &t->ncrit, &keys, &roots, &t->theta, &gsum, &eflags};
+    fmm_note_launch();
+    FMM_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_build_cells, dim3(nblk), dim3(CELL_BS), args, 0, st));
+    FMM_CUDA_TRY(cudaMemcpyAsync(H, S, sizeof(CellState), cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int l = level + 1; l <= H->level; l++) t->level_off.push_back(H->off[l + 1]);
+    lo = H->lo;
+    hi = H->hi;
+    level = H->level;
+    if (!H->full) break;
+    const size_t need = H->full, used = hi;
+    TRY(grow_keep(t->cx, need, used, st)); TRY(grow_keep(t->cy, need, used, st)); TRY(grow_keep(t->cz, need, used, st));
+    TRY(grow_keep(t->cid, need, used, st)); TRY(grow_keep(t->ix, need, used, st)); TRY(grow_keep(t->iy, need, used, st));
+    TRY(grow_keep(t->iz, need, used, st)); TRY(grow_keep(t->pstart, need, used, st));
+    TRY(grow_keep(t->pcount, need, used, st)); TRY(grow_keep(t->parent, need, used, st));
+    TRY(grow_keep(t->child_first, need, used, st)); TRY(grow_keep(t->child_mask, need, used, st));
+    TRY(grow_keep(t->clevel, need, used, st)); TRY(grow_keep(t->cr, need, used, st));
+    TRY(grow_keep(t->crmax, need, used, st)); TRY(grow_keep(t->crf, need, used, st));
+    TRY(grow_keep(t->csys, need, used, st));
   }
-  if (rc) return rc;
+  memcpy(&t->root, H->root, sizeof(t->root));
   t->ncells = hi;
   t->nlevels = level + 1;
-  // leaves
-  int nc = t->ncells;
-  TRY(fmm_reserve(t->leaf_cells, nc));
-  TRY(fmm_reserve(t->cell_leaf, nc));
-  TRY(tmp_reserve(t, (size_t)nc * 4 + fmm_scan_tmp_elems<uint32_t>(nc) * 4 + 64));
-  uint32_t *flag = (uint32_t *)t->tmp.p;
-  uint32_t *total = flag + nc;
-  uint32_t *stmp = total + 1;
-  fmm_note_launch(), k_leaf_flags<<<fmm_blocks(nc, 256), 256, 0, st>>>(nc, t->ncrit, t->pcount.p, flag);
-  TRY(fmm_scan<uint32_t>(flag, flag, nc, total, stmp, st));
-  TRY(fmm_reserve(t->p2p_units, (size_t)nc + (size_t)(N / 32) + 1));
-  fmm_note_launch(), k_leaf_compact<<<fmm_blocks(nc, 256), 256, 0, st>>>(
-      nc, t->ncrit, t->pcount.p, flag, t->leaf_cells.p, t->cell_leaf.p, t->p2p_units.p, t->d_eflags.p + 1);
-  FMM_CUDA_TRY(cudaGetLastError());
-  FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  FMM_CUDA_TRY(cudaMemcpyAsync(t->h_pinned + 1, t->d_eflags.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  FMM_CUDA_TRY(cudaStreamSynchronize(st));
-  t->nleaves = (int)t->h_pinned[0];
-  t->np2p_units = (int)t->h_pinned[2];
-  if (t->h_pinned[1] & FMM_EFLAG_KEYS) {
+  t->nleaves = (int)H->nleaves;
+  t->np2p_units = (int)H->nunits;
+  t->eflags = H->eflags;
+  if (H->eflags & FMM_EFLAG_KEYS) {
     *deeper = true;
-    FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, 2 * sizeof(uint32_t), st));
-    return FMM_OK;
+    FMM_CUDA_TRY(cudaMemsetAsync(t->d_eflags.p, 0, sizeof(uint32_t), st));
   }
-  TRY(fmm_reserve(t->wcell, 2 * (size_t)nc));
-  fmm_note_launch(), k_walk_cells<<<fmm_blocks(nc, 256), 256, 0, st>>>(
-      nc, t->csys.p, t->roots.p, t->cr.p, t->theta, t->ix.p, t->iy.p, t->iz.p, t->clevel.p, t->child_mask.p,
-      t->child_first.p, t->wcell.p);
-  FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
 }
 
