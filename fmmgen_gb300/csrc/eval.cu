@@ -650,6 +650,7 @@ static int run_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L, 
   TRY(rec(t, 2, st));
   // with an order model, P2P runs first: the predicted orders read its near field
   t->p2p_first = t->ord_mode == 2;
+  t->p2p_last = false;
   if (t->p2p_first) {
     TRY(fmm_p2p_launch(t, mixed, S, st));
     TRY(rec(t, 3, st));
@@ -913,12 +914,17 @@ static int evaluate_pass(DevTree *t, const double *S, double *F, int potential, 
 // ---------------------------------------------------------------------------
 // The multipoles need nothing of the interaction lists, so as soon as the
 // cells exist a second stream stages the particles and runs P2M and M2M
-// (near_start, beside the walk and the class build).  The M2L follows the classes on the
-// highest-priority stream -- its persistent CTAs take the SMs first -- and the
-// P2P starts beside it on the caller's stream (in the blocks the tuning
-// chose), as in the overlapped pass; L2L, L2P and the final sum follow.  Phase
-// records follow the streams: "M2L" spans the end of M2M to the end of M2L
-// (the class build included), "P2P" the near field's tail after it.
+// (near_start, beside the walk and the class build).  The P2P needs the lists
+// alone: it starts with them on the caller's stream, and the classes, the M2L,
+// L2L and L2P run on the highest-priority stream beside it, their kernels taking
+// SMs as P2P blocks end; the final sum waits for both.  (With the P2P behind the
+// class build, some 30 launches that leave the GPU idle, and the L2L behind the
+// P2P: 10^4 charges, p = 4, 711 us a step, now 646; 10^6, p = 8, 7.57 and
+// 7.27 ms; 10^5 clustered charges in FP64 11.7 and 9.8 ms.)  Two cases keep the P2P later: an order model reads the
+// near field, so its M2L waits for the P2P, and beside the tensor-core M2L, whose
+// CTAs leave room for one P2P block per SM, it starts with the M2L or after it.
+// Phase records follow the streams: "M2L" spans the end of M2M to the end of M2L
+// (the class build included), "P2P" the near field's tail after the last of them.
 // Stage the particles and run P2M and M2M on the near-field stream as soon as
 // the cells exist: the walk that builds the interaction lists runs beside them.
 struct NearStart {
@@ -980,6 +986,13 @@ static int fused_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L
   const int p = t->order, so = t->so, nl = t->nleaves;
   const double *cr = t->cr.p;
   FMM_CUDA_TRY(cudaEventRecord(t->ev_l, st));  // the interaction lists are built
+  const bool learned = t->ord_mode == 2;
+  // (a tree too deep has no leaf for some of its particles: its error comes with the classes)
+  const bool early = !learned && !(mixed && is_tc(t->tune.impl)) && !(t->eflags & FMM_EFLAG_DEPTH);
+  if (early) {
+    FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_s, 0));  // the staged particles
+    TRY(fmm_p2p_launch(t, mixed, S, st));
+  }
   // the classes (the host waits on this stream only), then the M2L
   FMM_CUDA_TRY(cudaStreamWaitEvent(t->s_hi, t->ev_l, 0));
   TRY(fmm_tree_finish_build(t, t->s_hi));
@@ -987,42 +1000,43 @@ static int fused_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L
   t->p2p_first = false;
   FMM_CUDA_TRY(cudaEventRecord(t->ev_c, t->s_hi));
   FMM_CUDA_TRY(cudaStreamWaitEvent(t->s_hi, t->ev_m, 0));
-  const bool learned = t->ord_mode == 2;
   if (learned) {  // the orders read the near field: P2P first
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_c, 0));
-    FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_s, 0));  // the staged particles
+    FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_s, 0));
     TRY(fmm_p2p_launch(t, mixed, S, st));
     FMM_CUDA_TRY(cudaEventRecord(t->ev_p, st));
     FMM_CUDA_TRY(cudaStreamWaitEvent(t->s_hi, t->ev_p, 0));
   }
   TRY(m2l_phase<T>(t, ps, M, L, mixed, impl, mstr, lstr, dstr, t->s_hi));
   TRY(rec(t, 3, t->s_hi));
-  FMM_CUDA_TRY(cudaEventRecord(t->ev_join, t->s_hi));
-  if (!learned) {  // launched after the M2L, beside it; behind the tensor-core M2L without the overlap
-                   // switch (its CTA leaves room for one P2P block per SM: side by side gains nothing there)
+  if (!learned && !early) {  // launched after the M2L, beside it; behind it without the overlap switch
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_c, 0));
     FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_s, 0));
-    if (!t->tune.overlap && mixed && is_tc(impl)) FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
+    if (!t->tune.overlap && is_tc(impl)) {
+      FMM_CUDA_TRY(cudaEventRecord(t->ev_p, t->s_hi));
+      FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_p, 0));
+    }
     TRY(fmm_p2p_launch(t, mixed, S, st));
   }
-  FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
-  TRY(rec(t, 4, st));
   for (int l = 1; l < t->nlevels; l++) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
     if (mixed)
-      TRY(fmm_l2l_tab(t, lo, hi, (float *)(void *)L, lstr, st));
+      TRY(fmm_l2l_tab(t, lo, hi, (float *)(void *)L, lstr, t->s_hi));
     else
-      fmm_note_launch(), k_l2l<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, st>>>(
+      fmm_note_launch(), k_l2l<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, t->s_hi>>>(
           ps->l2l, lo, hi, so, p, t->parent.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr, L, lstr);
   }
   FMM_CUDA_TRY(cudaGetLastError());
-  TRY(rec(t, 5, st));
-  fmm_note_launch(), k_l2p<T><<<fmm_blocks(nl, L2P_WARPS), 32 * L2P_WARPS, 0, st>>>(
+  TRY(rec(t, 4, t->s_hi));
+  fmm_note_launch(), k_l2p<T><<<fmm_blocks(nl, L2P_WARPS), 32 * L2P_WARPS, 0, t->s_hi>>>(
       t->leaf_cells.p, nl, t->pstart.p, t->pcount.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, t->px.p, t->py.p,
       t->pz.p, so, p, cr, L, t->Ffar.p, lstr);
   FMM_CUDA_TRY(cudaGetLastError());
-  TRY(rec(t, 6, st));
-  return FMM_OK;
+  TRY(rec(t, 5, t->s_hi));
+  FMM_CUDA_TRY(cudaEventRecord(t->ev_join, t->s_hi));
+  FMM_CUDA_TRY(cudaStreamWaitEvent(st, t->ev_join, 0));
+  t->p2p_last = true;
+  return rec(t, 6, st);
 }
 
 int fmm_tree_build_evaluate(DevTree *t, const double *pos, long N, long ncrit, int order, double theta, int so,
@@ -1145,6 +1159,7 @@ void fmm_eval_times(DevTree *t) {
     t->phase_ms[i] = ms;
   }
   if (t->p2p_first) std::swap(t->phase_ms[2], t->phase_ms[3]);  // the pass ran P2P, then M2L
+  if (t->p2p_last) std::rotate(t->phase_ms + 3, t->phase_ms + 5, t->phase_ms + 6);  // L2L, L2P, the P2P's tail
   for (int k = 0; k < 2; k++) {
     if (cudaEventElapsedTime(&ms, t->ev_mk[2 * k], t->ev_mk[2 * k + 1]) != cudaSuccess) {
       ms = -1.f;
