@@ -86,7 +86,7 @@ extern "C" int fmmgen_root_box_noalloc(const double *pos, long N, double *root4,
   if (rc) return rc;
   unsigned nbm = std::min<unsigned>(fmm_blocks(N, 256), 152 * 8);
   fmm_note_launch(), k_root_absmax<<<nbm, 256, 0, st>>>(pos, N, sums, mx);
-  fmm_note_launch(), k_root_final<<<1, 1, 0, st>>>(sums, mx, N, root4, lev, levf);
+  fmm_note_launch(), k_root_final<<<1, 32, 0, st>>>(sums, mx, N, root4, lev, levf);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
 }

@@ -58,24 +58,26 @@ __global__ void k_root_absmax(const double *__restrict__ pos, long N, const doub
   }
 }
 
-// root[0..3] = centre, r; lev[2l] = r_l, lev[2l+1] = rmax_l = sqrt(3*r_l*r_l)
+// root[0..3] = centre, r; lev[2l] = r_l, lev[2l+1] = rmax_l = sqrt(3*r_l*r_l).  A lane
+// per level, which halves r for itself (the halvings are exact, so as r / 2.0 one
+// after the other); on one thread the chain of divisions and roots took 14 us.
 __global__ void k_root_final(const double *sums, const unsigned long long *mx, long N, double *root,
                              double *lev, float2 *levf) {
-  double n = (double)N;
-  double ax = __ddiv_rn(sums[0], n), ay = __ddiv_rn(sums[1], n), az = __ddiv_rn(sums[2], n);
-  double xm = __longlong_as_double((long long)mx[0]);
-  double ym = __longlong_as_double((long long)mx[1]);
-  double zm = __longlong_as_double((long long)mx[2]);
-  double r = __dmul_rn((xm > ym ? (xm > zm ? xm : zm) : (ym > zm ? ym : zm)), 1.001);
-  root[0] = ax; root[1] = ay; root[2] = az; root[3] = r;
+  const int l = threadIdx.x;
+  const double n = (double)N;
+  const double xm = __longlong_as_double((long long)mx[0]);
+  const double ym = __longlong_as_double((long long)mx[1]);
+  const double zm = __longlong_as_double((long long)mx[2]);
+  const double r = __dmul_rn((xm > ym ? (xm > zm ? xm : zm) : (ym > zm ? ym : zm)), 1.001);
+  if (l < 3) root[l] = __ddiv_rn(sums[l], n);
+  if (l == 3) root[3] = r;
+  if (l > FMM_MAXLEVEL) return;
   double rl = r;
-  for (int l = 0; l <= FMM_MAXLEVEL; l++) {
-    lev[2 * l] = rl;
-    lev[2 * l + 1] = __dsqrt_rn(__dmul_rn(__dmul_rn(3.0, rl), rl));  // example/tree.cpp:15
-    float hi = (float)rl;
-    levf[l] = make_float2(hi, (float)(rl - (double)hi));
-    rl = __ddiv_rn(rl, 2.0);
-  }
+  for (int k = 0; k < l; k++) rl = __dmul_rn(rl, 0.5);
+  lev[2 * l] = rl;
+  lev[2 * l + 1] = __dsqrt_rn(__dmul_rn(__dmul_rn(3.0, rl), rl));  // example/tree.cpp:15
+  const float hi = (float)rl;
+  levf[l] = make_float2(hi, (float)(rl - (double)hi));
 }
 
 // ---------------------------------------------------------------------------
@@ -104,6 +106,57 @@ __global__ void k_keys(const double *__restrict__ pos, long N, const double *roo
   }
   keys[i] = key << (3 * (FMM_MAXLEVEL - nlev));
   idx[i] = (uint32_t)i;
+}
+
+// rank[i] += the keys below keys[i] among the block's share (blockIdx.y) of them
+constexpr int RANK_BS = 256;
+__global__ void __launch_bounds__(RANK_BS) k_rank(const uint64_t *keys, int n, int share, uint32_t *rank) {
+  __shared__ ulonglong2 sk[RANK_BS / 2];
+  const int i = blockIdx.x * RANK_BS + threadIdx.x;
+  const uint64_t k = i < n ? keys[i] : 0;
+  const int j1 = min(n, ((int)blockIdx.y + 1) * share);
+  uint32_t below = 0;
+  for (int j0 = blockIdx.y * share; j0 < j1; j0 += RANK_BS) {
+    __syncthreads();
+    ((uint64_t *)sk)[threadIdx.x] = j0 + (int)threadIdx.x < j1 ? keys[j0 + threadIdx.x] : ~0ull;
+    __syncthreads();
+#pragma unroll 8
+    for (int j = 0; j < RANK_BS / 2; j++) below += (sk[j].x < k) + (sk[j].y < k);
+  }
+  if (i < n && below) atomicAdd(&rank[i], below);
+}
+// (rank starts at zero; blocks to fill the SMs, eight each)
+static int rank_keys(const uint64_t *keys, int n, uint32_t *rank, cudaStream_t st) {
+  const unsigned nb = fmm_blocks(std::max(n, 1), RANK_BS), shares = std::max(1u, std::min(nb, 1216u / nb));
+  const int share = (int)((nb + shares - 1) / shares) * RANK_BS;
+  fmm_note_launch(), k_rank<<<dim3(nb, (nb * RANK_BS + share - 1) / share), RANK_BS, 0, st>>>(keys, n, share, rank);
+  FMM_CUDA_TRY(cudaGetLastError());
+  return FMM_OK;
+}
+
+// The particles of a small system in key order.  Up to KEY_RANK_MAX of them are
+// ranked by counting, their index in the key's free low bits breaking the ties: one
+// launch of n^2 comparisons where the radix sort's twelve launches, with few blocks,
+// wait for one another (10^4 particles: 100 -> 24 us; at the limit the comparisons take
+// some 30 us).
+constexpr long KEY_RANK_MAX = 16384;
+static_assert(3 * (FMM_MAXLEVEL - FMM_KEYLEVELS) >= 14, "free bits for the index");
+__global__ void k_key_index(long N, uint64_t *keys, uint32_t *rank) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  keys[i] |= (uint64_t)i;
+  rank[i] = 0;
+}
+__global__ void k_place(const double *__restrict__ pos, const uint64_t *keys, const uint32_t *rank, long N,
+                        uint64_t *kout, uint32_t *perm, double *px, double *py, double *pz) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const uint32_t r = rank[i];
+  kout[r] = keys[i] & ~(uint64_t)(KEY_RANK_MAX - 1);
+  perm[r] = (uint32_t)i;
+  px[r] = pos[3 * i];
+  py[r] = pos[3 * i + 1];
+  pz[r] = pos[3 * i + 2];
 }
 
 __global__ void k_gather_pos(const double *__restrict__ pos, const uint32_t *perm, long N, double *px,
@@ -674,24 +727,7 @@ __global__ void k_class_collect(const uint64_t *tab, uint32_t nslots, uint64_t *
   rank[r] = 0;
 }
 
-// rank[i] += the keys below uniq[i] among the block's share (blockIdx.y) of them
-constexpr int RANK_BS = 256;
 constexpr uint32_t RANK_MAX = 32768;
-__global__ void __launch_bounds__(RANK_BS) k_class_count(const uint64_t *uniq, int nu, int share, uint32_t *rank) {
-  __shared__ ulonglong2 sk[RANK_BS / 2];
-  const int i = blockIdx.x * RANK_BS + threadIdx.x;
-  const uint64_t k = i < nu ? uniq[i] : 0;
-  const int j1 = min(nu, ((int)blockIdx.y + 1) * share);
-  uint32_t below = 0;
-  for (int j0 = blockIdx.y * share; j0 < j1; j0 += RANK_BS) {
-    __syncthreads();
-    ((uint64_t *)sk)[threadIdx.x] = j0 + (int)threadIdx.x < j1 ? uniq[j0 + threadIdx.x] : CLS_EMPTY;
-    __syncthreads();
-#pragma unroll 8
-    for (int j = 0; j < RANK_BS / 2; j++) below += (sk[j].x < k) + (sk[j].y < k);
-  }
-  if (i < nu && below) atomicAdd(&rank[i], below);
-}
 
 // ids by rank (none: the keys are sorted); the class table entry of each key; *same cleared unless the sorted
 // keys are the previous build's, which they replace
@@ -830,7 +866,7 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
     unsigned nbm = std::min<unsigned>(fmm_blocks(N, 256), 152 * 8);
     fmm_note_launch(), k_root_absmax<<<nbm, 256, 0, st>>>(pos, N, dr, (unsigned long long *)(dr + 3));
     TRY(fmm_reserve(t->levf, FMM_MAXLEVEL + 1));
-    fmm_note_launch(), k_root_final<<<1, 1, 0, st>>>(dr, (const unsigned long long *)(dr + 3), N, t->roots.p,
+    fmm_note_launch(), k_root_final<<<1, 32, 0, st>>>(dr, (const unsigned long long *)(dr + 3), N, t->roots.p,
                                                      dr + 16, t->levf.p);
   } else {
     // a forest: each system's exact sequential means, side by side
@@ -861,30 +897,39 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
     fmm_note_launch(), k_keys<<<fmm_blocks(N, 256), 256, 0, st>>>(pos, N, t->roots.p, nsys > 1 ? t->psys.p : nullptr,
                                                                    nlev, t->keys.p, t->perm.p);
     FMM_CUDA_TRY(cudaGetLastError());
-    size_t nbh = fmm_rs_nblocks(N);
-    size_t hist_n = 256 * nbh;
-    const size_t sort_bytes = hist_n * 4 + fmm_scan_tmp_elems<uint32_t>(hist_n) * 4 + 1024;
-    TRY(tmp_reserve(t, sort_bytes + (nsys > 1 ? 16 * (size_t)N : 0)));
-    uint32_t *hist = (uint32_t *)t->tmp.p;
-    uint32_t *scantmp = hist + hist_n;
-    TRY(fmm_radix_sort(t->keys.p, t->perm.p, t->keys2.p, t->perm2.p, N, 3 * (FMM_MAXLEVEL - nlev),
-                       3 * FMM_MAXLEVEL, hist, scantmp, st));
-    if (nsys > 1) {
-      // stable sort by system: (system, key) order, each system's particles contiguous
-      uint32_t *ks = (uint32_t *)(t->tmp.p + sort_bytes);
-      uint32_t *idx = ks + N, *ks2 = idx + N, *idx2 = ks2 + N;
-      fmm_note_launch(), k_sorted_sys<<<fmm_blocks(N, 256), 256, 0, st>>>(t->perm.p, t->psys.p, N, ks, idx);
-      TRY(fmm_radix_sort<uint32_t>(ks, idx, ks2, idx2, N, 0, bits_for(nsys), hist, scantmp, st));
-      fmm_note_launch(), k_apply_order<<<fmm_blocks(N, 256), 256, 0, st>>>(idx, N, t->keys.p, t->perm.p,
-                                                                           t->keys2.p, t->perm2.p);
+    TRY(fmm_reserve(t->px, N)); TRY(fmm_reserve(t->py, N)); TRY(fmm_reserve(t->pz, N));
+    if (nsys == 1 && N <= KEY_RANK_MAX && nlev == FMM_KEYLEVELS) {
+      fmm_note_launch(), k_key_index<<<fmm_blocks(N, 256), 256, 0, st>>>(N, t->keys.p, t->perm2.p);
+      TRY(rank_keys(t->keys.p, (int)N, t->perm2.p, st));
+      fmm_note_launch(), k_place<<<fmm_blocks(N, 256), 256, 0, st>>>(pos, t->keys.p, t->perm2.p, N, t->keys2.p,
+                                                                     t->perm.p, t->px.p, t->py.p, t->pz.p);
       FMM_CUDA_TRY(cudaGetLastError());
       std::swap(t->keys, t->keys2);
-      std::swap(t->perm, t->perm2);
+    } else {
+      size_t nbh = fmm_rs_nblocks(N);
+      size_t hist_n = 256 * nbh;
+      const size_t sort_bytes = hist_n * 4 + fmm_scan_tmp_elems<uint32_t>(hist_n) * 4 + 1024;
+      TRY(tmp_reserve(t, sort_bytes + (nsys > 1 ? 16 * (size_t)N : 0)));
+      uint32_t *hist = (uint32_t *)t->tmp.p;
+      uint32_t *scantmp = hist + hist_n;
+      TRY(fmm_radix_sort(t->keys.p, t->perm.p, t->keys2.p, t->perm2.p, N, 3 * (FMM_MAXLEVEL - nlev),
+                         3 * FMM_MAXLEVEL, hist, scantmp, st));
+      if (nsys > 1) {
+        // stable sort by system: (system, key) order, each system's particles contiguous
+        uint32_t *ks = (uint32_t *)(t->tmp.p + sort_bytes);
+        uint32_t *idx = ks + N, *ks2 = idx + N, *idx2 = ks2 + N;
+        fmm_note_launch(), k_sorted_sys<<<fmm_blocks(N, 256), 256, 0, st>>>(t->perm.p, t->psys.p, N, ks, idx);
+        TRY(fmm_radix_sort<uint32_t>(ks, idx, ks2, idx2, N, 0, bits_for(nsys), hist, scantmp, st));
+        fmm_note_launch(), k_apply_order<<<fmm_blocks(N, 256), 256, 0, st>>>(idx, N, t->keys.p, t->perm.p,
+                                                                             t->keys2.p, t->perm2.p);
+        FMM_CUDA_TRY(cudaGetLastError());
+        std::swap(t->keys, t->keys2);
+        std::swap(t->perm, t->perm2);
+      }
+      fmm_note_launch(), k_gather_pos<<<fmm_blocks(N, 256), 256, 0, st>>>(pos, t->perm.p, N, t->px.p, t->py.p,
+                                                                           t->pz.p);
+      FMM_CUDA_TRY(cudaGetLastError());
     }
-    TRY(fmm_reserve(t->px, N)); TRY(fmm_reserve(t->py, N)); TRY(fmm_reserve(t->pz, N));
-    fmm_note_launch(), k_gather_pos<<<fmm_blocks(N, 256), 256, 0, st>>>(pos, t->perm.p, N, t->px.p, t->py.p,
-                                                                         t->pz.p);
-    FMM_CUDA_TRY(cudaGetLastError());
     TRY(rec(t, 2, st));
     bool deeper = false;
     TRY(build_cells(t, st, nlev, &deeper));
@@ -1330,9 +1375,7 @@ static int build_classes(DevTree *t, cudaStream_t st) {
                                                                               stat + 2);
   const bool counted = ncls <= RANK_MAX;
   if (counted) {
-    const unsigned nb = fmm_blocks(std::max(ncls, 1u), RANK_BS), shares = std::max(1u, std::min(nb, 1216u / nb));
-    const int share = (int)((nb + shares - 1) / shares) * RANK_BS;
-    fmm_note_launch(), k_class_count<<<dim3(nb, (nb * RANK_BS + share - 1) / share), RANK_BS, 0, st>>>(U1, (int)ncls, share, I2);
+    TRY(rank_keys(U1, (int)ncls, I2, st));
   } else {
     TRY(fmm_radix_sort<uint64_t>(U1, I1, U2, I2, ncls, 0, 64, uhist, uscan, st));
   }

@@ -184,3 +184,17 @@ def test_p2p_lists_sorted(fg, oracle_lib, n, ncrit, lo, hi):
     assert np.array_equal(p2p.reshape(t.nleaves, t.nleaves, 2)[:, :, 0], np.repeat(leaves[:, None], t.nleaves, 1))
     assert np.array_equal(p2p.reshape(t.nleaves, t.nleaves, 2)[:, :, 1], np.repeat(leaves[None], t.nleaves, 0))
     assert t.p2p_interactions == n * (n - 1)
+
+
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 5000, 16383, 16384, 16385])
+def test_key_order(fg, oracle_lib, n):
+    """The particles in key order, ranked by counting up to 16,384 and radix-sorted above: the oracle's leaves, and
+    particles at the same place in the order of their indices (the sort is stable)."""
+    rng = np.random.default_rng(n)
+    pos = rng.uniform(-1, 1, (n, 3))
+    pos[n // 2:2 * (n // 2)] = pos[:n // 2]
+    t, _ = oracle_check(fg, oracle_lib, pos, rng.uniform(-1, 1, (n, 1)), 20, 4, 0.5)
+    c = t.cells()
+    at = np.empty(n, int)
+    at[c["leaf_idx"]] = np.arange(n)
+    assert np.all(at[:n // 2] < at[n // 2:2 * (n // 2)])
