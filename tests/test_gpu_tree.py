@@ -198,3 +198,18 @@ def test_key_order(fg, oracle_lib, n):
     at = np.empty(n, int)
     at[c["leaf_idx"]] = np.arange(n)
     assert np.all(at[:n // 2] < at[n // 2:2 * (n // 2)])
+
+
+@pytest.mark.parametrize("shift", [0.0, 3.0, 1e5, 1e9])
+def test_keys_at_boundaries(fg, oracle_lib, shift):
+    """Particles on the cells' boundaries, some units in the last place and some 1e-4 of a cell beside them, in a root
+    cube around the origin (pairs p, -p keep the mean exact) and far from it: the oracle's leaves."""
+    rng = np.random.default_rng(7)
+    n = 1500
+    r = 1.001  # half-width of the root cube: the farthest coordinate is 1
+    b = r * rng.integers(-31, 32, (n, 3)) / 32
+    off = rng.choice([0.0, 1e-16, -1e-16, 3e-16, 1e-4 / 512, -1e-4 / 512, 6e-4 / 512, 0.01], (n, 3))
+    p = np.clip(np.where(rng.uniform(size=(n, 3)) < 0.7, b + off, rng.uniform(-1, 1, (n, 3))), -1, 1)
+    p[0] = 1.0
+    pos = np.stack([p, -p], 1).reshape(-1, 3) + shift
+    oracle_check(fg, oracle_lib, pos, rng.uniform(-1, 1, (2 * n, 1)), 8, 4, 0.5)
