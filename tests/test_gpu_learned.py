@@ -358,3 +358,37 @@ def test_trained_model_gain(fg):
     assert eL <= 1e-6
     assert wL < w12 / 3
     assert wL < wq
+
+
+@pytest.mark.parametrize("so,order", [(0, 4), (0, 12), (1, 7), (2, 12)])
+def test_mnorms_by_degree(fg, so, order):
+    """The features of a pair rest on each degree's 2-norm of the source's multipole, added up in FP64 over the lanes:
+    the features against those of the exported multipoles, degree by degree."""
+    from fmmgen_gb300 import learned
+
+    rng = np.random.default_rng(order)
+    n = 3000
+    t = fg.build_tree(cuda(rng.uniform(-1, 1, (n, 3))), cuda(rng.uniform(-1, 1, (n, [1, 3, 6][so]))), n, 40, order, 0.5,
+                      source_order=so)
+    t.compute_field_fmm(precision="fp64")
+    f = learned.order_features(t, 0.1).cpu().numpy()
+    M, _ = t.expansions()
+    c = t.cells()
+    row = {int(i): k for k, i in enumerate(c["id"])}
+    m2l, _ = t.lists()
+    deg = np.concatenate([np.full((d + 1) * (d + 2) // 2, d) for d in range(so, order + 1)])
+    src = np.array([row[int(b)] for b in m2l[:, 0]])
+    seen = 0
+    for k in rng.choice(len(src), 400, replace=False):
+        b = src[k]
+        norm = np.array([np.sqrt(np.sum(M[b][deg == d] ** 2)) for d in range(so, order + 1)])
+        part = f[k, 3 + max(so, 1) - 1:3 + order]
+        if so == 0:
+            norm = norm[1:]
+        lg = np.log10(np.maximum(norm, 1e-300))
+        if not (np.all(part > -29) and np.all(np.isfinite(lg))):
+            continue
+        seen += 1
+        # part_d = const + log10|M_d| - d log10(scale): the second difference in d removes both unknowns
+        assert np.allclose(np.diff(part, 2), np.diff(lg, 2), rtol=0, atol=2e-5)
+    assert seen > 100
