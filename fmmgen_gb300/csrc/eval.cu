@@ -188,38 +188,6 @@ __device__ __forceinline__ void warp_monomials(double vx, double vy, double vz, 
 }
 
 // ---------------------------------------------------------------------------
-// M2M for all parents of one level (example/calculate.cpp:163-187)
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(32 * FMM_WARPS) k_m2m(Plan P, int lo, int hi, int so, int order,
-                                                        const unsigned char *child_mask, const int *child_first,
-                                                        const unsigned char *clevel, const double *cx,
-                                                        const double *cy, const double *cz, const double *cr,
-                                                        T *M, int mstr) {
-  __shared__ T sA[FMM_WARPS][FMM_NTMAX], sB[FMM_WARPS][FMM_NTMAX], sS[FMM_WARPS][FMM_NTMAX + 32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = lo + blockIdx.x * FMM_WARPS + w;
-  if (c >= hi) return;
-  unsigned mask = child_mask[c];
-  if (!mask) return;
-  const int off = fmm_nterms(so - 1), msize = fmm_nterms(order) - off;
-  const double inv_s = 1.0 / cr[c];
-  for (int k = lane; k < P.nseg; k += 32) sS[w][k] = T(0);
-  int ch = child_first[c];
-  int nch = __popc(mask);
-  for (int q = 0; q < nch; q++, ch++) {
-    __syncwarp();
-    warp_monomials<T>((cx[c] - cx[ch]) * inv_s, (cy[c] - cy[ch]) * inv_s, (cz[c] - cz[ch]) * inv_s, order - so,
-                      sA[w], lane);
-    for (int j = lane; j < msize; j += 32) sB[w][j] = M[(size_t)ch * mstr + j] * exp2i<T>(-(int)c_mi[j + off][3]);
-    __syncwarp();
-    engine_run<T>(P, sA[w], sB[w], sS[w], lane);
-  }
-  __syncwarp();
-  for (int n = lane; n < msize; n += 32) M[(size_t)c * mstr + n] = engine_out<T>(P, sS[w], n);
-}
-
-// ---------------------------------------------------------------------------
 // M2L, one warp per target cell (example/calculate.cpp:190-206)
 // ---------------------------------------------------------------------------
 template <typename T>
@@ -491,32 +459,6 @@ __global__ void __launch_bounds__(32 * PackF<NP>::WARPS) k_m2l_pk(Plan P, int q,
 #define M2L_PACK 2
 
 // ---------------------------------------------------------------------------
-// L2L for all cells of one level (example/calculate.cpp:219-234)
-// ---------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(32 * FMM_WARPS) k_l2l(Plan P, int lo, int hi, int so, int order,
-                                                        const int *parent, const unsigned char *clevel,
-                                                        const double *cx, const double *cy, const double *cz,
-                                                        const double *cr, T *L, int lstr) {
-  __shared__ T sA[FMM_WARPS][FMM_NTMAX], sB[FMM_WARPS][FMM_NTMAX], sS[FMM_WARPS][FMM_NTMAX + 32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c = lo + blockIdx.x * FMM_WARPS + w;
-  if (c >= hi) return;
-  const int p = parent[c];
-  const int lsize = fmm_nterms(order - so);
-  const double inv_s = 1.0 / cr[p];
-  for (int k = lane; k < P.nseg; k += 32) sS[w][k] = T(0);
-  warp_monomials<T>((cx[c] - cx[p]) * inv_s, (cy[c] - cy[p]) * inv_s, (cz[c] - cz[p]) * inv_s, order - so, sA[w],
-                    lane);
-  for (int j = lane; j < lsize; j += 32) sB[w][j] = L[(size_t)p * lstr + j];
-  __syncwarp();
-  engine_run<T>(P, sA[w], sB[w], sS[w], lane);
-  __syncwarp();
-  for (int n = lane; n < lsize; n += 32)
-    L[(size_t)c * lstr + n] += engine_out<T>(P, sS[w], n) * exp2i<T>(-((int)c_mi[n][3] + 1));
-}
-
-// ---------------------------------------------------------------------------
 // L2P, one warp per leaf, one lane per particle (example/calculate.cpp:236-250)
 // ---------------------------------------------------------------------------
 #define L2P_WARPS 2
@@ -628,23 +570,17 @@ static int run_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L, 
                     int lstr, int dstr, cudaStream_t st) {
   const int p = t->order, so = t->so;
   const double *cr = t->cr.p;  // per-cell half-widths
-  const int nl = t->nleaves, nc = t->ncells;
+  const int nl = t->nleaves;
   // P2M
   fmm_note_launch(), k_p2m<T><<<fmm_blocks(nl, FMM_WARPS), 32 * FMM_WARPS, 0, st>>>(
       t->leaf_cells.p, nl, t->pstart.p, t->pcount.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, t->px.p, t->py.p,
       t->pz.p, t->perm.p, S, so, p, cr, M, mstr);
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(rec(t, 1, st));
-  // M2M, deepest parents first (mixed pass: the eight fixed child-shift
-  // operators, shift.cu; FP64: the contraction engine)
+  // M2M, deepest parents first
   for (int l = t->nlevels - 2; l >= 0; l--) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
-    if (mixed)
-      TRY(fmm_m2m_tab(t, lo, hi, (float *)(void *)M, mstr, st));
-    else
-      fmm_note_launch(), k_m2m<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, st>>>(
-          ps->m2m, lo, hi, so, p, t->child_mask.p, t->child_first.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr, M,
-          mstr);
+    TRY(fmm_m2m<T>(t, lo, hi, M, mstr, st));
   }
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(rec(t, 2, st));
@@ -661,14 +597,10 @@ static int run_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L, 
   } else {
     TRY(m2l_p2p<T>(t, ps, S, M, L, mixed, impl, mstr, lstr, dstr, st));
   }
-  // L2L, top-down (as M2M: fixed child-shift operators in the mixed pass)
+  // L2L, top-down
   for (int l = 1; l < t->nlevels; l++) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
-    if (mixed)
-      TRY(fmm_l2l_tab(t, lo, hi, (float *)(void *)L, lstr, st));
-    else
-      fmm_note_launch(), k_l2l<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, st>>>(
-          ps->l2l, lo, hi, so, p, t->parent.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr, L, lstr);
+    TRY(fmm_l2l<T>(t, lo, hi, L, lstr, st));
   }
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(rec(t, 5, st));
@@ -967,12 +899,7 @@ static int near_start(DevTree *t, void *arg) {
   TRY(rec(t, 1, sn));
   for (int l = t->nlevels - 2; l >= 0; l--) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
-    if (a.mixed)
-      TRY(fmm_m2m_tab(t, lo, hi, (float *)(void *)M, mstr, sn));
-    else
-      fmm_note_launch(), k_m2m<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, sn>>>(
-          a.ps->m2m, lo, hi, so, p, t->child_mask.p, t->child_first.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr,
-          M, mstr);
+    TRY(fmm_m2m<T>(t, lo, hi, M, mstr, sn));
   }
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(rec(t, 2, sn));
@@ -1020,11 +947,7 @@ static int fused_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L
   }
   for (int l = 1; l < t->nlevels; l++) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
-    if (mixed)
-      TRY(fmm_l2l_tab(t, lo, hi, (float *)(void *)L, lstr, t->s_hi));
-    else
-      fmm_note_launch(), k_l2l<T><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, t->s_hi>>>(
-          ps->l2l, lo, hi, so, p, t->parent.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr, L, lstr);
+    TRY(fmm_l2l<T>(t, lo, hi, L, lstr, t->s_hi));
   }
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(rec(t, 4, t->s_hi));
@@ -1130,9 +1053,7 @@ int fmm_tree_evaluate_bh(DevTree *t, const double *S, double *F, int potential, 
       t->py.p, t->pz.p, t->perm.p, S, so, p, cr, t->M.p, msize);
   for (int l = t->nlevels - 2; l >= 0; l--) {
     int lo = t->level_off[l], hi = t->level_off[l + 1];
-    fmm_note_launch(), k_m2m<double><<<fmm_blocks(hi - lo, FMM_WARPS), 32 * FMM_WARPS, 0, st>>>(
-        ps->m2m, lo, hi, so, p, t->child_mask.p, t->child_first.p, t->clevel.p, t->cx.p, t->cy.p, t->cz.p, cr,
-        t->M.p, msize);
+    TRY(fmm_m2m<double>(t, lo, hi, t->M.p, msize, st));
   }
   FMM_CUDA_TRY(cudaGetLastError());
   TRY(fmm_bh_walk(t, S, F, potential, field, st));

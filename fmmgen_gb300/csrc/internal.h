@@ -20,7 +20,7 @@ struct Plan {
 };
 struct PlanSet {
   int order = -1, so = -1;
-  Plan m2l, m2m, l2l;
+  Plan m2l;
   void *dmem = nullptr;  // one allocation holding every table
 };
 const PlanSet *fmm_get_plans(int order, int so);  // cached per device
@@ -250,8 +250,8 @@ int fmm_bh_walk(DevTree *t, const double *S, double *F, int potential, int field
 // and each list by descending order (tp_perm)
 int fmm_m2l_targets(DevTree *t, const unsigned char *ord, cudaStream_t st);
 bool fmm_m2l_tc_boxes_ok(DevTree *t, cudaStream_t st);  // the level-grid path can run on this build
-// M2M of the parents / L2L into the children of cells [lo, hi), FP32 scaled expansions (shift.cu)
-int fmm_m2m_tab(DevTree *t, int lo, int hi, float *M, int mstr, cudaStream_t st);
-int fmm_l2l_tab(DevTree *t, int lo, int hi, float *L, int lstr, cudaStream_t st);
+// M2M of the parents in [lo, hi) / L2L into the cells [lo, hi) of one level, scaled expansions, float or double (shift.cu)
+template <typename T> int fmm_m2m(DevTree *t, int lo, int hi, T *M, int mstr, cudaStream_t st);
+template <typename T> int fmm_l2l(DevTree *t, int lo, int hi, T *L, int lstr, cudaStream_t st);
 int fmm_direct(const double *pos, const double *S, long N, const long *targets, long ntargets, int so,
                int potential, int field, double *F, cudaStream_t st);

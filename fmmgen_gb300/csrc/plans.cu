@@ -1,8 +1,8 @@
 // plans.cu -- task plans of the warp contraction engine.
 //
-// M2M, M2L and L2L all have the form out[n] = sum_t A[a_t] * B[b_t] over a
-// fixed, order-dependent set of (n, a, b) index triples (the sums of
-// fmmgen/expansions.py:42-78, 144-172, 175-194).  Their lengths vary strongly
+// The M2L has the form out[n] = sum_t A[a_t] * B[b_t] over a fixed,
+// order-dependent set of (n, a, b) index triples (the sums of
+// fmmgen/expansions.py:144-172).  Their lengths vary strongly
 // with |n| (M2L at p=8: 165 terms for n=0, 1 for |n|=8), so giving each lane
 // whole outputs leaves most lanes idle.  A plan flattens the triples in output
 // order and cuts the list into 32 equal contiguous lane ranges; each lane keeps
@@ -121,34 +121,6 @@ HostPlan plan_m2l(int p, int so) {
   return make_plan(tk, nl);
 }
 
-HostPlan plan_m2m(int p, int so) {
-  std::vector<std::array<int, 3>> tk;
-  int off = fmm_nterms(so - 1), nm = fmm_nterms(p);
-  for (int i = off; i < nm; i++) {
-    MI n = fmm_decode(i);
-    for (int kx = 0; kx <= n.x; kx++)
-      for (int ky = 0; ky <= n.y; ky++)
-        for (int kz = 0; kz <= n.z; kz++) {
-          if (n.d - kx - ky - kz < so) continue;
-          tk.push_back({i - off, fmm_idx3(kx, ky, kz), fmm_idx3(n.x - kx, n.y - ky, n.z - kz) - off});
-        }
-  }
-  return make_plan(tk, nm - off);
-}
-
-HostPlan plan_l2l(int p, int so) {
-  std::vector<std::array<int, 3>> tk;
-  int pl = p - so, nl = fmm_nterms(pl);
-  for (int i = 0; i < nl; i++) {
-    MI n = fmm_decode(i);
-    for (int j = 0; j < fmm_nterms(pl - n.d); j++) {
-      MI k = fmm_decode(j);
-      tk.push_back({i, j, fmm_idx3(n.x + k.x, n.y + k.y, n.z + k.z)});
-    }
-  }
-  return make_plan(tk, nl);
-}
-
 std::mutex g_mu;
 PlanSet *g_plans[16][FMM_PMAX + 1][3] = {};
 
@@ -160,32 +132,23 @@ const PlanSet *fmm_get_plans(int order, int so) {
   if (order < 0 || order > FMM_PMAX || so < 0 || so > 2) return nullptr;
   std::lock_guard<std::mutex> lk(g_mu);
   if (g_plans[dev][order][so]) return g_plans[dev][order][so];
-  HostPlan hp[3] = {plan_m2l(order, so), plan_m2m(order, so), plan_l2l(order, so)};
-  size_t bytes = 0;
-  // each of the two arrays of a plan is padded up to a 256-byte boundary
-  for (auto &h : hp) bytes += h.task.size() * 4 + h.out_seg.size() * 4 + 2 * 256;
+  const HostPlan hp = plan_m2l(order, so);
+  // the task array, padded up to a 256-byte boundary, then the outputs' segments
+  const size_t at = (hp.task.size() * 4 + 255) & ~(size_t)255, bytes = at + hp.out_seg.size() * 4;
   char *d = nullptr;
   if (cudaMalloc((void **)&d, bytes) != cudaSuccess) return nullptr;
   std::vector<char> host(bytes, 0);
+  memcpy(host.data(), hp.task.data(), hp.task.size() * 4);
+  memcpy(host.data() + at, hp.out_seg.data(), hp.out_seg.size() * 4);
   PlanSet *ps = new PlanSet();
   ps->order = order;
   ps->so = so;
   ps->dmem = d;
-  size_t o = 0;
-  Plan *dst[3] = {&ps->m2l, &ps->m2m, &ps->l2l};
-  for (int k = 0; k < 3; k++) {
-    memcpy(host.data() + o, hp[k].task.data(), hp[k].task.size() * 4);
-    dst[k]->task = (const uint32_t *)(d + o);
-    o += hp[k].task.size() * 4;
-    o = (o + 255) & ~(size_t)255;
-    memcpy(host.data() + o, hp[k].out_seg.data(), hp[k].out_seg.size() * 4);
-    dst[k]->out_seg = (const int *)(d + o);
-    o += hp[k].out_seg.size() * 4;
-    o = (o + 255) & ~(size_t)255;
-    dst[k]->iters = hp[k].iters;
-    dst[k]->nout = hp[k].nout;
-    dst[k]->nseg = hp[k].nseg;
-  }
+  ps->m2l.task = (const uint32_t *)d;
+  ps->m2l.out_seg = (const int *)(d + at);
+  ps->m2l.iters = hp.iters;
+  ps->m2l.nout = hp.nout;
+  ps->m2l.nseg = hp.nseg;
   if (cudaMemcpy(d, host.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaFree(d);
     delete ps;
