@@ -686,7 +686,7 @@ static int m2l_phase(DevTree *t, const PlanSet *ps, const T *M, T *L, bool mixed
   if (is_tc(impl) && t->ord_mode == 0 && t->nm2l > 0 && !fmm_m2l_tc_boxes_ok(t, st)) impl = M2L_H;
   // every M2L but the tensor cores' reads the target lists
   if (t->ord_mode != 0 || !(mixed && (is_tc(impl) || impl == M2L_CM))) TRY(fmm_m2l_csr(t, st));
-  // a tuned choice pins the per-pair-order kernels: 2 the engine, 4 class-major, else target-major
+  // a tuned choice pins the per-pair-order kernels: 2 the engine, 4 class-major, else harmonic
   const int timpl = t->tune.impl;
   if (t->ord_mode != 0) {
     // per-pair orders: predicted now from this pass's multipoles, or given
