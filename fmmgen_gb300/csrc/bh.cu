@@ -93,7 +93,7 @@ __device__ __forceinline__ void m2p(const BhWeight *__restrict__ W, double yx, d
 // the leaves it opens go into queues of its own, which the warp works off
 // together, each lane on its own next cell or source: neighbours accept much
 // the same number of cells, but half of them not the same ones.
-// Bound by the FP64 pipe (20 clocks of an SM per instruction, whatever its
+// Bound by the FP64 pipe (16 clocks of an SM per instruction, whatever its
 // active lanes): hence the queues (a thread per particle with its own stack ran
 // with 15 of 32 lanes active, the common walk without them with 17), ~260
 // operations per M2P at p = 4 (all derivatives in local memory took ~1,200), tests

@@ -619,7 +619,7 @@ static int run_pass(DevTree *t, const PlanSet *ps, const double *S, T *M, T *L, 
 // p = 8: 1.63 ms (tensor cores 2.58, class-major 5.3); p = 6: 0.86 (1.74, 1.87);
 // p = 4: 0.50 (0.95, 1.06); 10^4 charges, p = 4: 25 us (466); 2x10^6 Plummer
 // dipoles, p = 6: 2.8 ms (24.6); 3x10^5 charges, p = 12: 1.03 ms (the 18,564-term
-// kernels 24); FP64, 10^6 charges, p = 8: 48.9 ms (engine 184).
+// kernels 24); FP64, 10^6 charges, p = 8: 37.1 ms (engine 184).
 // Choice 0, once tensor cores with source rows gathered one by one, is the
 // harmonic kernels: its best, 4.04 ms at 10^6 charges and p = 8, was never the
 // faster one.

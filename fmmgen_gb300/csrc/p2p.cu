@@ -8,8 +8,8 @@
 // ---------------------------------------------------------------------------
 // P2P in FP64 (example/calculate.cpp:24-40, 208-216)
 // ---------------------------------------------------------------------------
-// Bound by the FP64 pipe: 1.60 operations per clock and SM measured on this
-// part (FP32: 120), so a warp's FP64 instruction takes 20 clocks of its SM and
+// Bound by the FP64 pipe: two operations per clock and SM (FP32: 128), so a
+// warp's FP64 instruction takes 16 clocks of its SM and
 // everything else -- shared-memory reads, index arithmetic, shuffles, staging
 // the sources again -- hides behind it.  What counts is that no lane idles.
 // A leaf's targets are therefore cut into groups that fill the warp: chunks of
@@ -602,7 +602,7 @@ __device__ __forceinline__ void pair_add(float &s, float &c, float s2, float c2)
   c = (c + c2) - e;
 }
 // s - c in FP64.  The conversions are done on the integer pipe: the FP64 pipe
-// would take 20 clocks of the SM for each.
+// would take 16 clocks of the SM for each.
 __device__ __forceinline__ double f2d(float x) {
   const unsigned b = __float_as_uint(x), e = (b >> 23) & 255u, m = b & 0x7fffffu;
   const unsigned E = e == 0u ? 0u : e == 255u ? 2047u : e + 896u;
