@@ -284,12 +284,11 @@ template <int P> int walk(DevTree *t, const double *S, const BhWeight *W, double
 // set when a walk was deeper than its stack.
 int fmm_bh_walk(DevTree *t, const double *S, double *F, int potential, int field, cudaStream_t st) {
   const int p = t->order, hstr = h_terms(p), nw = h_terms(p + 1);
-  TRY(fmm_reserve(t->hM, sizeof(double) * (size_t)t->ncells * hstr));
+  TRY(fmm_reserve(t->bhM, (size_t)t->ncells * hstr));
   TRY(fmm_reserve(t->bhW, (size_t)t->ncells * nw));
-  TRY(fmm_h_fold(t, t->M.p, fmm_nterms(p) - fmm_nterms(t->so - 1), (double *)t->hM.p, hstr, st));
+  TRY(fmm_h_fold(t, t->M.p, fmm_nterms(p) - fmm_nterms(t->so - 1), t->bhM.p, hstr, st));
   const long n = (long)t->ncells * nw;
-  fmm_note_launch(), k_bh_weights<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(t->ncells, p, (const double *)t->hM.p,
-                                                                               hstr, t->bhW.p);
+  fmm_note_launch(), k_bh_weights<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(t->ncells, p, t->bhM.p, hstr, t->bhW.p);
   FMM_CUDA_TRY(cudaGetLastError());
   return walk<1>(t, S, t->bhW.p, F, potential, field, st);
 }

@@ -136,7 +136,10 @@ struct DevTree {
   DevBuf<int> cm_woff, cm_wstep;          // per (tile, warp of 32 rows): its steps with a pair
   uint64_t cm_wserial = ~0ull, cm_wversion = ~0ull;  // ... of this schedule (build, cell order)
   DevBuf<BhWeight> bhW;                   // Barnes-Hut: weights of each cell's harmonic derivatives (bh.cu)
-  DevBuf<char> hM, hL, hD;                // harmonic M2L: folded multipoles, outputs, operators (m2l_h.cu)
+  // harmonic M2L, FP32 and FP64: folded multipoles, outputs, operators (m2l_h.cu).  A set for each precision, and
+  // Barnes-Hut has its own: a recorded pass holds the pointers, and no call in between may move its buffers.
+  DevBuf<char> hM[2], hL[2], hD[2];
+  DevBuf<double> bhM;                     // Barnes-Hut: folded multipoles
   DevBuf<int> tp_perm;                    // per target list: pair indices by descending per-pair order
   DevBuf<int> tp_tgt;                     // targets by list length (of this build and cell order); with per-pair
                                           // orders by level, then by their count of high-order pairs

@@ -97,11 +97,12 @@ static int run(DevTree *t, const T *M, int mstr, T *L, int lstr, const unsigned 
   }
   if (int rc = fmm_m2l_csr(t, st)) return rc;
   const int mh = line_stride<T>(h_terms(p)), lh = line_stride<T>(h_terms(pl)), dh = line_stride<T>(h_dterms(p));
-  if (fmm_reserve(t->hM, sizeof(T) * (size_t)nc * mh) || fmm_reserve(t->hL, sizeof(T) * (size_t)nc * lh) ||
-      fmm_reserve(t->hD, sizeof(T) * (size_t)t->nclasses * dh))
+  DevBuf<char> &hM = t->hM[sizeof(T) == 8], &hL = t->hL[sizeof(T) == 8], &hD = t->hD[sizeof(T) == 8];
+  if (fmm_reserve(hM, sizeof(T) * (size_t)nc * mh) || fmm_reserve(hL, sizeof(T) * (size_t)nc * lh) ||
+      fmm_reserve(hD, sizeof(T) * (size_t)t->nclasses * dh))
     return FMM_ERR_CUDA;
   if (int rc = fmm_m2l_targets(t, ord, st)) return rc;
-  T *Mh = (T *)t->hM.p, *Lh = (T *)t->hL.p, *Dh = (T *)t->hD.p;
+  T *Mh = (T *)hM.p, *Lh = (T *)hL.p, *Dh = (T *)hD.p;
   fmm_note_launch(), k_h_operators<T><<<grid_of((long)t->nclasses * fmm_nterms(p)), H_BLOCK, 0, st>>>(
       t->nclasses, p, t->cls_D.p, Dh, dh);
   fmm_note_launch(), k_h_fold<T><<<grid_of((long)nc * h_terms(p)), H_BLOCK, 0, st>>>(nc, p, so, M, mstr, Mh, mh);

@@ -1592,7 +1592,10 @@ void fmm_tree_destroy(DevTree *t) {
   fmm_release(t->child_mask); fmm_release(t->clevel); fmm_release(t->leaf_cells); fmm_release(t->cell_leaf);
   fmm_release(t->m2l_off); fmm_release(t->m2l_src); fmm_release(t->m2l_cls); fmm_release(t->m2l_order);
   fmm_release(t->m2l_cls_raw);
-  fmm_release(t->hM); fmm_release(t->hL); fmm_release(t->hD); fmm_release(t->bhW);
+  for (int k = 0; k < 2; k++) {
+    fmm_release(t->hM[k]); fmm_release(t->hL[k]); fmm_release(t->hD[k]);
+  }
+  fmm_release(t->bhM); fmm_release(t->bhW);
   t->csr_serial = ~0ull;
   fmm_release(t->p2p_off); fmm_release(t->p2p_src);
   fmm_release(t->cls_key4); fmm_release(t->cls_D); fmm_release(t->cls_Df); fmm_release(t->cls_table);
