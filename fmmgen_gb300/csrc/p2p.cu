@@ -960,8 +960,8 @@ __global__ void __launch_bounds__(32 * DIR_WARPS) k_direct(const double *pos, co
   // m targets per group, f = 32 / m lanes per target
   const int f = 32 / m, tl = lane / f, slice = lane - tl * f;
   const long t = (long)(blockIdx.x / nrank) * m + tl;
-  const bool ok = tl < m && t < nt;
-  const long i = ok ? (targets ? targets[t] : t) : -1;
+  const long i = tl < m && t < nt ? (targets ? targets[t] : t) : -1;
+  const bool ok = i >= 0;  // a negative target has no particle: its row stays as it is
   double xi = 0, yi = 0, zi = 0;
   if (ok) {
     xi = pos[3 * i];
