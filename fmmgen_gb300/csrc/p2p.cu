@@ -15,9 +15,10 @@
 // A leaf's targets are therefore cut into groups that fill the warp: chunks of
 // 32, then 16 and 8 targets with 2 and 4 lanes each, then the last m <= 7 with
 // floor(32 / m) lanes each; the f lanes of a target take every f-th source of
-// the stream and their sums are added at the end.  One warp per (leaf, group):
-// the groups of a leaf are independent warps, so leaves of several chunks do
-// not make a tail of long warps.  With one lane per target and chunks of 32 a
+// the stream and their sums are added at the end.  One warp per group, from the
+// build's units of up to 32 targets: the groups of a leaf are independent warps,
+// so leaves of several chunks do not make a tail of long warps, and the grid
+// grows with the particles, not with the largest leaf there could be.  With one lane per target and chunks of 32 a
 // leaf of 14 left 56 % of the lanes idle and one of 40 took two full passes.
 // The sources of the leaf's list are one stream (the leaves' particle ranges
 // one after the other), staged 64 at a time.
@@ -63,36 +64,23 @@ __device__ __forceinline__ void p64_one(double dx, double dy, double dz, const d
 }
 
 template <int SO, bool POT>
-__global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int *leaf_cells, int nleaves, int nlb, int nchunk,
-                                                          const int *pstart, const int *pcount, const int *off_,
-                                                          const int *src, const double *px, const double *py,
-                                                          const double *pz, const uint32_t *perm, const double *S,
-                                                          double *Fnear) {
+__global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int4 *units, int nunits, int nub, const int *pstart,
+                                                          const int *pcount, const int *off_, const int *src,
+                                                          const double *px, const double *py, const double *pz,
+                                                          const uint32_t *perm, const double *S, double *Fnear) {
   constexpr int NQ = p64_nq(SO);
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ double sp[P2P_WARPS][3][P64_CHUNK], sq[P2P_WARPS][NQ][P64_CHUNK];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int y = blockIdx.x / nlb;  // blocks by group: every leaf's first chunk, then the second ones, ...
-  const int leaf = (blockIdx.x - y * nlb) * P2P_WARPS + w;
-  if (leaf >= nleaves) return;
-  const int A = leaf_cells[leaf];
+  const int y = blockIdx.x / nub;  // blocks by group: every unit's 32 or 16 targets, then the groups of 8, then the rest
+  const int u = (blockIdx.x - y * nub) * P2P_WARPS + w;
+  if (u >= nunits) return;
+  const int4 unit = units[u];
+  const int A = unit.x, rest = unit.z & 31;  // rest: of a leaf's last unit, where that is not full
   const int a0 = pstart[A], na = pcount[A];
   // this warp's group of targets: [tb, tb + m)
-  const int full = na & ~31, rest = na & 31;
-  int tb, m;
-  if (y < nchunk) {  // a chunk of 32
-    tb = 32 * y;
-    m = tb < full ? 32 : 0;
-  } else if (y == nchunk) {
-    tb = full;
-    m = rest & 16;
-  } else if (y == nchunk + 1) {
-    tb = full + (rest & 16);
-    m = rest & 8;
-  } else {
-    tb = full + (rest & 24);
-    m = rest & 7;
-  }
+  const int tb = unit.y + (y == 0 ? 0 : y == 1 ? rest & 16 : rest & 24);
+  const int m = y == 0 ? (rest ? rest & 16 : 32) : y == 1 ? rest & 8 : rest & 7;
   if (m == 0) return;
   const int f = 32 / m;  // lanes per target
   const int tl = lane / f, slice = lane - tl * f;
@@ -904,16 +892,14 @@ int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st) {
     else
       fmm_note_launch(), k_p2p64_gather<false><<<grid, 128, 0, st>>>(P, nl);
   } else {
-    // a leaf holds fewer than ncrit particles (a root leaf fewer than N): its full chunks of 32, then three groups
-    const int nchunk = (int)(std::min(t->ncrit - 1, t->N) / 32);
-    const int nlb = (int)fmm_blocks(nl, P2P_WARPS);
+    const int nub = (int)fmm_blocks(t->np2p_units, P2P_WARPS);
     decltype(&k_p2p64<0, true>) k = so == 0   ? (pot ? k_p2p64<0, true> : k_p2p64<0, false>)
                                     : so == 1 ? (pot ? k_p2p64<1, true> : k_p2p64<1, false>)
                                               : k_p2p64<2, true>;
     if (int rc = fmm_mark_kernel(t, 2, st)) return rc;
-    fmm_note_launch(), k<<<(unsigned)nlb * (nchunk + 3), 32 * P2P_WARPS, 0, st>>>(
-        t->leaf_cells.p, nl, nlb, nchunk, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p, t->py.p, t->pz.p,
-        t->perm.p, S, t->Fnear.p);
+    fmm_note_launch(), k<<<3 * (unsigned)nub, 32 * P2P_WARPS, 0, st>>>(
+        t->p2p_units.p, t->np2p_units, nub, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p, t->py.p,
+        t->pz.p, t->perm.p, S, t->Fnear.p);
   }
   FMM_CUDA_TRY(cudaGetLastError());
   return fmm_mark_kernel(t, 3, st);
