@@ -185,18 +185,19 @@ __global__ void __launch_bounds__(SH_BS) k_l2l(int lo, int hi, int p, const unsi
 
 constexpr long SH_GRID = 152 * 8;
 
-template <typename K> int shift_smem_attr(K k, size_t bytes) {
-  if (bytes > 32 * 1024) FMM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return FMM_OK;
-}
+// The M2M's rows.  Its limit is that of the longest ones: it holds for the process, and another thread may be about to
+// launch them.
+template <typename T> constexpr size_t m2m_bytes(int nterms) { return 16 * sizeof(T) * (size_t)nterms; }
 
 }  // namespace
 
 // the multipoles of the parents in [lo, hi), the cells of one level, from their children's
 template <typename T> int fmm_m2m(DevTree *t, int lo, int hi, T *M, int mstr, cudaStream_t st) {
   if (hi <= lo) return FMM_OK;
-  const size_t bytes = 16 * sizeof(T) * (size_t)fmm_nterms(t->order);
-  if (int rc = shift_smem_attr(k_m2m<T>, bytes)) return rc;
+  const size_t bytes = m2m_bytes<T>(fmm_nterms(t->order));
+  if (bytes > 32 * 1024)
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2m<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)m2m_bytes<T>(FMM_NTMAX)));
   fmm_note_launch(), k_m2m<T><<<(unsigned)std::min<long>(hi - lo, SH_GRID), SH_BS, bytes, st>>>(
       lo, hi, t->order, t->so, t->child_mask.p, t->child_first.p, t->cx.p, t->cy.p, t->cz.p, t->cr.p, M, mstr);
   FMM_CUDA_TRY(cudaGetLastError());
@@ -211,7 +212,7 @@ template <typename T> int fmm_l2l(DevTree *t, int lo, int hi, T *L, int lstr, cu
   if (l >= t->nlevels) return FMM_ERR_STATE;
   const int plo = t->level_off[l - 1], phi = t->level_off[l], p = t->order - t->so;
   const size_t bytes = 7 * sizeof(T) * (size_t)fmm_nterms(p);
-  if (int rc = shift_smem_attr(k_l2l<T>, bytes)) return rc;
+  static_assert(7 * sizeof(T) * FMM_NTMAX <= 32 * 1024, "within every kernel's limit");
   fmm_note_launch(), k_l2l<T><<<(unsigned)std::min<long>(phi - plo, SH_GRID), SH_BS, bytes, st>>>(
       plo, phi, p, t->child_mask.p, t->child_first.p, t->cx.p, t->cy.p, t->cz.p, t->cr.p, L, lstr);
   FMM_CUDA_TRY(cudaGetLastError());

@@ -1447,7 +1447,7 @@ static int build_classes(DevTree *t, cudaStream_t st) {
 // classes than a bitmap in shared memory holds.  15.7M pairs (10^6 charges, with the
 // targets' order): 0.67 ms with an atomic per pair, 0.31 with one per run of a
 // target's; a step of 10^6 charges 8.81 -> 8.55 ms, of 512 forests 52.6 -> 49.7.
-constexpr int CSR_MAX_CLASSES = 65536 / 8 * 32;
+constexpr int CSR_SMEM = 65536, CSR_MAX_CLASSES = CSR_SMEM / 8 * 32;
 // one atomic for a warp's pairs of one target (the walk emits a target's pairs in runs)
 __global__ void k_csr_count(const int *tgt, long n, int *cnt) {
   const long i = blockIdx.x * 256l + threadIdx.x;
@@ -1524,9 +1524,10 @@ int fmm_m2l_csr(DevTree *t, cudaStream_t st) {
     FMM_CUDA_TRY(cudaMemcpyAsync(cur, t->m2l_off.p, sizeof(int) * nc, cudaMemcpyDeviceToDevice, st));
     fmm_note_launch(), k_csr_scatter<<<fmm_blocks(n, 256), 256, 0, st>>>(t->m2l_tgt_raw.p, t->m2l_src_raw.p,
                                                                          t->m2l_cls_raw.p, n, cur, list);
-    const int nw = (t->nclasses + 31) / 32, warps = std::max(1, std::min(8, (int)(65536 / (8 * nw))));
+    const int nw = (t->nclasses + 31) / 32, warps = std::max(1, std::min(8, CSR_SMEM / (8 * nw)));
     const size_t smem = (size_t)8 * nw * warps;
-    FMM_CUDA_TRY(cudaFuncSetAttribute(k_csr_place, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most it ever takes: the limit holds for the process, and another thread may be about to launch with more
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_csr_place, cudaFuncAttributeMaxDynamicSharedMemorySize, CSR_SMEM));
     fmm_note_launch(), k_csr_place<<<fmm_blocks(nc, warps), 32 * warps, smem, st>>>(t->m2l_off.p, nc, nw, list,
                                                                                     t->m2l_src.p, t->m2l_cls.p);
     FMM_CUDA_TRY(cudaGetLastError());
