@@ -39,7 +39,15 @@ __host__ __device__ __forceinline__ MI fmm_decode(int i) {
 #define FMM_EFLAG_RANGE 2u     // an M2L offset outside the class table's range
 #define FMM_EFLAG_BOUNDS 4u    // an index check failed (never expected)
 #define FMM_EFLAG_KEYS 8u      // the particle keys need more levels (the build recomputes them)
+#define FMM_EFLAG_WIDE 16u     // not an error: pairs across more levels than FP32 factors hold (fmm_wide_levels)
 #define FMM_KEYLEVELS 10       // levels of digits in the first keys of a build
+
+// Level differences up to which an FP32 M2L scales the source's coefficients, by
+// 2^(degree x difference), inside FP32's exponents, with room for the coefficients
+// themselves: 2^96 at most, by the order's family of generated kernels (m2l_h.cuh).
+__host__ __device__ __forceinline__ constexpr int fmm_wide_levels(int p) {
+  return p <= 4 ? 24 : p <= 6 ? 16 : p <= 8 ? 12 : 8;
+}
 
 // Quadrupole sources (source order 2): S holds the degree-2 multipole
 // coefficients (xx, xy, xz, yy, yz, zz) and a source at offset r = target -

@@ -630,6 +630,10 @@ bool fmm_m2l_gen_supported(int p, int so) {
   int kt[4];
   return m2l_reg_kernels(p, so, kg, kt) > 0;
 }
+// The other FP32 CUDA-core kernels have no way with pairs across many levels (m2l_h.cu).
+static bool cuda_cores_wide(const DevTree *t, bool mixed, int impl) {
+  return mixed && (t->eflags & FMM_EFLAG_WIDE) && (impl == M2L_GEN || impl == M2L_ENGINE || impl == M2L_CM);
+}
 static int m2l_impl(const DevTree *t, int precision) {
   if (precision == 0) return t->tune.impl == M2L_ENGINE ? M2L_ENGINE : M2L_H;
   const bool tc_ok = fmm_m2l_tc_supported(t->order, t->so), gen_ok = fmm_m2l_gen_supported(t->order, t->so);
@@ -638,6 +642,7 @@ static int m2l_impl(const DevTree *t, int precision) {
   if (is_tc(impl) && (!tc_ok || t->nclasses > 262144)) impl = M2L_H;  // class bitmap of the tile schedule
   if (impl == M2L_CM && (!fmm_m2l_cm_supported(t->order, t->so) || t->nclasses > 262144)) impl = M2L_H;
   if (impl == M2L_GEN && !gen_ok) impl = M2L_H;
+  if (cuda_cores_wide(t, true, impl)) impl = M2L_H;
   return impl;
 }
 
@@ -687,7 +692,7 @@ static int m2l_phase(DevTree *t, const PlanSet *ps, const T *M, T *L, bool mixed
   // every M2L but the tensor cores' reads the target lists
   if (t->ord_mode != 0 || !(mixed && (is_tc(impl) || impl == M2L_CM))) TRY(fmm_m2l_csr(t, st));
   // a tuned choice pins the per-pair-order kernels: 2 the engine, 4 class-major, else harmonic
-  const int timpl = t->tune.impl;
+  const int timpl = cuda_cores_wide(t, mixed, t->tune.impl) ? (int)M2L_H : t->tune.impl;
   if (t->ord_mode != 0) {
     // per-pair orders: predicted now from this pass's multipoles, or given
     if (t->ord_mode == 2) TRY(fmm_learned_orders(t, st));
@@ -1001,7 +1006,7 @@ int fmm_tree_build_evaluate(DevTree *t, const double *pos, long N, long ncrit, i
   } else {
     rc = fused_pass<double>(t, ps, S, t->M.p, t->L.p, false, precision, (int)msize, (int)lsize, fmm_nterms(p), st);
   }
-  if (rc == FMM_OK && t->eflags) {  // the build's own error, after the near-field stream is done
+  if (rc == FMM_OK && (t->eflags & (FMM_EFLAG_DEPTH | FMM_EFLAG_RANGE))) {  // the build's own error, after the near-field stream is done
     FMM_CUDA_TRY(cudaStreamSynchronize(t->s_near));
     return (t->eflags & FMM_EFLAG_DEPTH) ? FMM_ERR_DEPTH : FMM_ERR_RANGE;
   }

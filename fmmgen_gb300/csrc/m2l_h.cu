@@ -63,16 +63,69 @@ __global__ void k_h_unfold(int ncells, int pl, const T *Lh, int hstr, T *L, int 
   L[(size_t)c * lstr + i] = (j & 1) ? -v : v;
 }
 
-// the operator entries with k_z <= 2 of every class
+// the operator entries with k_z <= 2 of every class; FP32: zeros for the classes that k_h_wide takes
 template <typename T>
-__global__ void k_h_operators(int ncls, int p, const double *D, T *Dh, int hstr) {
+__global__ void k_h_operators(int ncls, int p, const int *key4, const double *D, T *Dh, int hstr) {
   const int nt = fmm_nterms(p);
   const long g = blockIdx.x * (long)H_BLOCK + threadIdx.x;
   const long c = g / nt;
   const int i = (int)(g - c * nt);
   if (c >= ncls) return;
   const MI k = fmm_decode(i);
-  if (k.z <= 2) Dh[(size_t)c * hstr + h_dindex(k.x, k.y, k.z)] = (T)D[(size_t)c * nt + i];
+  const bool none = sizeof(T) == 4 && -key4[4 * c] > fmm_wide_levels(p);
+  if (k.z <= 2) Dh[(size_t)c * hstr + h_dindex(k.x, k.y, k.z)] = none ? T(0) : (T)D[(size_t)c * nt + i];
+}
+
+// The pairs of a mixed pass whose source is a cell so much larger than the target
+// that FP32 holds neither 2^(degree x levels) nor the operator of high degree
+// (fmm_wide_levels), in FP64 and added to L: few in any tree (coarse leaves that a
+// deep cluster just accepts), so the plain contraction, a warp per target cell.  The
+// other direction needs nothing: a much smaller source's higher degrees vanish.
+constexpr int WIDE_WARPS = 4;
+__global__ void __launch_bounds__(32 * WIDE_WARPS) k_h_wide(int ncells, int p, int so, const unsigned char *clevel,
+                                                            const int *off, const int *src, const int *cls,
+                                                            const unsigned char *ord, const double *D, const float *M,
+                                                            int mstr, float *L, int lstr) {
+  __shared__ double sM[WIDE_WARPS][FMM_NTMAX], sL[WIDE_WARPS][FMM_NTMAX];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int A = blockIdx.x * WIDE_WARPS + w;
+  if (A >= ncells) return;
+  const int la = clevel[A], wide = fmm_wide_levels(p);
+  if (la <= wide) return;
+  const int moff = fmm_nterms(so - 1), nl = fmm_nterms(p - so), nt = fmm_nterms(p);
+  const int k0 = off[A], k1 = off[A + 1];
+  bool some = false;
+  for (int kb = k0; kb < k1; kb += 32) {
+    const int k = kb + lane;
+    unsigned todo = __ballot_sync(0xffffffffu, k < k1 && la - (int)clevel[src[min(k, k1 - 1)]] > wide);
+    while (todo) {
+      const int j = kb + __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int B = src[j], dl = la - (int)clevel[B], q = ord ? min(max((int)ord[j], so + 1), p) : p;
+      const double *Dc = D + (size_t)cls[j] * nt;
+      if (!some)
+        for (int i = lane; i < nl; i += 32) sL[w][i] = 0.0;
+      some = true;
+      __syncwarp();
+      for (int i = moff + lane; i < fmm_nterms(q); i += 32)
+        sM[w][i] = (double)M[(size_t)B * mstr + i - moff] * h_exp2<double>(dl * (int)fmm_decode(i).d);
+      __syncwarp();
+      for (int i = lane; i < nl; i += 32) {
+        const MI n = fmm_decode(i);
+        double v = 0;
+        int m = moff;
+        for (int d = so; d <= q - n.d; d++)
+          for (int x = d; x >= 0; x--)
+            for (int y = d - x; y >= 0; y--, m++) v += Dc[fmm_idx3(n.x + x, n.y + y, n.z + d - x - y)] * sM[w][m];
+        sL[w][i] += v;
+      }
+    }
+  }
+  if (some)
+    for (int i = lane; i < nl; i += 32) {
+      float *o = L + (size_t)A * lstr + i;
+      *o = (float)((double)*o + sL[w][i]);
+    }
 }
 
 unsigned grid_of(long n) { return (unsigned)((n + H_BLOCK - 1) / H_BLOCK); }
@@ -104,7 +157,7 @@ static int run(DevTree *t, const T *M, int mstr, T *L, int lstr, const unsigned 
   if (int rc = fmm_m2l_targets(t, ord, st)) return rc;
   T *Mh = (T *)hM.p, *Lh = (T *)hL.p, *Dh = (T *)hD.p;
   fmm_note_launch(), k_h_operators<T><<<grid_of((long)t->nclasses * fmm_nterms(p)), H_BLOCK, 0, st>>>(
-      t->nclasses, p, t->cls_D.p, Dh, dh);
+      t->nclasses, p, t->cls_key4.p, t->cls_D.p, Dh, dh);
   fmm_note_launch(), k_h_fold<T><<<grid_of((long)nc * h_terms(p)), H_BLOCK, 0, st>>>(nc, p, so, M, mstr, Mh, mh);
   HParams<T> P;
   P.tgt = t->tp_tgt.p;
@@ -129,6 +182,10 @@ static int run(DevTree *t, const T *M, int mstr, T *L, int lstr, const unsigned 
   if (!rc) rc = fmm_mark_kernel(t, 1, st);
   if (rc) return rc;
   fmm_note_launch(), k_h_unfold<T><<<grid_of((long)nc * fmm_nterms(pl)), H_BLOCK, 0, st>>>(nc, pl, Lh, lh, L, lstr);
+  if constexpr (sizeof(T) == 4)
+    if (t->eflags & FMM_EFLAG_WIDE)
+      fmm_note_launch(), k_h_wide<<<fmm_blocks(nc, WIDE_WARPS), 32 * WIDE_WARPS, 0, st>>>(
+          nc, p, so, t->clevel.p, t->m2l_off.p, t->m2l_src.p, t->m2l_cls.p, ord, t->cls_D.p, M, mstr, L, lstr);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
 }

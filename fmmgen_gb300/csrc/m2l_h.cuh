@@ -45,7 +45,9 @@ template <int N> __device__ __forceinline__ void h_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 template <typename T> __device__ __forceinline__ T h_exp2(int e);
-template <> __device__ __forceinline__ float h_exp2<float>(int e) { return __int_as_float((e + 127) << 23); }
+template <> __device__ __forceinline__ float h_exp2<float>(int e) {  // e <= 127; zero below FP32's normal numbers
+  return e < -126 ? 0.f : __int_as_float((e + 127) << 23);
+}
 template <> __device__ __forceinline__ double h_exp2<double>(int e) {
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
@@ -143,11 +145,13 @@ struct HList {
     if (!on) B = c = -1;
     return on_any;
   }
-  // orders and level difference of the current pair; whether a next one follows
-  __device__ __forceinline__ void look_ahead(int dmin) {
+  // orders and level difference of the current pair; whether a next one follows.  A pair across more than `wide`
+  // levels has an operator of zeros (k_h_operators): its source stays as it is.
+  __device__ __forceinline__ void look_ahead(int dmin, int wide = 1 << 20) {
     const bool on = q >= dmin, onn = qn >= dmin;
     ql = on ? q : -1;
     dl = on ? la - (int)clevel[B] : 0;
+    if (dl > wide) dl = 0;
     rescale = __any_sync(0xffffffffu, dl != 0);
     on_next = __any_sync(0xffffffffu, onn);  // lists go by descending order: no lane on, none later
     qmaxn = (int)__reduce_max_sync(0xffffffffu, (unsigned)(onn ? qn : 0));

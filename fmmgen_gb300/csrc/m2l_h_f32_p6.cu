@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(256, 1) k_m2lh_f32_p6_0(const HParams<float> P
     h_commit();
   }
   while (it.on_any) {
-    it.look_ahead(0);
+    it.look_ahead(0, fmm_wide_levels(6));
     const int ql = it.ql;
     h_wait<1>();  // the source row and the operator's first half
     __syncwarp();

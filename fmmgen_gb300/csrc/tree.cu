@@ -761,12 +761,14 @@ constexpr uint32_t RANK_MAX = 32768;
 // ids by rank (none: the keys are sorted); the class table entry of each key; *same cleared unless the sorted
 // keys are the previous build's, which they replace
 __global__ void k_class_rank(const uint64_t *uniq, int nu, const uint32_t *slot, const uint32_t *rank, int *tabval,
-                             int *key4, uint64_t *prev, uint32_t *same) {
+                             int *key4, uint64_t *prev, uint32_t *same, int wide, uint32_t *eflags) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nu) return;
   const uint32_t r = rank ? rank[i] : (uint32_t)i;
   tabval[slot[i]] = (int)r;
-  key_decode(uniq[i], key4 + 4 * (size_t)r);
+  int *k4 = key4 + 4 * (size_t)r;
+  key_decode(uniq[i], k4);
+  if (abs(k4[0]) > wide) atomicOr(eflags, FMM_EFLAG_WIDE);
   if (prev[r] != uniq[i]) {
     *same = 0;
     prev[r] = uniq[i];
@@ -1418,7 +1420,8 @@ static int build_classes(DevTree *t, cudaStream_t st) {
   t->ncls_prev = (int)ncls;
   t->order_prev = p;
   fmm_note_launch(), k_class_rank<<<fmm_blocks(std::max(ncls, 1u), 256), 256, 0, st>>>(
-      U1, (int)ncls, I1, counted ? I2 : nullptr, t->cls_table.p, t->cls_key4.p, t->cls_prev.p, t->d_cls_same.p);
+      U1, (int)ncls, I1, counted ? I2 : nullptr, t->cls_table.p, t->cls_key4.p, t->cls_prev.p, t->d_cls_same.p,
+      fmm_wide_levels(p), t->d_eflags.p);
   // the class of each walk-order pair
   fmm_note_launch(), k_class_lookup<<<fmm_blocks(n, 256), 256, 0, st>>>(keys, n, t->cls_hkeys.p, hsize - 1,
                                                                          t->cls_table.p, t->m2l_cls_raw.p);

@@ -165,7 +165,7 @@ def emit(pmax, ki, kern, tag, typ, size):
         L.append("    h_commit();" if s is None else s)
     L += ["    h_commit();", "  }"]
     L.append("  while (it.on_any) {")
-    L.append(f"    it.look_ahead({dmin});")
+    L.append(f"    it.look_ahead({dmin}{f', fmm_wide_levels({pmax})' if f32 else ''});")
     L.append("    const int ql = it.ql;")
     if f32:
         L.append("    h_wait<1>();  // the source row and the operator's first half")

@@ -253,7 +253,10 @@ int fmmgen_tree_m2l_work(fmmgen_tree *tree, double *out4);
  * orders up to 12 for charges, 8 for dipoles.  FP64 passes run 5, or the
  * engine with impl 2.  Per-pair M2L orders (fmmgen_tree_set_m2l_orders, an
  * order model) run on 5, on the class-major kernels with impl 4 (mixed
- * passes), on the engine with impl 2.
+ * passes), on the engine with impl 2.  Mixed passes of a build with M2L pairs
+ * across so many levels that FP32 cannot hold the factors between the cells'
+ * scales (24 levels for p <= 4, 16 for p <= 6, 12 for p <= 8, else 8) run 5 in
+ * place of 1, 2 and 4; those pairs are done in FP64.
  * nslots: tensor-core pipeline depth (operand slots), 0 = as many as fit.
  * grouping: order of a level's cells in M2L tiles and warps, 0 by octant
  * within the parent, 1 Morton.  overlap: 1 (2) runs the tensor-core M2L on a
