@@ -58,7 +58,7 @@ struct DevTree {
   DevBuf<uint32_t> perm, perm2;           // sorted position -> caller's particle index
   DevBuf<double> px, py, pz;              // sorted positions (FP64)
   DevBuf<float4> phi4, plo4, sdip;        // FP32 P2P staging: (hi offset from root centre, q), (lo, index), dipole
-  DevBuf<float4> lorg;                    // per leaf: origin of its frame in FP32, a coordinate outside the root cube
+  DevBuf<float> lpad;                     // per leaf: a coordinate outside its root cube
   DevBuf<float2> levf;                    // per-level half-width as an FP32 (hi, lo) pair
   // cells, level-major, Morton order within a level
   DevBuf<double> cx, cy, cz;

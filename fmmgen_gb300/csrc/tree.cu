@@ -1586,7 +1586,7 @@ void fmm_tree_destroy(DevTree *t) {
   t->gstream = nullptr;
   fmm_release(t->keys); fmm_release(t->keys2); fmm_release(t->perm); fmm_release(t->perm2);
   fmm_release(t->px); fmm_release(t->py); fmm_release(t->pz);
-  fmm_release(t->phi4); fmm_release(t->plo4); fmm_release(t->sdip); fmm_release(t->lorg); fmm_release(t->p2p_units);
+  fmm_release(t->phi4); fmm_release(t->plo4); fmm_release(t->sdip); fmm_release(t->lpad); fmm_release(t->p2p_units);
   fmm_release(t->sym_own); fmm_release(t->sym_get); fmm_release(t->sym_place); fmm_release(t->sym_shares);
   fmm_release(t->sym_units); fmm_release(t->sym_totals);
   fmm_release(t->levf);
