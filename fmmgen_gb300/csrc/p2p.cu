@@ -583,12 +583,13 @@ __device__ __forceinline__ void pair_add(float &s, float &c, float s2, float c2)
   s = t;
   c = (c + c2) - e;
 }
-// s - c in FP64.  The conversions are done on the integer pipe: the FP64 pipe
-// would take 16 clocks of the SM for each.
+// x in FP64, by the integer pipe: the FP64 pipe would take 16 clocks of the SM for
+// each.  (It does take subnormal numbers, which have no leading one.)
 __device__ __forceinline__ double f2d(float x) {
   const unsigned b = __float_as_uint(x), e = (b >> 23) & 255u, m = b & 0x7fffffu;
+  if (e == 0u && m) return (double)x;
   const unsigned E = e == 0u ? 0u : e == 255u ? 2047u : e + 896u;
-  return __hiloint2double((int)((b & 0x80000000u) | (E << 20) | (E ? m >> 3 : 0u)), (int)(E ? m << 29 : 0u));
+  return __hiloint2double((int)((b & 0x80000000u) | (E << 20) | (m >> 3)), (int)(m << 29));
 }
 
 // ---- two sources per instruction (packed FP32x2) ----
