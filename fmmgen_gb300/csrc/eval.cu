@@ -1070,6 +1070,7 @@ int fmm_tree_evaluate_bh(DevTree *t, const double *S, double *F, int potential, 
     return FMM_ERR_DEPTH;
   }
   t->last_prec = 0;  // the FP64 multipoles of this pass are in t->M
+  t->p64_last = false;
   return FMM_OK;
 }
 

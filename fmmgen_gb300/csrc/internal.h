@@ -100,8 +100,9 @@ struct DevTree {
   DevBuf<int4> sym_units;
   DevBuf<unsigned long long> sym_totals;
   DevBuf<double> sym_shares;
-  long sym_places = 0, sym_nunits = 0;
-  uint64_t sym_serial = ~0ull;
+  long sym_places = -1, sym_nunits = 0;   // places: -1 where this build's pairs go one way
+  uint64_t sym_serial = ~0ull;            // the build they belong to
+  bool p64_last = false;                  // the last evaluation had an FP64 near field
   // M2L translation classes: operator vectors D^(k)(d/s_target), |k| <= order
   DevBuf<int> cls_key4;                   // [nclasses][4]: dlev, dx, dy, dz
   DevBuf<double> cls_D;                   // [nclasses][Nterms(order)]
@@ -234,6 +235,8 @@ bool fmm_m2l_tc_step_work(int p, int so, long long *mmas, double *flops);
 // tensor-core M2L with source rows boxed from level grids (FMM_ERR_STATE where a level is not complete)
 int fmm_m2l_tc(DevTree *t, const float *M, int mstr, float *L, int lstr, cudaStream_t st);
 void fmm_tcg_release(DevTree *t);
+// FP64 near field: lays this build's pairs out where the last evaluation had one (p2p.cu)
+int fmm_p2p_prepare(DevTree *t, cudaStream_t st);
 // marks the start (which 0) / end (1) of the pass's M2L kernels, the start (2) / end (3) of its
 // P2P kernel, on their streams
 int fmm_mark_kernel(DevTree *t, int which, cudaStream_t st);

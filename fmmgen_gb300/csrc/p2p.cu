@@ -188,7 +188,9 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int4 *units, int
 // barrier orders the steps.
 // An entry whose reverse is not listed (the walk gives symmetric lists; nothing
 // here relies on it) and the leaf itself go one way.  The buffer is at most
-// P64_SHARES; systems that would need more take k_p2p64.
+// P64_SHARES; systems that would need more take k_p2p64, which adds in another
+// order: the choice is the tree's alone, not that of the memory that happens to be
+// free (but for a device that has none left for the buffer).
 // Measured (one GB300): 10^6 charges: 158 -> 114 ms, the 86,400 dipoles 10.2 -> 8.8 ms.
 constexpr size_t P64_SHARES = (size_t)4 << 30;
 
@@ -450,50 +452,45 @@ __global__ void __launch_bounds__(128) k_p2p64_gather(const P64Args P, int nleav
   }
 }
 
-// The owners and places of this build's pairs and room for the shares; *places:
-// particles in the buffer, or -1 where the pairs are to be done one way: more
-// shares than P64_SHARES, no memory to spare for them, or a capture of a build
-// whose pairs are not laid out yet.  Reads the totals back, once per build.
-static int p64_pairs(DevTree *t, long *places, cudaStream_t st) {
+// The owners and places of this build's pairs and room for the shares: once per
+// build, with a wait for the totals.  No room on the device leaves the build without
+// them, for all its passes.
+static int p64_layout(DevTree *t, cudaStream_t st) {
+  if (t->sym_serial == t->build_serial) return FMM_OK;
   const int nl = t->nleaves;
-  *places = -1;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  FMM_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
-  if (t->sym_serial != t->build_serial) {
-    if (cap != cudaStreamCaptureStatusNone) return FMM_OK;
-    const size_t n = (size_t)std::max(t->np2p, 1L), nu = (size_t)nl + n / 32;
-    if (fmm_reserve(t->sym_own, n) || fmm_reserve(t->sym_get, n) || fmm_reserve(t->sym_place, n + (size_t)nl) ||
-        fmm_reserve(t->sym_units, nu) || fmm_reserve(t->sym_totals, 2)) {
-      cudaGetLastError();
-      return FMM_OK;
-    }
-    FMM_CUDA_TRY(cudaMemsetAsync(t->sym_totals.p, 0, 2 * sizeof(unsigned long long), st));
-    fmm_note_launch(), k_sym_places<<<fmm_blocks(nl, 8), 256, 0, st>>>(
-        t->leaf_cells.p, nl, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->sym_place.p, t->sym_place.p + n,
-        t->sym_units.p, t->sym_totals.p);
-    fmm_note_launch(), k_sym_pairs<<<fmm_blocks(nu, 8), 256, 0, st>>>(t->sym_units.p, t->sym_totals.p, t->p2p_off.p,
-                                                                      t->p2p_src.p, t->sym_place.p, t->sym_own.p,
-                                                                      t->sym_get.p);
-    FMM_CUDA_TRY(cudaGetLastError());
-    unsigned long long v[2] = {0, 0};
-    FMM_CUDA_TRY(cudaMemcpyAsync(v, t->sym_totals.p, sizeof(v), cudaMemcpyDeviceToHost, st));
-    FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    t->sym_nunits = (long)v[0];
-    t->sym_places = (long)v[1];
-    t->sym_serial = t->build_serial;
+  const size_t n = (size_t)std::max(t->np2p, 1L), nu = (size_t)nl + n / 32;
+  t->sym_serial = t->build_serial;
+  t->sym_places = -1;
+  if (fmm_reserve(t->sym_own, n) || fmm_reserve(t->sym_get, n) || fmm_reserve(t->sym_place, n + (size_t)nl) ||
+      fmm_reserve(t->sym_units, nu) || fmm_reserve(t->sym_totals, 2)) {
+    cudaGetLastError();
+    return FMM_OK;
   }
-  const size_t room = 4 * (size_t)std::max(t->sym_places, 1L);
+  FMM_CUDA_TRY(cudaMemsetAsync(t->sym_totals.p, 0, 2 * sizeof(unsigned long long), st));
+  fmm_note_launch(), k_sym_places<<<fmm_blocks(nl, 8), 256, 0, st>>>(
+      t->leaf_cells.p, nl, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->sym_place.p, t->sym_place.p + n, t->sym_units.p,
+      t->sym_totals.p);
+  fmm_note_launch(), k_sym_pairs<<<fmm_blocks(nu, 8), 256, 0, st>>>(t->sym_units.p, t->sym_totals.p, t->p2p_off.p,
+                                                                    t->p2p_src.p, t->sym_place.p, t->sym_own.p,
+                                                                    t->sym_get.p);
+  FMM_CUDA_TRY(cudaGetLastError());
+  unsigned long long v[2] = {0, 0};
+  FMM_CUDA_TRY(cudaMemcpyAsync(v, t->sym_totals.p, sizeof(v), cudaMemcpyDeviceToHost, st));
+  FMM_CUDA_TRY(cudaStreamSynchronize(st));
+  const size_t room = 4 * std::max((size_t)v[1], (size_t)1);
   if (room * sizeof(double) > P64_SHARES) return FMM_OK;
-  if (room > t->sym_shares.cap) {
-    size_t avail = 0, all = 0;  // an eighth of what is free at most: the rest of the pass needs its buffers too
-    if (cap != cudaStreamCaptureStatusNone || cudaMemGetInfo(&avail, &all) != cudaSuccess ||
-        room * sizeof(double) > avail / 8 || fmm_reserve(t->sym_shares, room)) {
-      cudaGetLastError();
-      return FMM_OK;
-    }
+  if (fmm_reserve(t->sym_shares, room)) {
+    cudaGetLastError();
+    return FMM_OK;
   }
-  *places = t->sym_places;
+  t->sym_nunits = (long)v[0];
+  t->sym_places = (long)v[1];
   return FMM_OK;
+}
+
+// At the end of a build of a tree last evaluated in FP64: the next pass may be captured.
+int fmm_p2p_prepare(DevTree *t, cudaStream_t st) {
+  return t->so <= 1 && t->p64_last ? p64_layout(t, st) : FMM_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -829,6 +826,7 @@ __global__ void __launch_bounds__(32, SO ? 24 : 16) k_p2p32(const P2PArgs P) {
 // ---------------------------------------------------------------------------
 int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st) {
   const int nl = t->nleaves, so = t->so;
+  t->p64_last = !mixed;
   if (mixed && so <= 1) {  // quadrupole sources take the FP64 kernel in every precision
     const bool pot = t->pass_potential;
     decltype(&k_p2p32<true, 0>) k = so ? (pot ? k_p2p32<true, 1> : k_p2p32<false, 1>)
@@ -841,10 +839,15 @@ int fmm_p2p_launch(DevTree *t, bool mixed, const double *S, cudaStream_t st) {
     return fmm_mark_kernel(t, 3, st);
   }
   const bool pot = t->pass_potential;
-  long places = -1;
-  if (so <= 1)
-    if (int rc = p64_pairs(t, &places, st)) return rc;
-  if (places >= 0) {
+  bool once = so <= 1;
+  if (once) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    FMM_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    if (cap == cudaStreamCaptureStatusNone)
+      if (int rc = p64_layout(t, st)) return rc;
+    once = t->sym_serial == t->build_serial && t->sym_places >= 0;  // a captured first pass may have none: one way
+  }
+  if (once) {
     const P64Args P = {t->sym_units.p, t->leaf_cells.p, t->pstart.p, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->px.p,
                        t->py.p, t->pz.p, t->perm.p, S, t->sym_own.p, t->sym_get.p,
                        t->sym_place.p + std::max(t->np2p, 1L), t->sym_shares.p, t->Fnear.p};
@@ -1083,8 +1086,9 @@ int fmm_direct(const double *pos, const double *S, long N, const long *targets, 
       if (so == 0) fmm_note_launch(), k_direct_sym<0><<<nb, DIR_TILE, 0, st>>>(pos, S, N, (int)tiles, parts);
       else fmm_note_launch(), k_direct_sym<1><<<nb, DIR_TILE, 0, st>>>(pos, S, N, (int)tiles, parts);
       fmm_note_launch(), k_direct_sum<<<(unsigned)tiles, DIR_TILE, 0, st>>>(parts, N, (int)tiles, potential, field, F);
-      FMM_CUDA_TRY(cudaGetLastError());
+      const cudaError_t e = cudaGetLastError();
       FMM_CUDA_TRY(cudaFreeAsync(parts, st));
+      FMM_CUDA_TRY(e);
       return FMM_OK;
     }
     cudaGetLastError();  // no memory: one way

@@ -977,6 +977,7 @@ int fmm_tree_build(DevTree *t, const double *pos, long N, long ncrit, int order,
 // defer_classes leaves them to this call).
 int fmm_tree_finish_build(DevTree *t, cudaStream_t st) {
   TRY(build_classes(t, st));
+  if (!(t->eflags & FMM_EFLAG_DEPTH)) TRY(fmm_p2p_prepare(t, st));
   TRY(rec(t, 5, st));
   FMM_CUDA_TRY(cudaMemcpyAsync(&t->eflags, t->d_eflags.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   FMM_CUDA_TRY(cudaStreamSynchronize(st));

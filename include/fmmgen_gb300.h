@@ -161,7 +161,10 @@ int fmmgen_tree_set_graph(fmmgen_tree *tree, int enable);
 
 /* Tree::compute_field_exact / evaluate_direct (example/calculate.cpp:252-264):
  * FP64 O(N^2) sum for the targets listed in `targets` (device, NULL = all N);
- * F is [ntargets][OUTPUTSIZE] in the order of `targets`. */
+ * F is [ntargets][OUTPUTSIZE] in the order of `targets`.  All N charges or
+ * dipoles, 4,096 of them or more: each pair once, with N^2 / 8 bytes (up to 4 GiB,
+ * N = 185,000) from the stream's memory pool for the call; without them, above
+ * that, and in a captured call one way, which adds in another order. */
 int fmmgen_gpu_direct(const double *pos, const double *S, long N, const long *targets, long ntargets,
                       int source_order, int potential, int field, double *F, void *stream);
 
