@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(32 * P2P_WARPS) k_p2p64(const int4 *units, int
 // barrier orders the steps.
 // An entry whose reverse is not listed (the walk gives symmetric lists; nothing
 // here relies on it) and the leaf itself go one way.  The buffer is at most
-// P64_SHARES; systems that would need more take k_p2p64, which adds in another
-// order: the choice is the tree's alone, not that of the memory that happens to be
+// P64_SHARES; systems that would need more, or whose leaves are few and large
+// (p64_pays), take k_p2p64, which adds in another order: the choice is the tree's alone, not that of the memory that happens to be
 // free (but for a device that has none left for the buffer).
 // Measured (one GB300): 10^6 charges: 158 -> 114 ms, the 86,400 dipoles 10.2 -> 8.8 ms.
 constexpr size_t P64_SHARES = (size_t)4 << 30;
@@ -198,31 +198,42 @@ __device__ __forceinline__ bool p64_owns(int A, int B) { return ((A ^ B) & 1) ? 
 
 // Places in the buffer (in particles): for each leaf the sums of its units, one
 // after the other, then what its owned entries leave for their sources, place[k];
-// and the units (cell, leaf, batch of 32 entries).  totals: units, places (64 bits).
+// and the units (cell, leaf, batch of 32 entries).  totals: units, places, then for
+// p64_pays, in interactions: the largest unit, all of them one way, and the most
+// that a warp of k_p2p64 takes (32 targets, or a smaller leaf's, on all its sources).
 __global__ void k_sym_places(const int *leaf_cells, int nleaves, const int *pcount, const int *off, const int *src,
                              uint32_t *place, uint32_t *leaf_place, int4 *units, unsigned long long *totals) {
   constexpr unsigned FULL = 0xffffffffu;
   const int leaf = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (leaf >= nleaves) return;
   const int A = leaf_cells[leaf], k0 = off[A], k1 = off[A + 1], nb = (k1 - k0 + 31) >> 5, na = pcount[A];
-  unsigned sum = 0;
+  unsigned sum = 0, all = 0;
   for (int k = k0 + lane; k < k1; k += 32) {
     const int B = src[k];
-    if (A != B && p64_owns(A, B)) sum += (unsigned)pcount[B];
+    const unsigned n = (unsigned)pcount[B];
+    all += n;
+    if (A != B && p64_owns(A, B)) sum += n;
   }
-  for (int d = 16; d; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+  for (int d = 16; d; d >>= 1) {
+    sum += __shfl_xor_sync(FULL, sum, d);
+    all += __shfl_xor_sync(FULL, all, d);
+  }
   unsigned long long at = 0, ub = 0;
   if (lane == 0) {
     at = atomicAdd(&totals[1], (unsigned long long)sum + (unsigned long long)na * nb);
     ub = atomicAdd(&totals[0], (unsigned long long)nb);
     leaf_place[leaf] = (uint32_t)at;
+    atomicAdd(&totals[3], (unsigned long long)na * all);
+    atomicMax(&totals[4], (unsigned long long)min(na, 32) * all);
   }
   uint32_t run = __shfl_sync(FULL, (uint32_t)at, 0) + (uint32_t)(na * nb);
   ub = __shfl_sync(FULL, ub, 0);
   for (int b = lane; b < nb; b += 32) units[ub + b] = make_int4(A, leaf, b, 0);
+  unsigned most = 0;  // sources of the unit that has most
   for (int kb = k0; kb < k1; kb += 32) {
     const int k = kb + lane, B = k < k1 ? src[k] : A;
     const int n = A != B && p64_owns(A, B) ? pcount[B] : 0;
+    const bool self = __any_sync(FULL, k < k1 && A == B);
     int incl = n;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -230,8 +241,11 @@ __global__ void k_sym_places(const int *leaf_cells, int nleaves, const int *pcou
       if (lane >= d) incl += v;
     }
     if (k < k1) place[k] = run + (uint32_t)(incl - n);
-    run += (uint32_t)__shfl_sync(FULL, incl, 31);
+    const unsigned both = (unsigned)__shfl_sync(FULL, incl, 31);
+    run += both;
+    most = max(most, both + (self ? (unsigned)na : 0u));
   }
+  if (lane == 0) atomicMax(&totals[2], (unsigned long long)na * most);
 }
 // own[k]: place of the shares entry k's target leaves for its source, -1: one way,
 // -2: the source owns the pair, and leaves the target's shares at get[k] (else -1).
@@ -452,6 +466,18 @@ __global__ void __launch_bounds__(128) k_p2p64_gather(const P64Args P, int nleav
   }
 }
 
+// Whether each pair once is the faster way.  A unit is one warp, all targets of its
+// leaf on up to 32 leaves, so in trees of few large leaves the largest unit decides:
+// a warp does 2.6e7 of its pairs a second (dipoles 1.5e7).  One way a warp does 4.7e7
+// (3.0e7) interactions, and the chip 2.4e10 (1.5e10).  Uniform charges, ms each pair
+// once / one way: one leaf of 300 1.87 / 0.21, of 10^4 2,047 / 6.9; 10^4 in 64 leaves 14.8 /
+// 6.9, in 512 0.76 / 2.1; 3x10^4 in 64 leaves 129 / 36, in 512 5.5 / 11.2; 10^5 in 64 leaves
+// 1,357 / 321, in 512 57.8 / 91.7; 3,000 in 64 leaves 1.65 / 1.96, in 8 19.5 / 2.1.
+static bool p64_pays(const unsigned long long *totals) {
+  const double unit = (double)totals[2], all = (double)totals[3], warp = (double)totals[4];
+  return unit <= std::max(all / 950.0, 0.53 * warp);
+}
+
 // The owners and places of this build's pairs and room for the shares: once per
 // build, with a wait for the totals.  No room on the device leaves the build without
 // them, for all its passes.
@@ -462,27 +488,28 @@ static int p64_layout(DevTree *t, cudaStream_t st) {
   t->sym_serial = t->build_serial;
   t->sym_places = -1;
   if (fmm_reserve(t->sym_own, n) || fmm_reserve(t->sym_get, n) || fmm_reserve(t->sym_place, n + (size_t)nl) ||
-      fmm_reserve(t->sym_units, nu) || fmm_reserve(t->sym_totals, 2)) {
+      fmm_reserve(t->sym_units, nu) || fmm_reserve(t->sym_totals, 5)) {
     cudaGetLastError();
     return FMM_OK;
   }
-  FMM_CUDA_TRY(cudaMemsetAsync(t->sym_totals.p, 0, 2 * sizeof(unsigned long long), st));
+  FMM_CUDA_TRY(cudaMemsetAsync(t->sym_totals.p, 0, 5 * sizeof(unsigned long long), st));
   fmm_note_launch(), k_sym_places<<<fmm_blocks(nl, 8), 256, 0, st>>>(
       t->leaf_cells.p, nl, t->pcount.p, t->p2p_off.p, t->p2p_src.p, t->sym_place.p, t->sym_place.p + n, t->sym_units.p,
       t->sym_totals.p);
-  fmm_note_launch(), k_sym_pairs<<<fmm_blocks(nu, 8), 256, 0, st>>>(t->sym_units.p, t->sym_totals.p, t->p2p_off.p,
-                                                                    t->p2p_src.p, t->sym_place.p, t->sym_own.p,
-                                                                    t->sym_get.p);
   FMM_CUDA_TRY(cudaGetLastError());
-  unsigned long long v[2] = {0, 0};
+  unsigned long long v[5] = {};
   FMM_CUDA_TRY(cudaMemcpyAsync(v, t->sym_totals.p, sizeof(v), cudaMemcpyDeviceToHost, st));
   FMM_CUDA_TRY(cudaStreamSynchronize(st));
   const size_t room = 4 * std::max((size_t)v[1], (size_t)1);
-  if (room * sizeof(double) > P64_SHARES) return FMM_OK;
+  if (room * sizeof(double) > P64_SHARES || !p64_pays(v)) return FMM_OK;
   if (fmm_reserve(t->sym_shares, room)) {
     cudaGetLastError();
     return FMM_OK;
   }
+  fmm_note_launch(), k_sym_pairs<<<fmm_blocks(nu, 8), 256, 0, st>>>(t->sym_units.p, t->sym_totals.p, t->p2p_off.p,
+                                                                    t->p2p_src.p, t->sym_place.p, t->sym_own.p,
+                                                                    t->sym_get.p);
+  FMM_CUDA_TRY(cudaGetLastError());
   t->sym_nunits = (long)v[0];
   t->sym_places = (long)v[1];
   return FMM_OK;
