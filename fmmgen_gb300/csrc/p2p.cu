@@ -468,14 +468,16 @@ __global__ void __launch_bounds__(128) k_p2p64_gather(const P64Args P, int nleav
 
 // Whether each pair once is the faster way.  A unit is one warp, all targets of its
 // leaf on up to 32 leaves, so in trees of few large leaves the largest unit decides:
-// a warp does 2.6e7 of its pairs a second (dipoles 1.5e7).  One way a warp does 4.7e7
-// (3.0e7) interactions, and the chip 2.4e10 (1.5e10).  Uniform charges, ms each pair
-// once / one way: one leaf of 300 1.87 / 0.21, of 10^4 2,047 / 6.9; 10^4 in 64 leaves 14.8 /
-// 6.9, in 512 0.76 / 2.1; 3x10^4 in 64 leaves 129 / 36, in 512 5.5 / 11.2; 10^5 in 64 leaves
-// 1,357 / 321, in 512 57.8 / 91.7; 3,000 in 64 leaves 1.65 / 1.96, in 8 19.5 / 2.1.
+// a warp does 3.3e7 of its pairs a second (dipoles 2e7).  One way a warp does 4.7e7
+// (3e7) interactions, and the chip 2.4e10 (1.5e10), of which uneven leaves reach two
+// thirds.  Charges, ms each pair once / one way: one leaf of 300 1.87 / 0.21, of 10^4
+// 2,047 / 6.9; 10^4 uniform in 64 leaves 14.8 / 6.9, in 512 0.76 / 2.1; 3x10^4 in 64 leaves
+// 129 / 36, in 512 5.5 / 11.2; 10^5 in 64 leaves 1,357 / 321, in 512 57.8 / 91.7; 3,000 in 64
+// leaves 1.65 / 1.96, in 8 19.5 / 2.1; 3x10^4 clustered in 800 leaves 10.4 / 15.9, in 190 98 /
+// 35; 10^5 clustered in 954 99 / 73.
 static bool p64_pays(const unsigned long long *totals) {
   const double unit = (double)totals[2], all = (double)totals[3], warp = (double)totals[4];
-  return unit <= std::max(all / 950.0, 0.53 * warp);
+  return unit <= std::max(all / 730.0, 0.69 * warp);
 }
 
 // The owners and places of this build's pairs and room for the shares: once per
