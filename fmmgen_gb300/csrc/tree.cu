@@ -1268,31 +1268,19 @@ static int build_lists(DevTree *t, cudaStream_t st) {
   const int nc = t->ncells;
   const WalkCells W{t->wcell.p, t->cx.p, t->cy.p, t->cz.p, t->crmax.p, (float)(t->theta * t->theta)};
   // raw lists in the walk's order; the buffers keep their capacity between
-  // builds, so a rebuild of a similar tree allocates nothing.  At first: what
-  // uniform and clustered trees need (a list of up to ~480 M2L and 140 P2P
-  // sources a cell), or less where that is more than an eighth of the free memory
+  // builds, so a rebuild of a similar tree allocates nothing.  At first 64 a cell
+  // (2 KB in all), which a tree of short lists never outgrows; a level that does
+  // not fit is walked again with room for it
   DevBuf<int> &m2l_src_raw = t->m2l_src_raw, &m2l_tgt_raw = t->m2l_tgt_raw;
   DevBuf<int> &p2p_tgt_raw = t->p2p_tgt_raw, &p2p_src_raw = t->p2p_src_raw;
   DevBuf<int> *fr[2][2] = {{&t->fa, &t->fb}, {&t->fa2, &t->fb2}};
   TRY(fmm_reserve(t->d_walk, sizeof(WalkState)));
   WalkState *S = (WalkState *)t->d_walk.p, *H = (WalkState *)(t->h_pinned + FMM_PINNED_WALK);
-  const size_t all = (size_t)nc * nc;
-  auto room = [&](size_t m2l, size_t p2p, size_t f) {
-    const size_t cm = std::min(m2l * nc, all) + 1024 + t->nsys, cp = std::min(p2p * nc, all) + 1024 + t->nsys,
-                 cf = std::min(f * nc, all) + 1024 + t->nsys;
-    for (auto &b : fr)
-      if (fmm_reserve(*b[0], cf) || fmm_reserve(*b[1], cf)) return FMM_ERR_CUDA;
-    return fmm_reserve(m2l_src_raw, cm) || fmm_reserve(m2l_tgt_raw, cm) || fmm_reserve(p2p_tgt_raw, cp) ||
-                   fmm_reserve(p2p_src_raw, cp)
-               ? FMM_ERR_CUDA
-               : FMM_OK;
-  };
-  size_t avail = ~(size_t)0, total = 0;
-  if (m2l_src_raw.cap < std::min((size_t)480 * nc, all) && cudaMemGetInfo(&avail, &total) != cudaSuccess) avail = 0;
-  if (avail / 8 < (size_t)nc * 4 * (2 * 480 + 2 * 160 + 4 * 320) || room(480, 160, 320)) {
-    cudaGetLastError();
-    TRY(room(64, 64, 64));
-  }
+  const size_t cap0 = std::min((size_t)64 * nc, (size_t)nc * nc) + 1024 + t->nsys;
+  TRY(fmm_reserve(m2l_src_raw, cap0)); TRY(fmm_reserve(m2l_tgt_raw, cap0));
+  TRY(fmm_reserve(p2p_tgt_raw, cap0)); TRY(fmm_reserve(p2p_src_raw, cap0));
+  for (auto &b : fr)
+    for (DevBuf<int> *q : b) TRY(fmm_reserve(*q, cap0));
   size_t nm2l = 0, np2p = 0;
   uint32_t nf = (uint32_t)t->nsys;
   int cur = 0;  // the frontier to read
