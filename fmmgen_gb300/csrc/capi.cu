@@ -547,7 +547,7 @@ int fmmgen_tree_set_tune(fmmgen_tree *tree, int impl, int nslots, int grouping, 
     fmm_set_error_text("no generated CUDA-core M2L kernels for this order / source order");
     return ret(FMM_ERR_ARG);
   }
-  if ((impl == 4 || impl == 5) && !fmm_m2l_cm_supported(t.order, t.so)) {
+  if (impl == 4 && !fmm_m2l_cm_supported(t.order, t.so)) {
     fmm_set_error_text("no class-major CUDA-core M2L kernels for this order / source order");
     return ret(FMM_ERR_ARG);
   }

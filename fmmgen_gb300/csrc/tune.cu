@@ -40,8 +40,8 @@ int fmm_autotune(DevTree *t, const double *S, int precision, int reps, int max_c
       if (gen) cands.push_back({1, 0, g, 0});
       if (cm) cands.push_back({4, 0, g, 0});
     }
-    // the harmonic kernels, by a number that set_tune takes for this order and source order
-    cands.push_back({maxs > 0 ? 0 : cm ? 5 : -1, 0, g, 0});
+    // the harmonic kernels, as the default where choice 0 can be set
+    cands.push_back({maxs > 0 ? 0 : 5, 0, g, 0});
     cands.push_back({2, 0, g, 0});
   }
   // one pass for the multipoles (the field into a scratch output)

@@ -252,8 +252,8 @@ int fmmgen_tree_m2l_work(fmmgen_tree *tree, double *out4);
  * complete (one system, all 8^l cells of every level), else the default,
  * 4 class-major CUDA-core kernels (a warp takes 32 target cells' pairs of one
  * translation class per step), 5 the kernels over harmonic coefficients (a
- * thread per target cell over a share of its list).  4 and 5 can be chosen for
- * orders up to 12 for charges, 8 for dipoles.  FP64 passes run 5, or the
+ * thread per target cell over a share of its list; every order and source
+ * order).  4 can be chosen for orders up to 12 for charges, 8 for dipoles.  FP64 passes run 5, or the
  * engine with impl 2.  Per-pair M2L orders (fmmgen_tree_set_m2l_orders, an
  * order model) run on 5, on the class-major kernels with impl 4 (mixed
  * passes), on the engine with impl 2.  Mixed passes of a build with M2L pairs
