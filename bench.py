@@ -370,8 +370,8 @@ def main():
             [c["impl"], c["nslots"], c["grouping"], c["overlap"], round(c["ms"], 3)] for c in r["table"]],
             "legend": "impl 0 the default (as 5) / 1 generated CUDA-core / 2 contraction engine / 3 tensor cores "
                       "(level-grid boxes) / 4 generated class-major / 5 harmonic coefficients; nslots = tensor-core "
-                      "pipeline depth; grouping 0 by octant / 1 Morton; overlap 1 / 2 = M2L and P2P side by side "
-                      "(P2P blocks of 4 / 2 warps); M2L + P2P median ms"}
+                      "pipeline depth; grouping 0 by octant / 1 Morton; overlap 1 = M2L and P2P side by side; "
+                      "M2L + P2P median ms"}
     model = None
     if a.dist == "mixture":  # learned per-pair M2L orders: every pass predicts them from its multipoles
         from fmmgen_gb300 import learned

@@ -658,10 +658,10 @@ static int side_stream(DevTree *t) {
 
 // M2L, then P2P (phase records 3 and 4).  With the overlap switch and the
 // tensor-core M2L, the M2L runs on a highest-priority side stream -- its
-// persistent CTAs take one SM each first -- and the P2P blocks run beside it
-// in the registers and shared memory the M2L CTA leaves free (one 4-warp block
-// per SM), so the P2P's FP32 work fills issue slots of the latency-bound MMA
-// pipeline; record 3 marks the M2L's end, record 4 the join.
+// persistent CTAs take one SM each first -- and the P2P's one-warp blocks run
+// beside it in the registers and shared memory the M2L CTA leaves free, so the
+// P2P's FP32 work fills issue slots of the latency-bound MMA pipeline; record 3
+// marks the M2L's end, record 4 the join.
 template <typename T>
 static int m2l_p2p(DevTree *t, const PlanSet *ps, const double *S, const T *M, T *L, bool mixed, int impl, int mstr,
                    int lstr, int dstr, cudaStream_t st) {
@@ -859,7 +859,7 @@ static int evaluate_pass(DevTree *t, const double *S, double *F, int potential, 
 // P2P: 10^4 charges, p = 4, 711 us a step, now 646; 10^6, p = 8, 7.57 and
 // 7.27 ms; 10^5 clustered charges in FP64 11.7 and 9.8 ms.)  Two cases keep the P2P later: an order model reads the
 // near field, so its M2L waits for the P2P, and beside the tensor-core M2L, whose
-// CTAs leave room for one P2P block per SM, it starts with the M2L or after it.
+// CTAs leave little room on an SM, it starts with the M2L or after it.
 // Phase records follow the streams: "M2L" spans the end of M2M to the end of M2L
 // (the class build included), "P2P" the near field's tail after the last of them.
 // Stage the particles and run P2M and M2M on the near-field stream as soon as

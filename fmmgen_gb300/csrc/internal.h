@@ -84,7 +84,7 @@ struct DevTree {
     int nslots = 0;     // tensor-core pipeline depth (operand slots), 0: as many as fit
     int grouping = 0;   // cell order within a level: 0 by octant within the parent, 1 Morton
     int overlap = 0;    // tensor-core M2L on a high-priority side stream, P2P beside it on the SMs' spare
-                        // room in blocks of 4 (1) or 2 (2) warps
+                        // room (1; 2 is the same)
   } tune;
   cudaStream_t s_hi = nullptr;            // the side stream (highest priority)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

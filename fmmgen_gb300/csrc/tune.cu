@@ -7,7 +7,7 @@
 //                   ones, and on trees whose levels are all complete the tensor
 //                   cores (p <= 9); the warp contraction engine;
 //   tensor-core pipeline depth: 2 .. the operand slots that fit in shared memory;
-//   tensor cores alone, or overlapped with the P2P (in 4- or 2-warp blocks);
+//   tensor cores alone, or overlapped with the P2P;
 //   grouping of the cells into tiles / warps: by octant within the parent, or Morton.
 // One evaluation pass computes the multipoles and stages the particles; then
 // the M2L and P2P phases alone are timed `reps` times per candidate with CUDA
@@ -35,7 +35,7 @@ int fmm_autotune(DevTree *t, const double *S, int precision, int reps, int max_c
   for (int g = 0; g < 2; g++) {
     if (precision != 0) {
       if (g == 0 && boxes)  // (their tiles do not depend on the grouping)
-        for (int ov = 0; ov < 3; ov++)
+        for (int ov = 0; ov < 2; ov++)
           for (int s = 2; s <= maxs; s++) cands.push_back({3, s, g, ov});
       if (gen) cands.push_back({1, 0, g, 0});
       if (cm) cands.push_back({4, 0, g, 0});

@@ -237,8 +237,7 @@ class Tree:
         orders),
         tensor-core pipeline depth
         (0: as deep as fits), cell grouping (0 by octant, 1 Morton) and
-        overlap (1 / 2: tensor-core M2L and P2P side by side on the SMs, the
-        P2P in blocks of 4 / 2 warps)."""
+        overlap (1, or 2: tensor-core M2L and P2P side by side on the SMs)."""
         check(lib().fmmgen_tree_set_tune(self._h, int(impl), int(nslots), int(grouping), int(overlap)))
         return self
 

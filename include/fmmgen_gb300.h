@@ -262,9 +262,9 @@ int fmmgen_tree_m2l_work(fmmgen_tree *tree, double *out4);
  * place of 1, 2 and 4; those pairs are done in FP64.
  * nslots: tensor-core pipeline depth (operand slots), 0 = as many as fit.
  * grouping: order of a level's cells in M2L tiles and warps, 0 by octant
- * within the parent, 1 Morton.  overlap: 1 (2) runs the tensor-core M2L on a
- * highest-priority side stream with the P2P beside it on the same SMs, in
- * blocks of 4 (2) warps.
+ * within the parent, 1 Morton.  overlap: 1 (or 2, the same) runs the
+ * tensor-core M2L on a highest-priority side stream with the P2P beside it on
+ * the same SMs.
  * Unsupported choices are rejected. */
 int fmmgen_tree_set_tune(fmmgen_tree *tree, int impl, int nslots, int grouping, int overlap);
 int fmmgen_tree_get_tune(fmmgen_tree *tree, int *tune4);
