@@ -321,6 +321,32 @@ def run_reference(a, rank, world):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
+def m2l_work(order, pairs, orders, tuned, tensor_steps, learned_info):
+    """The M2L kernel of a mixed pass and the flops it executes: `flops` (the tensor-core kernel: the algorithm's, the
+    MMA flops are counted by the kernel), and those of the Cartesian basis for the same pairs."""
+    from fmmgen_gb300 import gen_m2l_h
+
+    if orders is None:
+        cartesian = 2.0 * math.comb(order + 6, 6) * pairs
+        harmonic = 2.0 * gen_m2l_h.multiply_adds(order) * pairs
+    else:  # each pair at its own order
+        cartesian = 2.0 * learned_info["m2l_multiply_adds"]
+        q, n = np.unique(orders, return_counts=True)
+        harmonic = 2.0 * sum(gen_m2l_h.multiply_adds(int(k)) * int(c) for k, c in zip(q, n))
+    if tensor_steps:
+        return {"kernel": "M2L (k_m2l_tcg, tcgen05 kind::f16, source rows boxed from level grids)", "flops": cartesian,
+                "cartesian_flops": cartesian, "work": "2*C(p+6,6) flop x M2L pairs"}
+    full = {1: "M2L (k_m2l_reg_*, generated FP32, a thread per target)",
+            4: "M2L (k_m2l_cm_*, generated FP32, class-major)", 2: "M2L (k_m2l_pk, FP32 contraction engine)"}
+    if tuned in full and orders is None:
+        return {"kernel": full[tuned], "flops": cartesian, "cartesian_flops": cartesian,
+                "work": "2*C(p+6,6) flop x M2L pairs"}
+    return {"kernel": "M2L (k_m2lh_*, generated FP32 over harmonic coefficients, a thread per target"
+                      + (", each pair at its own order)" if orders is not None else ")"),
+            "flops": harmonic, "cartesian_flops": cartesian,
+            "work": "2 flop x the harmonic multiply-adds (p = 8: 1,365) x M2L pairs"}
+
+
 def main():
     a = args_parse()
     rank, world, local = dist_env()
@@ -429,6 +455,8 @@ def main():
     eval_ms, _ = timed(a.steps, lambda: tree.compute_field_fmm(F, potential=a.potential, field=a.field,
                                                                   precision="mixed"))
     tree.set_graph(False)
+    tree.compute_field_fmm(F, potential=a.potential, field=a.field, precision="mixed")
+    alone = tree.kernel_ms()
     eval_max = max_over_ranks(eval_ms, pg, dev)
     eval_only = {"value": job_throughput(a.n, a.steps, world, eval_max), "unit": UNIT, "ms_per_step": eval_max / a.steps,
                  "note": "P2M..L2P only, tree built once; the pass is replayed from its recorded CUDA graph"}
@@ -526,16 +554,11 @@ def main():
     sm_max = peaks.get("sm_max_mhz", 2070.0)
     fp32_peak = 152 * 128 * 2 * sm_max * 1e6 / 1e12  # TFLOP/s, nominal at the max SM clock
     p2p_flops = (20.0 if a.so == 0 else 38.0) * tree.p2p_interactions
-    m2l_flops = 2.0 * math.comb(a.order + 6, 6) * tree.nm2l
-    if learned_info:
-        m2l_flops = 2.0 * learned_info["m2l_multiply_adds"]  # at each pair's own order
-    # each kernel's own device time (events on its stream around its launches; the M2L phase also holds
-    # its schedule and operand preparation), the phase time where a kernel was not timed
-    def ktime(k):
-        v = ph.get("kernel_" + k, -1.0)
-        return v if v > 0 else ph.get(k, 0.0)
-
-    cand = {"P2P": (ktime("P2P"), p2p_flops), "M2L": (ktime("M2L"), m2l_flops)}
+    tuned = tree.get_tune()["impl"]
+    m2l = m2l_work(a.order, tree.nm2l, m2l_orders, tuned, m2l_steps, learned_info)
+    # each kernel's own device time (events on its stream around its launches) in an evaluation, where the M2L and the
+    # P2P run one after the other; in the fused step they share the SMs
+    cand = {"P2P": (alone["P2P"], p2p_flops), "M2L": (alone["M2L"], m2l["flops"])}
     dom = max(cand, key=lambda k: cand[k][0])
     dom_ms, dom_flops = cand[dom]
     traffic, traffic_current = None, None
@@ -550,57 +573,55 @@ def main():
                     # the capture describes the kernel only while its source is unchanged
                     with open(os.path.join(ROOT, f[2]), "rb") as src:
                         traffic_current = hashlib.sha256(src.read()).hexdigest()[:16] == f[3]
+                    if not traffic_current:
+                        traffic = None
         except OSError:
             pass
     achieved = dom_flops / (dom_ms / 1e3) / 1e12 if dom_ms > 0 else 0.0
     roofline = {"kernel": dom, "bound": "fp32", "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak, "traffic": traffic, "traffic_capture_current": traffic_current,
-                "kernel_ms": dom_ms, "time_source": "CUDA events on the kernel's stream around its launches, "
-                                                    "mean over the timed steps (M2L and P2P may run side by side)",
+                "kernel_ms": dom_ms, "kernel_ms_in_step": ph.get("kernel_" + dom),
+                "time_source": "CUDA events on the kernel's stream around its launches, one evaluation after the timed "
+                               "ones (M2L and P2P one after the other; in the step they may run side by side)",
                 "peak_source": "nominal: 152 SMs x 128 FP32 lanes x 2 flop x sm_max_mhz of MEASURED_PEAKS.json "
                                "(no measured FP32 figure exists)",
-                "work": f"{'20 flop x P2P interactions' if dom == 'P2P' else '2*C(p+6,6) flop x M2L pairs'} "
+                "work": f"{'20 flop (dipoles 38) x P2P interactions' if dom == 'P2P' else m2l['work']} "
                         f"per launch = {dom_flops:.3e} flop"}
     m2l_ms, _ = cand["M2L"]
     tpeak = peaks.get("bf16_tflops")  # dense 16-bit tensor peak (FP16 runs at the bf16 rate)
-    exec_tf = m2l_exec_flops / (m2l_ms / 1e3) / 1e12 if m2l_ms > 0 else 0.0
-    alg_tf = m2l_flops / (m2l_ms / 1e3) / 1e12 if m2l_ms > 0 else 0.0
-    tuned = tree.get_tune()["impl"]
-    if m2l_steps:
-        m2l_kernel = "M2L (k_m2l_tcg, tcgen05 kind::f16, source rows boxed from level grids)"
-    elif learned_info:
-        m2l_kernel = ("M2L (k_m2lh_*, generated FP32 over harmonic coefficients, a thread per target, each pair at its "
-                      "own order; the phase includes the pairs' features and the order model's inference)")
+    rate = lambda fl: fl / (m2l_ms / 1e3) / 1e12 if m2l_ms > 0 else 0.0  # noqa: E731
+    roofline_m2l = {"kernel": m2l["kernel"], "kernel_ms": m2l_ms, "unit": "TFLOP/s",
+                    "cartesian_equivalent_tflops": rate(m2l["cartesian_flops"])}
+    if m2l_steps:  # executed: MMA flops issued
+        roofline_m2l.update({
+            "bound": "tensor", "achieved": rate(m2l_exec_flops), "peak": tpeak,
+            "frac": rate(m2l_exec_flops) / tpeak if tpeak else None,
+            "executed_flops_per_launch": m2l_exec_flops, "class_steps": m2l_steps, "mma_instructions": m2l_mmas,
+            "source_rows": "boxed from level grids (tensor-map copies)" if m2l_boxes else None,
+            "note": "achieved = MMA flops issued (3 FP16 products per 16-term chunk, 1 for the chunks of degree >= 6; "
+                    "128-row tiles over the union of the tile's classes, triangular N per chunk); peak = measured bf16 "
+                    "dense (MEASURED_PEAKS.json)"})
     else:
-        m2l_kernel = {1: "M2L (k_m2l_reg_*, generated FP32, a thread per target)",
-                      4: "M2L (k_m2l_cm_*, generated FP32, class-major)",
-                      2: "M2L (k_m2l_pk, FP32 contraction engine)"}.get(
-                          tuned, "M2L (k_m2lh_*, generated FP32 over harmonic coefficients, a thread per target)")
-    roofline_m2l = {"kernel": m2l_kernel,
-                    "bound": "tensor", "achieved": exec_tf, "algorithmic_tflops": alg_tf, "peak": tpeak,
-                    "unit": "TFLOP/s", "frac": exec_tf / tpeak if tpeak else None,
-                    "algorithmic_frac": alg_tf / tpeak if tpeak else None,
-                    "class_steps": m2l_steps, "mma_instructions": m2l_mmas,
-                    "executed_flops_per_launch": m2l_exec_flops, "algorithmic_flops_per_launch": m2l_flops,
-                    "source_rows": "boxed from level grids (tensor-map copies)" if m2l_boxes else None,
-                    "note": "executed = MMA flops issued (3 FP16 products per 16-term chunk, 1 for the chunks of "
-                            "degree >= 6; 128-row tiles over the union of the tile's classes, "
-                            "triangular N per chunk); algorithmic = 2*C(p+6,6) per pair; "
-                            "peak = measured bf16 dense (MEASURED_PEAKS.json)"}
+        roofline_m2l.update({
+            "bound": "fp32", "achieved": rate(m2l["flops"]), "peak": fp32_peak, "frac": rate(m2l["flops"]) / fp32_peak,
+            "executed_flops_per_launch": m2l["flops"],
+            "note": f"achieved = {m2l['work']}; cartesian_equivalent = 2*C(q+6,6) flop per pair, which this kernel does "
+                    "not execute where it works on harmonic coefficients"})
 
     if dom == "M2L":
-        roofline["kernel"] = m2l_kernel
+        roofline["kernel"] = m2l["kernel"]
     if dom == "M2L" and m2l_steps and tpeak:
         # the dominant M2L ran on the tensor cores: its roofline is the measured
         # dense 16-bit tensor peak (algorithmic flops, as for every bound); the
         # FP32 CUDA-core view stays beside it
         roofline_fp32 = roofline
-        roofline = {"kernel": roofline_m2l["kernel"], "bound": "tensor", "achieved": alg_tf, "peak": tpeak,
-                    "unit": "TFLOP/s", "frac": alg_tf / tpeak, "traffic": traffic,
+        roofline = {"kernel": m2l["kernel"], "bound": "tensor", "achieved": rate(m2l["flops"]), "peak": tpeak,
+                    "unit": "TFLOP/s", "frac": rate(m2l["flops"]) / tpeak, "traffic": traffic,
                     "traffic_capture_current": traffic_current, "kernel_ms": m2l_ms,
                     "time_source": roofline_fp32["time_source"],
                     "peak_source": "measured bf16 dense burst (MEASURED_PEAKS.json bf16_tflops)",
-                    "work": roofline_fp32["work"], "executed_achieved": exec_tf, "executed_frac": exec_tf / tpeak,
+                    "work": roofline_fp32["work"], "executed_achieved": rate(m2l_exec_flops),
+                    "executed_frac": rate(m2l_exec_flops) / tpeak,
                     "fp32_view": {k: roofline_fp32[k] for k in ("achieved", "peak", "frac", "peak_source")}}
 
     line = {"metric": metric_name(a), "value": value, "unit": UNIT, "n_gpus": world, "steps": a.steps, "warmup": a.warmup,

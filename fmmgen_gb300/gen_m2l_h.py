@@ -45,6 +45,11 @@ def d_terms(d):
     return 0 if d < 0 else 1 + 3 * d * (d + 1) // 2
 
 
+def multiply_adds(q):
+    """Multiply-adds of a pair at order q, whatever the family and the source order."""
+    return sum((2 * n + 1) * (2 * m + 1) for n in range(q + 1) for m in range(q + 1 - n))
+
+
 def coeffs(p):
     """The coefficient indices (x, y, z), z <= 1, in layout order."""
     return [(x, d - z - x, z) for d in range(p + 1) for z in range(min(d, 1) + 1) for x in range(d - z, -1, -1)]
