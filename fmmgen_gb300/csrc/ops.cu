@@ -9,7 +9,7 @@
 #include "deriv.cuh"
 
 // Every kernel here but P2P and M2P takes one warp per application and, in FP64,
-// is bound by the FP64 pipe (20 clocks of an SM per warp instruction): what
+// is bound by the FP64 pipe (16 clocks of an SM per warp instruction): what
 // counts is the number of those.  20,000 applications, p = 8, FP64, one GB300:
 // P2M 1.48 -> 0.045 ms, M2M and L2L 1.77 -> 0.12 and 0.14 ms, M2L 0.59 -> 0.50 ms,
 // L2P 1.54 -> 0.07 ms.

@@ -18,13 +18,14 @@
 // the stream and their sums are added at the end.  One warp per group, from the
 // build's units of up to 32 targets: the groups of a leaf are independent warps,
 // so leaves of several chunks do not make a tail of long warps, and the grid
-// grows with the particles, not with the largest leaf there could be.  With one lane per target and chunks of 32 a
-// leaf of 14 left 56 % of the lanes idle and one of 40 took two full passes.
-// The sources of the leaf's list are one stream (the leaves' particle ranges
-// one after the other), staged 64 at a time.
-// Measured (one GB300): 10^6 uniform charges, 30 per leaf, 4.79e9 interactions:
-// 229 -> 158 ms; 100,003 clustered charges, 14 per leaf: the whole step 28.0 -> 17.1 ms; 86,400 dipoles, 11 per
-// leaf: 25.8 -> 10.2 ms.
+// grows with the particles, not with the largest leaf there could be.  With one
+// lane per target and chunks of 32 a leaf of 14 left 56 % of the lanes idle and one
+// of 40 took two full passes.  The sources of the leaf's list are one stream (the
+// leaves' particle ranges one after the other), staged 64 at a time.
+// For quadrupoles, and for charges and dipoles where each pair once does not pay
+// or has no room (below).  Measured (one GB300), a warp per leaf before and now: 10^6
+// uniform charges, 30 per leaf, 4.79e9 interactions: 229 and 158 ms; 86,400 dipoles, 11
+// per leaf: 25.8 and 10.2 ms; one leaf of 10,000 charges: 2,000 and 6.9 ms.
 #define P2P_WARPS 4
 #define P64_CHUNK 64
 // components staged per source
@@ -1012,8 +1013,10 @@ __global__ void __launch_bounds__(32 * DIR_WARPS) k_direct(const double *pos, co
 // pair of tiles of 256 particles, a warp 32 of the first tile's as targets, and
 // the block goes over the second tile's in chunks of 32; each warp adds the
 // chunk's side up in shared memory of its own.  Both sides' sums go into
-// parts[tile][other tile][256], which k_direct_sum adds up in order.  From 16 tiles
-// on the pairs of tiles fill the SMs.  30,011 charges: 32.9 -> 18.6 ms.
+// parts[tile][other tile][256], which k_direct_sum adds up in order.  The line: 16
+// tiles, whose 136 pairs come near the number of SMs.  Charges, one way and each pair
+// once: 3,000 0.52 and 0.56 ms, 4,096 0.69 and 0.57, 5,000 1.25 and 0.97, 12,000 4.87 and
+// 3.36, 30,011 32.9 and 18.6 ms; 4,096 dipoles 1.09 and 0.95.
 constexpr int DIR_TILE = 32 * DIR_WARPS;
 constexpr long DIR_SYM_MIN = 16 * DIR_TILE;
 template <int SO>

@@ -17,7 +17,7 @@ A thread takes one target cell and a slice of its list (csrc/m2l_h.cuh has the p
 registers.  Per pair the warp copies the 32 lanes' source and operator rows into shared memory with asynchronous copies,
 eight lanes per row so that each copy instruction covers whole 128-byte lines, a pair ahead of the multiply-adds.  FP32:
 the source row moves into registers and its buffer is refilled at once; the operator is read as 16-byte words.  FP64: the
-FP64 pipe issues one warp instruction per 20 clocks of an SM, so the source row stays in shared memory and each
+FP64 pipe issues one warp instruction per 16 clocks of an SM, so the source row stays in shared memory and each
 multiply-add loads its own operand.  Every index is resolved here; the terms are nested by the degree of k so that a lane
 stops at its pair's order.  Outputs with many terms per pair sum a pair's terms first (rounding grows with the pairs).
 

@@ -40,9 +40,9 @@ extern "C" {
 /* precision modes of fmmgen_tree_compute_field_fmm */
 #define FMMGEN_PREC_FP64 0   /* every phase in FP64 */
 #define FMMGEN_PREC_MIXED 1  /* FP32 sweeps/M2L/P2P, FP64 operator assembly and final accumulation;
-                                M2L on the tensor cores (3 FP16 products per term, FP32
-                                accumulation) for orders <= 9 */
-#define FMMGEN_PREC_MIXED_SIMT 2  /* as FMMGEN_PREC_MIXED with the M2L on the FP32 CUDA cores */
+                                the M2L on the FP32 CUDA cores unless fmmgen_tree_set_tune chooses
+                                the tensor cores (3 FP16 products per term, FP32 accumulation) */
+#define FMMGEN_PREC_MIXED_SIMT 2  /* as FMMGEN_PREC_MIXED, whose default M2L it once differed from */
 
 const char *fmmgen_last_error(void);
 const char *fmmgen_version(void);
@@ -127,7 +127,13 @@ typedef struct fmmgen_tree fmmgen_tree;
  * reference's root cube, ncrit split rule and FP64 centre arithmetic, and the
  * M2L/P2P interaction lists of interact_dehnen_lazy (example/calculate.cpp:81-133).
  * pos: device [N][3].  *tree may be NULL (a new handle is made) or an existing
- * handle whose device buffers are reused.  Synchronises `stream`. */
+ * handle whose device buffers are reused.  Synchronises `stream`.
+ * A handle keeps its buffers until it is freed: about 200 bytes a particle, and
+ * for each cell some 300 bytes, 2 KB of walk buffers or one and a half times what
+ * the lists need (8 bytes a pair as the walk leaves them, 12 as the passes read
+ * them), the expansions and, after an FP64 pass of charges or dipoles, up to 4 GiB
+ * for the near field's shares (10^6 uniform charges, 30 per leaf: 2.6 GB), after
+ * Barnes-Hut 32 (p + 2)^2 + 8 (p + 1)^2 bytes a cell. */
 int fmmgen_tree_build(const double *pos, long N, long ncrit, int order, double theta, int source_order,
                       void *stream, fmmgen_tree **tree);
 
@@ -146,7 +152,11 @@ int fmmgen_forest_build(const double *pos, const long *sys_off, int nsys, long n
 /* Tree::compute_field_fmm (example/tree.cpp:243-271): F (device
  * [N][OUTPUTSIZE], caller's particle order) is overwritten with phi / E from
  * the sources S (device [N][SOURCESIZE], caller's particle order).  Does not
- * synchronise. */
+ * synchronise, but for the first passes after a build, which reserve buffers
+ * and (FP64, charges and dipoles) wait for the near field's layout.  FP64 fields
+ * are the same bits in every pass over a build, whatever else is on the device,
+ * as long as it has room for the near field's shares; a captured first pass of a
+ * tree not evaluated in FP64 before adds in another order. */
 int fmmgen_tree_compute_field_fmm(fmmgen_tree *tree, const double *S, double *F, int potential, int field,
                                   int precision, void *stream);
 
@@ -314,7 +324,9 @@ int fmmgen_tree_set_m2l_orders(fmmgen_tree *tree, const unsigned char *orders, v
  * use): every evaluate then runs P2P before M2L, computes the features for
  * the error target eps from its own multipoles and near field, and applies
  * pair k at the lowest order whose cumulative predicted probability reaches
- * 1 - delta.  params == NULL detaches it. */
+ * 1 - delta.  params == NULL detaches it.  Features and prediction cost more
+ * than the lower orders save: without a model, at p = 12, a mixed step measures
+ * faster at every size from 4x10^5 to 8x10^6 clustered charges (by 11 to 21 %). */
 int fmmgen_tree_set_order_model(fmmgen_tree *tree, const float *params, float delta, double eps);
 /* Host copy of the per-pair orders the last evaluate used (uint8 [nm2l]);
  * all p when it used one order. */
