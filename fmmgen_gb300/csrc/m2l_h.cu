@@ -145,8 +145,9 @@ static int run(DevTree *t, const T *M, int mstr, T *L, int lstr, const unsigned 
   const int p = t->order, so = t->so, nc = t->ncells, pl = p - so;
   if (!fmm_m2l_h_supported(p, so)) return FMM_ERR_STATE;
   if (t->nm2l == 0) {
+    int rc = fmm_mark_kernel(t, 0, st);  // no kernel, and not the time of an earlier pass
     FMM_CUDA_TRY(cudaMemset2DAsync(L, sizeof(T) * lstr, 0, sizeof(T) * fmm_nterms(pl), nc, st));
-    return FMM_OK;
+    return rc ? rc : fmm_mark_kernel(t, 1, st);
   }
   if (int rc = fmm_m2l_csr(t, st)) return rc;
   const int mh = line_stride<T>(h_terms(p)), lh = line_stride<T>(h_terms(pl)), dh = line_stride<T>(h_dterms(p));
