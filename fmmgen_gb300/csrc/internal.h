@@ -117,7 +117,7 @@ struct DevTree {
   DevBuf<float> Mf, Lf;
   DevBuf<double> Fnear, Ffar;             // [N][4] sorted order
   // scratch
-  DevBuf<int> fa, fb, fa2, fb2;           // traversal frontiers
+  DevBuf<int> front;                      // one of the walk's frontiers (the others: m2l_src, m2l_cls, m2l_cls_raw)
   DevBuf<int> m2l_tgt_raw, m2l_src_raw;   // walk output in frontier order (kept between builds)
   DevBuf<int> p2p_tgt_raw, p2p_src_raw;
   uint32_t *h_pinned = nullptr;           // pinned host words for count readbacks

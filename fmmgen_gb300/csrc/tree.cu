@@ -1276,7 +1276,8 @@ static int build_lists(DevTree *t, cudaStream_t st) {
   // every tree: first builds of 10^6 charges 3.4 -> 4.2 ms, of 512 systems 11.0 -> 16.4.)
   DevBuf<int> &m2l_src_raw = t->m2l_src_raw, &m2l_tgt_raw = t->m2l_tgt_raw;
   DevBuf<int> &p2p_tgt_raw = t->p2p_tgt_raw, &p2p_src_raw = t->p2p_src_raw;
-  DevBuf<int> *fr[2][2] = {{&t->fa, &t->fb}, {&t->fa2, &t->fb2}};
+  // the frontiers: in the lists that are made from the walk's output afterwards
+  DevBuf<int> *fr[2][2] = {{&t->m2l_src, &t->m2l_cls}, {&t->m2l_cls_raw, &t->front}};
   TRY(fmm_reserve(t->d_walk, sizeof(WalkState)));
   WalkState *S = (WalkState *)t->d_walk.p, *H = (WalkState *)(t->h_pinned + FMM_PINNED_WALK);
   const double shorter = std::min(1.0, 0.125 / (t->theta * t->theta * t->theta)), few = 4.0 * nc / t->nsys;
@@ -1612,7 +1613,7 @@ void fmm_tree_destroy(DevTree *t) {
   t->ncls_prev = t->order_prev = -1;
   fmm_release(t->M); fmm_release(t->L); fmm_release(t->Mf); fmm_release(t->Lf);
   fmm_release(t->Fnear); fmm_release(t->Ffar);
-  fmm_release(t->fa); fmm_release(t->fb); fmm_release(t->fa2); fmm_release(t->fb2);
+  fmm_release(t->front);
   fmm_release(t->m2l_tgt_raw); fmm_release(t->m2l_src_raw);
   fmm_release(t->p2p_tgt_raw); fmm_release(t->p2p_src_raw);
   fmm_release(t->tc_T);

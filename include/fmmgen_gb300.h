@@ -129,9 +129,9 @@ typedef struct fmmgen_tree fmmgen_tree;
  * pos: device [N][3].  *tree may be NULL (a new handle is made) or an existing
  * handle whose device buffers are reused.  Synchronises `stream`.
  * A handle keeps its buffers until it is freed: about 200 bytes a particle, and
- * for each cell some 300 bytes, up to 10 KB of walk buffers (less for theta above
- * 0.5 and for small systems) or one and a half times what the lists need (8 bytes
- * a pair as the walk leaves them, 12 as the passes read them), the expansions and, after an FP64 pass of charges or dipoles, up to 4 GiB
+ * for each cell some 300 bytes, 11 KB for the lists and the walk that makes them
+ * (less for theta above 0.5 and for small systems) or, where lists are longer,
+ * about 30 bytes an M2L and 12 a P2P pair, the expansions and, after an FP64 pass of charges or dipoles, up to 4 GiB
  * for the near field's shares (10^6 uniform charges, 30 per leaf: 2.6 GB), after
  * Barnes-Hut 32 (p + 2)^2 + 8 (p + 1)^2 bytes a cell. */
 int fmmgen_tree_build(const double *pos, long N, long ncrit, int order, double theta, int source_order,
