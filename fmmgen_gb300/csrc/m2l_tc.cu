@@ -55,6 +55,8 @@ constexpr int TC_MAXSLOTS = 4;
 constexpr int TC_ACC_COLS = 256;  // tensor-memory columns per accumulator
 constexpr int TC_EBIAS = 14;      // operands are scaled to [2^14, 2^15) in magnitude
 constexpr uint32_t TC_WAIT_LIMIT = 1u << 24;
+constexpr int TC_SMEM = 227 * 1024;          // shared memory of a block
+constexpr int TC_BITMAP_SMEM = 160 * 1024;   // a tile schedule's bitmap, at most
 
 __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -597,7 +599,7 @@ bool tc_plan(int p, int so, TcPlan &pl) {
   for (int b = 0; b < pl.nkb; b++)
     bmax = std::max(bmax, pl.choff[std::min(4 * b + 4, pl.kch)] - pl.choff[4 * b]);
   pl.slot_bytes = (2 * TC_A_BYTES + bmax + 1023) / 1024 * 1024;
-  const int budget = 227 * 1024 - 1024 - (int)sizeof(TcShared);
+  const int budget = TC_SMEM - 1024 - (int)sizeof(TcShared);
   pl.nslots = std::min(TC_MAXSLOTS, budget / pl.slot_bytes);
   if (pl.nslots < 2) return false;
   pl.smem = 1024 + pl.nslots * pl.slot_bytes + (int)sizeof(TcShared);
@@ -977,12 +979,11 @@ int tcg_prepare(DevTree *t, const TcPlan &pl, cudaStream_t st) {
                                                                      t->m2l_cls_raw.p, n, t->cls_key4.p, t->ix.p,
                                                                      t->iy.p, t->iz.p, t->clevel.p, s->flag.p);
   const int nparts = 2 * tc_sm_count();
-  if (nbm * sizeof(unsigned) <= 160 * 1024 && n >= 64L * nparts) {
+  if (nbm * sizeof(unsigned) <= TC_BITMAP_SMEM && n >= 64L * nparts) {
     // per-block copies in shared memory, OR-reduced (no hot global atomics)
     const int sbytes = (int)(nbm * sizeof(unsigned));
     if (fmm_reserve(s->part, (size_t)nparts * nbm)) return FMM_ERR_CUDA;
-    if (sbytes > 48 * 1024)
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_tc_bitmap_part, cudaFuncAttributeMaxDynamicSharedMemorySize, sbytes));
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_tc_bitmap_part, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_BITMAP_SMEM));
     fmm_note_launch(), k_tc_bitmap_part<<<nparts, 512, sbytes, st>>>(t->m2l_tgt_raw.p, t->m2l_cls_raw.p, n, s->pos.p,
                                                                       nwords, (int)nbm, s->part.p);
     fmm_note_launch(), k_tc_bitmap_or<<<fmm_blocks(nbm, 256), 256, 0, st>>>(s->part.p, nparts, (int)nbm,
@@ -1059,7 +1060,8 @@ int tcg_full_chunks(const TcPlan &pl) {
 }
 
 template <int NOUT> int tcg_launch(const TcgMaps &maps, const TcgParams &P, int smem, int grid, cudaStream_t st) {
-  FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tcg<NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // the most a block can have: the limit holds for the process, and another thread may be about to launch with more slots
+  FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tcg<NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
   fmm_note_launch(), k_m2l_tcg<NOUT><<<grid, TCG_THREADS, smem, st>>>(maps, P);
   FMM_CUDA_TRY(cudaGetLastError());
   return FMM_OK;
@@ -1201,11 +1203,10 @@ int fmm_tc_schedule(DevTree *t, cudaStream_t st) {
   const long n = t->nm2l;
   fmm_note_launch(), k_tc_pos<<<fmm_blocks(nc, 256), 256, 0, st>>>(t->m2l_order.p, nc, t->tc_pos.p);
   const int nparts = 2 * tc_sm_count();
-  if (nbm * sizeof(unsigned) <= 160 * 1024 && n >= 64L * nparts) {
+  if (nbm * sizeof(unsigned) <= TC_BITMAP_SMEM && n >= 64L * nparts) {
     const int sbytes = (int)(nbm * sizeof(unsigned));
     if (fmm_reserve(t->tc_stab, (size_t)nparts * nbm)) return FMM_ERR_CUDA;  // scratch until the table
-    if (sbytes > 48 * 1024)
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_tc_bitmap_part, cudaFuncAttributeMaxDynamicSharedMemorySize, sbytes));
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_tc_bitmap_part, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_BITMAP_SMEM));
     unsigned *part = (unsigned *)t->tc_stab.p;
     fmm_note_launch(), k_tc_bitmap_part<<<nparts, 512, sbytes, st>>>(t->m2l_tgt_raw.p, t->m2l_cls_raw.p, n,
                                                                       t->tc_pos.p, nwords, (int)nbm, part);
