@@ -14,16 +14,16 @@ def system(n, so, seed):
 
 
 def test_free_memory_does_not_matter(fg):
-    n = 300_000
+    n = 1_000_000
     pos, S = system(n, 0, 1)
-    ref = fg.build_tree(pos, S, n, 64, 3, 0.5).compute_field_fmm(precision="fp64")
+    ref = fg.build_tree(pos, S, n, 128, 3, 0.5).compute_field_fmm(precision="fp64")
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     free = torch.cuda.mem_get_info()[0]
-    # 4 GB stay free: the shares of this tree (~0.8 GB) are more than an eighth of that
-    filler = torch.empty(max(free - (4 << 30), 0), dtype=torch.uint8, device="cuda")
+    # 14 GB stay free: the shares of this tree (2.6 GB) are more than an eighth of that
+    filler = torch.empty(max(free - (14 << 30), 0), dtype=torch.uint8, device="cuda")
     try:
-        t = fg.build_tree(pos, S, n, 64, 3, 0.5)
+        t = fg.build_tree(pos, S, n, 128, 3, 0.5)
         assert torch.equal(t.compute_field_fmm(precision="fp64"), ref)
     finally:
         del filler
